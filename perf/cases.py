@@ -164,20 +164,20 @@ def _state(case, seed):
     psi, at, ax, ay, rho = _columns(case["mu"], case["vy"], case["nz"])
     shape = (case["nz"], case["ny"], case["nx"])
 
-    def wave(amp):
-        # a flow: a smooth disturbance of a gauge field, zero at the boundary
+    def flow():
+        # a uniform flow with a small smooth disturbance, zero at the boundary
         k = torch.randint(1, 4, (2,), device="cuda", generator=g)
         x = torch.arange(case["nx"], dtype=torch.float64, device="cuda") / case["nx"]
         y = torch.arange(case["ny"], dtype=torch.float64, device="cuda") / case["ny"]
         s = torch.sin(2 * math.pi * (k[0] * x[None, :] + k[1] * y[:, None]))
         r = torch.linspace(1, 0, case["nz"], dtype=torch.float64, device="cuda")
-        return amp * r[:, None, None] * s[None]
+        return r[:, None, None] * (0.3 + 1e-3 * s[None])
 
     col = [c.to("cuda")[:, None, None] for c in (psi, at, ax, ay)]
     Z1 = (col[0] * _plane(case, g)[None]).contiguous()
     Z2 = (col[1] + torch.zeros(shape, dtype=torch.float64, device="cuda")).contiguous()
-    Z3 = (col[2] + wave(0.3)).contiguous()
-    Z4 = (col[3] + wave(0.3)).contiguous()
+    Z3 = (col[2] + flow()).contiguous()
+    Z4 = (col[3] + flow()).contiguous()
     return [Z1, Z2, Z3, Z4, torch.full(shape, rho, dtype=torch.float64, device="cuda")]
 
 
