@@ -56,6 +56,11 @@ struct hqt_ctx {
     FFTPlan planx{}, plany{};
     double2 *rootsx = nullptr, *rootsy = nullptr;
     float2 *rootsx32 = nullptr, *rootsy32 = nullptr;
+    // FP64 in-place transforms (np = 0: no such plan): twiddles per pass, and
+    // the digit reversals a runtime plan reads
+    LPlan lpx{}, lpy{};
+    double2 *twx = nullptr, *twy = nullptr;
+    int *freqx = nullptr, *freqy = nullptr, *posx = nullptr, *posy = nullptr;
     double *mx = nullptr, *my = nullptr;
     // x-spectral columns zeroed by the symmetrised filter weight,
     // mx(kx) = mx(-kx) = 0: one contiguous range (dead0 > dead1 when empty)
@@ -100,7 +105,7 @@ struct hqt_ctx {
     DevStatus *st = nullptr;
     // launch geometry
     int NBx_rhs = 1, NBx_2 = 1, TXy_rhs = 1, TXy_2 = 1, TXy_filt = 1;
-    bool cx = false, cy = false;  // compile-time line transforms along x / y
+    bool cx = false, cy = false;  // compile-time line passes along x / y
     bool px = false, py = false;  // prime-factor tensor-core transforms along x / y
     // mixed precision with the filter on the prime-factor engine: the filter
     // passes leave the slice means and the FP32 stage-1 copies of the state,
@@ -214,6 +219,7 @@ bool ct_supported(int n) {
     return false;
 }
 
+// FP32 pass of a compile-time length
 int ct_dispatch(hqt_ctx *c, int n, int kind, const void *args, dim3 grid, size_t smem) {
     switch (n) {
 #define HQT_CD(N)                                                    \
@@ -224,6 +230,53 @@ int ct_dispatch(hqt_ctx *c, int n, int kind, const void *args, dim3 grid, size_t
 #undef HQT_CD
     }
     return fail(c, HQT_EUNSUPPORTED, "no compile-time transform for this length");
+}
+
+// Whether the FP64 passes along an axis run on the in-place transforms.
+bool in_place(const hqt_ctx *c, bool y) {
+    return y ? !c->py && c->lpy.np > 0 : !c->px && c->lpx.np > 0;
+}
+
+// Tables and runtime geometry of an in-place axis; `half`: half the lines per
+// block (a candidate of the autotuner).
+LineTab<double> line_tab(const hqt_ctx *c, bool y, bool half) {
+    const LPlan &p = y ? c->lpy : c->lpx;
+    LineTab<double> t{};
+    if (p.np == 0) return t;
+    t.tw = y ? c->twy : c->twx;
+    t.freq = y ? c->freqy : c->freqx;
+    t.pos = y ? c->posy : c->posx;
+    int nbl = lnbl(p.n, y);
+    if (half && nbl > 0) --nbl;
+    t.g.n_ = p.n;
+    t.g.nbl_ = nbl;
+    t.g.np_ = p.np;
+    t.g.th_ = lthreads(p.n, nbl);
+    t.g.swz_ = lswz(p.n, nbl, sizeof(double2));
+    for (int i = 0; i < p.np; ++i) {
+        t.g.R_[i] = p.R[i];
+        t.g.s_[i] = p.s[i];
+        t.g.tw_[i] = p.tw[i];
+        t.g.mg_[i] = (unsigned)(((1ull << 32) + p.s[i] - 1) / p.s[i]);
+    }
+    return t;
+}
+
+// An FP64 in-place pass along x or y (nsl: z slices of a y pass).
+int line_pass(hqt_ctx *c, bool y, int kind, const void *args, int nsl) {
+    if (y ? c->cy : c->cx) {
+        switch (y ? c->ny : c->nx) {
+#define HQT_CD(N)                                                         \
+    case N:                                                               \
+        CK(y ? ct_launch_y64<N>(kind, args, nsl, c->stream)               \
+             : ct_launch_x64<N>(kind, args, c->stream));                  \
+        return HQT_OK;
+            HQT_LN_LIST(HQT_CD)
+#undef HQT_CD
+        }
+    }
+    CK(y ? line_rt_launch_y(kind, args, nsl, c->stream) : line_rt_launch_x(kind, args, c->stream));
+    return HQT_OK;
 }
 
 template <typename P> int dalloc(hqt_ctx *c, P **ptr, size_t bytes) {
@@ -257,6 +310,7 @@ int launch_x_rhs(hqt_ctx *c, const double2 *psi, const double *ax, const double 
     a.plan = c->planx;
     a.roots = c->rootsx;
     a.NB = c->NBx_rhs;
+    a.lt = line_tab(c, false, c->NBx_rhs < pick_lines(c->nx, 3, 32));
     a.nlines = c->ny * c->nz;
     const double two_pi = 2.0 * 3.14159265358979323846;
     a.s1 = two_pi / c->p.Lx / c->nx;
@@ -274,11 +328,7 @@ int launch_x_rhs(hqt_ctx *c, const double2 *psi, const double *ax, const double 
         CK(pfa_launch_301(CT_X_RHS, &a, a.nlines, c->stream));
         return HQT_OK;
     }
-    if (c->cx) {
-        const int nb = ct_lines(c->nx, 3);
-        RC(ct_dispatch(c, c->nx, CT_X_RHS, &a, dim3((a.nlines + nb - 1) / nb), smem_x(c->nx, 3, nb)));
-        return HQT_OK;
-    }
+    if (in_place(c, false)) return line_pass(c, false, CT_X_RHS, &a, 0);
     CK(launch_x_rhs(a, grid, smem_x(c->nx, 3, a.NB), c->stream));
     return HQT_OK;
 }
@@ -288,6 +338,7 @@ int launch_y_rhs(hqt_ctx *c, const double2 *psi, const double *ax, const double 
     a.plan = c->plany;
     a.roots = c->rootsy;
     a.TX = c->TXy_rhs;
+    a.lt = line_tab(c, true, c->TXy_rhs < pick_lines(c->ny, 4, 16));
     a.nx = c->nx;
     a.ny = c->ny;
     const double two_pi = 2.0 * 3.14159265358979323846;
@@ -309,12 +360,7 @@ int launch_y_rhs(hqt_ctx *c, const double2 *psi, const double *ax, const double 
         CK(pfa_launch_301(CT_Y_RHS, &a, c->nz, c->stream));
         return HQT_OK;
     }
-    if (c->cy) {
-        const int nb = ct_lines_y(c->ny, 3);
-        RC(ct_dispatch(c, c->ny, CT_Y_RHS, &a, dim3((c->nx + nb - 1) / nb, c->nz),
-                       smem_x(c->ny, 3, nb)));
-        return HQT_OK;
-    }
+    if (in_place(c, true)) return line_pass(c, true, CT_Y_RHS, &a, c->nz);
     CK(launch_y_rhs(a, grid, smem_x(c->ny, 4, a.TX), c->stream));
     return HQT_OK;
 }
@@ -324,6 +370,7 @@ int launch_x_d1(hqt_ctx *c, FieldIn<double> in, FieldOut<double> out, int nslice
     a.plan = c->planx;
     a.roots = c->rootsx;
     a.NB = c->NBx_2;
+    a.lt = line_tab(c, false, c->NBx_2 < pick_lines(c->nx, 2, 32));
     a.nlines = c->ny * (nslices > 0 ? nslices : c->nz);
     a.s1 = 2.0 * 3.14159265358979323846 / c->p.Lx / c->nx;
     a.in = in;
@@ -334,11 +381,7 @@ int launch_x_d1(hqt_ctx *c, FieldIn<double> in, FieldOut<double> out, int nslice
         CK(pfa_launch_301(CT_X_D1, &a, a.nlines, c->stream));
         return HQT_OK;
     }
-    if (c->cx) {
-        const int nb = ct_lines(c->nx, 2);
-        RC(ct_dispatch(c, c->nx, CT_X_D1, &a, dim3((a.nlines + nb - 1) / nb), smem_x(c->nx, 2, nb)));
-        return HQT_OK;
-    }
+    if (in_place(c, false)) return line_pass(c, false, CT_X_D1, &a, 0);
     CK(launch_x_d1(a, grid, smem_x(c->nx, 2, a.NB), c->stream));
     return HQT_OK;
 }
@@ -350,6 +393,7 @@ int launch_y_d1(hqt_ctx *c, FieldIn<double> in, const double *add_re, FieldOut<d
     a.plan = c->plany;
     a.roots = c->rootsy;
     a.TX = c->TXy_2;
+    a.lt = line_tab(c, true, c->TXy_2 < pick_lines(c->ny, 2, 16));
     a.nx = c->nx;
     a.ny = c->ny;
     a.s1 = 2.0 * 3.14159265358979323846 / c->p.Ly / c->ny;
@@ -362,12 +406,7 @@ int launch_y_d1(hqt_ctx *c, FieldIn<double> in, const double *add_re, FieldOut<d
         CK(pfa_launch_301(CT_Y_D1, &a, nsl, c->stream));
         return HQT_OK;
     }
-    if (c->cy) {
-        const int nb = ct_lines_y(c->ny, 2);
-        RC(ct_dispatch(c, c->ny, CT_Y_D1, &a, dim3((c->nx + nb - 1) / nb, nsl),
-                       smem_x(c->ny, 2, nb)));
-        return HQT_OK;
-    }
+    if (in_place(c, true)) return line_pass(c, true, CT_Y_D1, &a, nsl);
     CK(launch_y_d1(a, grid, smem_x(c->ny, 2, a.TX), c->stream));
     return HQT_OK;
 }
@@ -507,6 +546,7 @@ int launch_filter(hqt_ctx *c, int nf, const FieldIn<double> *in, const FieldOut<
         a.plan = c->planx;
         a.roots = c->rootsx;
         a.NB = c->NBx_2;
+        a.lt = line_tab(c, false, c->NBx_2 < pick_lines(c->nx, 2, 32));
         a.nlines = c->ny * c->nz;
         a.ny = c->ny;
         a.nf = nf;
@@ -521,10 +561,8 @@ int launch_filter(hqt_ctx *c, int nf, const FieldIn<double> *in, const FieldOut<
         Prof pr(c, K_FILT_X_FWD);
         if (c->px) {
             CK(pfa_launch_301(CT_FX_FWD, &a, a.nlines, c->stream));
-        } else if (c->cx) {
-            const int nb = ct_lines(c->nx, 2);
-            RC(ct_dispatch(c, c->nx, CT_FX_FWD, &a, dim3((a.nlines + nb - 1) / nb),
-                           smem_x(c->nx, 2, nb)));
+        } else if (in_place(c, false)) {
+            RC(line_pass(c, false, CT_FX_FWD, &a, 0));
         } else {
             CK(launch_x_filt_fwd(a, grid, smem_x(c->nx, 2, a.NB), c->stream));
         }
@@ -534,6 +572,7 @@ int launch_filter(hqt_ctx *c, int nf, const FieldIn<double> *in, const FieldOut<
         a.plan = c->plany;
         a.roots = c->rootsy;
         a.TX = c->TXy_filt;
+        a.lt = line_tab(c, true, c->TXy_filt < pick_lines(c->ny, 6, 16));
         a.nx = c->nx;
         a.ny = c->ny;
         a.nf = nf;
@@ -552,10 +591,8 @@ int launch_filter(hqt_ctx *c, int nf, const FieldIn<double> *in, const FieldOut<
         Prof pr(c, K_FILT_Y);
         if (c->py) {
             CK(pfa_launch_301(CT_FY, &a, c->nz, c->stream));
-        } else if (c->cy) {
-            const int tx = ct_lines_y(c->ny, 6);
-            RC(ct_dispatch(c, c->ny, CT_FY, &a, dim3((c->nx + tx - 1) / tx, c->nz),
-                           smem_x(c->ny, 2, 3 * tx)));
+        } else if (in_place(c, true)) {
+            RC(line_pass(c, true, CT_FY, &a, c->nz));
         } else {
             CK(launch_y_filt(a, grid, smem_x(c->ny, 2, a.TX * 3), c->stream));
         }
@@ -565,6 +602,7 @@ int launch_filter(hqt_ctx *c, int nf, const FieldIn<double> *in, const FieldOut<
         a.plan = c->planx;
         a.roots = c->rootsx;
         a.NB = c->NBx_2;
+        a.lt = line_tab(c, false, c->NBx_2 < pick_lines(c->nx, 2, 32));
         a.nlines = c->ny * c->nz;
         a.nf = nf;
         for (int f = 0; f < nf; ++f) {
@@ -588,10 +626,8 @@ int launch_filter(hqt_ctx *c, int nf, const FieldIn<double> *in, const FieldOut<
         Prof pr(c, K_FILT_X_INV);
         if (c->px) {
             CK(pfa_launch_301(CT_FX_INV, &a, a.nlines, c->stream));
-        } else if (c->cx) {
-            const int nb = ct_lines(c->nx, 2);
-            RC(ct_dispatch(c, c->nx, CT_FX_INV, &a, dim3((a.nlines + nb - 1) / nb),
-                           smem_x(c->nx, 2, nb)));
+        } else if (in_place(c, false)) {
+            RC(line_pass(c, false, CT_FX_INV, &a, 0));
         } else {
             CK(launch_x_filt_inv(a, grid, smem_x(c->nx, 2, a.NB), c->stream));
         }
@@ -1101,7 +1137,7 @@ bool same_geom(const LineGeom &a, const LineGeom &b) {
            a.TXy_2 == b.TXy_2 && a.TXy_filt == b.TXy_filt;
 }
 
-const char *engine_name(bool p, bool ct) { return p ? "prime-factor" : ct ? "stockham" : "runtime"; }
+const char *engine_name(bool p, bool ct) { return p ? "prime-factor" : ct ? "compile-time" : "runtime"; }
 
 std::string geom_json(const LineGeom &g) {
     char b[256];
@@ -1215,10 +1251,11 @@ int autotune(hqt_ctx *c) {
     std::vector<LineGeom> cand;
     std::vector<std::pair<bool, bool>> ex, ey;  // (prime-factor, stockham)
     if (pfa_length(c->nx)) ex.push_back({true, false});
-    if (ct_supported(c->nx)) ex.push_back({false, true});
+    // (a compile-time length without an in-place plan has only FP32 passes)
+    if (ct_supported(c->nx) && (c->mixed || c->lpx.np)) ex.push_back({false, true});
     ex.push_back({false, false});
     if (pfa_length(c->ny)) ey.push_back({true, false});
-    if (ct_supported(c->ny)) ey.push_back({false, true});
+    if (ct_supported(c->ny) && (c->mixed || c->lpy.np)) ey.push_back({false, true});
     ey.push_back({false, false});
     for (auto x : ex)
         for (auto y : ey) {
@@ -1291,6 +1328,42 @@ void signed_k(int n, double scale, std::vector<double> &k) {
             m = (i <= (n - 1) / 2) ? i : i - n;
         k[i] = scale * (double)m;
     }
+}
+
+// 2-D forward transform of one complex plane W into S (natural order).
+int forward_2d(hqt_ctx *c, const double2 *W, double2 *S) {
+    {
+        XFiltFwdArgs<double> a{};
+        a.plan = c->planx;
+        a.roots = c->rootsx;
+        a.NB = c->NBx_2;
+        a.lt = line_tab(c, false, c->NBx_2 < pick_lines(c->nx, 2, 32));
+        a.nlines = c->ny;
+        a.ny = c->ny;
+        a.nf = 1;
+        a.in[0] = FieldIn<double>{W, nullptr, nullptr};
+        a.spec[0] = S;
+        a.st = nullptr;
+        if (c->px) {
+            CK(pfa_launch_301(CT_FX_FWD, &a, a.nlines, c->stream));
+        } else if (in_place(c, false)) {
+            RC(line_pass(c, false, CT_FX_FWD, &a, 0));
+        } else {
+            CK(launch_x_filt_fwd(a, (c->ny + a.NB - 1) / a.NB, smem_x(c->nx, 2, a.NB), c->stream));
+        }
+    }
+    YFiltArgs<double> a{};
+    a.plan = c->plany;
+    a.roots = c->rootsy;
+    a.TX = c->TXy_2;
+    a.lt = line_tab(c, true, c->TXy_2 < pick_lines(c->ny, 2, 16));
+    a.nx = c->nx;
+    a.ny = c->ny;
+    a.nf = 1;
+    a.spec[0] = S;
+    if (in_place(c, true)) return line_pass(c, true, CT_Y_FWD, &a, 1);
+    CK(launch_y_fwd(a, dim3((c->nx + a.TX - 1) / a.TX, 1), smem_x(c->ny, 2, a.TX), c->stream));
+    return HQT_OK;
 }
 
 // Density-weighted boundary velocity of O (scripts/analysis/plots_cluster.m:92-93,
@@ -1434,35 +1507,7 @@ int structure_factor_dev(hqt_ctx *c, const double2 *Phi, double Lx, double Ly, i
     double2 *W = c->E, *S = c->dxpsi;
     k_vort_weights<<<kPartials, 256, 0, c->stream>>>(q, c->plane, W);
     CK(cudaGetLastError());
-    {
-        XFiltFwdArgs<double> a{};
-        a.plan = c->planx;
-        a.roots = c->rootsx;
-        a.NB = c->NBx_2;
-        a.nlines = c->ny;
-        a.ny = c->ny;
-        a.nf = 1;
-        a.in[0] = FieldIn<double>{W, nullptr, nullptr};
-        a.spec[0] = S;
-        a.st = nullptr;
-        if (c->cx) {
-            const int nb = ct_lines(c->nx, 2);
-            RC(ct_dispatch(c, c->nx, CT_FX_FWD, &a, dim3((c->ny + nb - 1) / nb), smem_x(c->nx, 2, nb)));
-        } else {
-            CK(launch_x_filt_fwd(a, (c->ny + a.NB - 1) / a.NB, smem_x(c->nx, 2, a.NB), c->stream));
-        }
-    }
-    {
-        YFiltArgs<double> a{};
-        a.plan = c->plany;
-        a.roots = c->rootsy;
-        a.TX = c->TXy_2;
-        a.nx = c->nx;
-        a.ny = c->ny;
-        a.nf = 1;
-        a.spec[0] = S;
-        CK(launch_y_fwd(a, dim3((c->nx + a.TX - 1) / a.TX, 1), smem_x(c->ny, 2, a.TX), c->stream));
-    }
+    RC(forward_2d(c, W, S));
     std::vector<double> ky, kx;
     signed_k(n0, dky, ky);
     signed_k(n1, dkx, kx);
@@ -1514,35 +1559,7 @@ int energy_spectrum(hqt_ctx *c, const double2 *O, int capacity, double *kout, do
     if (capacity < nbins) return fail(c, HQT_EINVAL, "spectrum capacity too small");
     double2 *U = c->E, *S = c->dxpsi;
     RC(boundary_velocity(c, O, U, nullptr, nullptr));
-    {
-        XFiltFwdArgs<double> a{};
-        a.plan = c->planx;
-        a.roots = c->rootsx;
-        a.NB = c->NBx_2;
-        a.nlines = c->ny;
-        a.ny = c->ny;
-        a.nf = 1;
-        a.in[0] = FieldIn<double>{U, nullptr, nullptr};
-        a.spec[0] = S;
-        a.st = nullptr;
-        if (c->cx) {
-            const int nb = ct_lines(c->nx, 2);
-            RC(ct_dispatch(c, c->nx, CT_FX_FWD, &a, dim3((c->ny + nb - 1) / nb), smem_x(c->nx, 2, nb)));
-        } else {
-            CK(launch_x_filt_fwd(a, (c->ny + a.NB - 1) / a.NB, smem_x(c->nx, 2, a.NB), c->stream));
-        }
-    }
-    {
-        YFiltArgs<double> a{};
-        a.plan = c->plany;
-        a.roots = c->rootsy;
-        a.TX = c->TXy_2;
-        a.nx = c->nx;
-        a.ny = c->ny;
-        a.nf = 1;
-        a.spec[0] = S;
-        CK(launch_y_fwd(a, dim3((c->nx + a.TX - 1) / a.TX, 1), smem_x(c->ny, 2, a.TX), c->stream));
-    }
+    RC(forward_2d(c, U, S));
     CK(cudaMemcpyAsync(c->kxv, kx.data(), sizeof(double) * c->nx, cudaMemcpyHostToDevice, c->stream));
     CK(cudaMemcpyAsync(c->kyv, ky.data(), sizeof(double) * c->ny, cudaMemcpyHostToDevice, c->stream));
     CK(cudaMemsetAsync(c->bins, 0, sizeof(double) * 3 * nbins, c->stream));
@@ -1654,6 +1671,8 @@ int hqt_create(const hqt_params *params, int device, hqt_ctx **out) {
     // Fourier plans, roots, filter masks
     c->planx = make_plan(p.nx);
     c->plany = make_plan(p.ny);
+    c->lpx = lplan(p.nx);
+    c->lpy = lplan(p.ny);
     if (c->planx.npass > kMaxPass || c->plany.npass > kMaxPass) {
         c->err = "line length has too many factors";
         return bail(HQT_EUNSUPPORTED);
@@ -1666,6 +1685,12 @@ int hqt_create(const hqt_params *params, int device, hqt_ctx **out) {
     A(&c->rootsy, sizeof(double2) * p.ny);
     A(&c->mx, sizeof(double) * p.nx);
     A(&c->my, sizeof(double) * p.ny);
+    A(&c->twx, sizeof(double2) * (c->lpx.ntw + 1));
+    A(&c->twy, sizeof(double2) * (c->lpy.ntw + 1));
+    A(&c->freqx, sizeof(int) * p.nx);
+    A(&c->freqy, sizeof(int) * p.ny);
+    A(&c->posx, sizeof(int) * p.nx);
+    A(&c->posy, sizeof(int) * p.ny);
     const size_t V = (size_t)c->vol, P2 = (size_t)c->plane;
     A(&c->psi, sizeof(double2) * V);
     A(&c->at, sizeof(double) * V);
@@ -1767,6 +1792,22 @@ int hqt_create(const hqt_params *params, int device, hqt_ctx **out) {
             c->err = "operator upload failed";
             return bail(HQT_ECUDA);
         }
+        for (int y = 0; y < 2; ++y) {
+            const LPlan &lp = y ? c->lpy : c->lpx;
+            if (lp.np == 0) continue;
+            std::vector<double2> tw;
+            std::vector<int> freq, pos;
+            make_line_tables(lp, y ? ry : rx, tw, freq, pos);
+            if (cudaMemcpy(y ? c->twy : c->twx, tw.data(), sizeof(double2) * tw.size(),
+                           cudaMemcpyHostToDevice) ||
+                cudaMemcpy(y ? c->freqy : c->freqx, freq.data(), sizeof(int) * freq.size(),
+                           cudaMemcpyHostToDevice) ||
+                cudaMemcpy(y ? c->posy : c->posx, pos.data(), sizeof(int) * pos.size(),
+                           cudaMemcpyHostToDevice)) {
+                c->err = "twiddle upload failed";
+                return bail(HQT_ECUDA);
+            }
+        }
     }
     // launch geometry and shared-memory opt-in
     c->NBx_rhs = pick_lines(p.nx, 3, 32);
@@ -1780,8 +1821,8 @@ int hqt_create(const hqt_params *params, int device, hqt_ctx **out) {
     c->py = pfa_length(p.ny);
     if (const char *env = std::getenv("HQT_PDL")) c->pdl = std::string(env) != "0";
     if (const char *env = std::getenv("HQT_LINE_ENGINE")) {
-        // "runtime" forces the runtime-plan engine, "stockham" the
-        // compile-time Stockham engine (the tests cover all three)
+        // "runtime" forces runtime plans, "stockham" only keeps the
+        // prime-factor engine out (the tests cover all engines)
         if (std::string(env) == "runtime") c->cx = c->cy = false;
         if (std::string(env) == "runtime" || std::string(env) == "stockham")
             c->px = c->py = false;
@@ -1811,11 +1852,18 @@ int hqt_create(const hqt_params *params, int device, hqt_ctx **out) {
         cudaError_t e = fft_init(tc.data(), ts.data(), (int)tc.size(), maxs);
         std::vector<double> bc, bs;
         make_big_tables(bc, bs);
+        if (e == cudaSuccess) e = pfa_init_301();
+        if (e == cudaSuccess) e = line_rt_init_x(maxs);
+        if (e == cudaSuccess) e = line_rt_init_y(maxs);
 #define HQT_CI(N)                                                                            \
     if (e == cudaSuccess)                                                                    \
         e = ct_init<N>(tc.data(), ts.data(), (int)tc.size(), bc.data(), bs.data(), (int)bc.size(), maxs);
         HQT_CN_LIST(HQT_CI)
 #undef HQT_CI
+#define HQT_LI(N) \
+    if (e == cudaSuccess) e = ct_init64<N>(maxs);
+        HQT_LN_LIST(HQT_LI)
+#undef HQT_LI
 #define HQT_Z(N) \
     if (e == cudaSuccess) e = z_init<N>(maxs);
         HQT_NZP_LIST(HQT_Z)

@@ -1,6 +1,7 @@
 // hqt_args.h -- kernel argument blocks (plain structs, host and device).
 #pragma once
 #include "hqt_common.cuh"
+#include "hqt_lineplan.h"
 
 namespace hqt {
 
@@ -27,6 +28,7 @@ __host__ __device__ inline bool real_field_d1(const FieldIn<T> &in, const FieldO
 }
 
 template <typename T> struct XRhsArgs {
+    LineTab<T> lt;  // in-place transforms
     FFTPlan plan;
     const C2<T> *roots;
     int NB, nlines;
@@ -38,6 +40,7 @@ template <typename T> struct XRhsArgs {
 };
 
 template <typename T> struct YRhsArgs {
+    LineTab<T> lt;  // in-place transforms
     FFTPlan plan;
     const C2<T> *roots;
     int TX, nx, ny;
@@ -51,6 +54,7 @@ template <typename T> struct YRhsArgs {
 };
 
 template <typename T> struct XD1Args {
+    LineTab<T> lt;  // in-place transforms
     FFTPlan plan;
     const C2<T> *roots;
     int NB, nlines;
@@ -60,6 +64,7 @@ template <typename T> struct XD1Args {
 };
 
 template <typename T> struct YD1Args {
+    LineTab<T> lt;  // in-place transforms
     FFTPlan plan;
     const C2<T> *roots;
     int TX, nx, ny;
@@ -70,6 +75,7 @@ template <typename T> struct YD1Args {
 };
 
 template <typename T> struct XFiltFwdArgs {
+    LineTab<T> lt;  // in-place transforms
     FFTPlan plan;
     const C2<T> *roots;
     int NB, nlines, ny;
@@ -82,6 +88,7 @@ template <typename T> struct XFiltFwdArgs {
 };
 
 template <typename T> struct YFiltArgs {
+    LineTab<T> lt;  // in-place transforms
     FFTPlan plan;
     const C2<T> *roots;
     int TX, nx, ny;
@@ -98,6 +105,7 @@ template <typename T> struct YFiltArgs {
 };
 
 template <typename T> struct XFiltInvArgs {
+    LineTab<T> lt;  // in-place transforms
     FFTPlan plan;
     const C2<T> *roots;
     int NB, nlines;

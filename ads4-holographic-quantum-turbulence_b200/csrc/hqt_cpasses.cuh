@@ -1,5 +1,6 @@
-// hqt_cpasses.cuh -- the spectral passes of hqt_passes.cuh with a
-// compile-time line length N (hqt_cfft.cuh).  One translation unit per N
+// hqt_cpasses.cuh -- the FP32 stage passes (mixed precision) of
+// hqt_passes.cuh with a compile-time line length N (hqt_cfft.cuh; the FP64
+// passes run in place, hqt_line_passes.cuh).  One translation unit per N
 // (hqt_c<N>.cu) instantiates them.  A block always transforms its full
 // compile-time batch; lines past the end of the grid are zero-filled and
 // never stored.
@@ -44,29 +45,6 @@ __device__ __forceinline__ void cx_load_pair_async(int buf, int valid, long long
             cp_async<sizeof(T)>(&d.y, im + g0 + t);
         } else {
             d = mk2<T>(T(0), T(0));
-        }
-    }
-}
-// a FieldIn (complex, or re with optional im) into the x-line layout of
-// cx_load by cp.async (zero past `valid` and for a missing im); the caller
-// commits and waits
-template <typename T, int N, int NB>
-__device__ __forceinline__ void cx_load_field_async(int buf, int valid, long long g0,
-                                                    const FieldIn<T> &f) {
-    const CtView<T, N> s = ctv<T, N>(buf);
-    for (int t = threadIdx.x; t < N * NB; t += ct_threads<T, N, NB>()) {
-        const int b = t / N, e = t - b * N;
-        C2<T> &d = s[e * NB + b];
-        if (b >= valid) {
-            d = mk2<T>(T(0), T(0));
-        } else if (f.c) {
-            cp_async<sizeof(C2<T>)>(&d, f.c + g0 + t);
-        } else {
-            cp_async<sizeof(T)>(&d.x, f.re + g0 + t);
-            if (f.im)
-                cp_async<sizeof(T)>(&d.y, f.im + g0 + t);
-            else
-                d.y = T(0);
         }
     }
 }
@@ -393,146 +371,6 @@ __global__ void HQT_CT_BOUNDS k_y_d1r_c(YD1Args<T> a) {
             if (r0 < nr) a.out.re[gy + r0] = v.x + x[i].x;
             if (r1 < nr) a.out.re[gy + r1] = v.y + x[i].y;
         }
-    }
-}
-
-template <typename T, int N>
-__global__ void HQT_CT_BOUNDS k_x_filt_fwd_c(XFiltFwdArgs<T> a) {
-    constexpr int NB = ct_lines(N, 2, sizeof(C2<T>));
-    const int L0 = blockIdx.x * NB;
-    const int valid = min(NB, a.nlines - L0);
-    constexpr int R = 0, A = N, B = N + NB * N;
-    const long long g0 = (long long)L0 * N;
-    ct_load_roots<T, N>(R, a.roots);
-    pdl_wait();
-    const int w = a.st ? a.st->winding : 0;
-    // field 0 (with the winding phase) is loaded directly; field f + 1 comes
-    // by cp.async into the buffer the transform of field f left free, while
-    // field f is stored
-    cx_load<T, N, NB>(A, valid, [&](int t) {
-        C2<T> v = load_field(a.in[0], g0 + t);
-        if (w != 0) {
-            // phase -2*pi*y*w/ny of line L0 + t/N (tevol_driven_cluster.m:139)
-            const int y = (L0 + t / N) % a.ny;
-            const long long q = ((long long)y * w) % a.ny;
-            double sn, cs;
-            sincospi(-2.0 * (double)q / (double)a.ny, &sn, &cs);
-            v = mk2<T>(v.x * (T)cs - v.y * (T)sn, v.x * (T)sn + v.y * (T)cs);
-        }
-        return v;
-    });
-    __syncthreads();
-    int src = A;
-    for (int f = 0; f < a.nf; ++f) {
-        const int X = ct_fft<T, N, NB, -1>(src, src == A ? B : A, R);
-        const int F = (X == A) ? B : A;
-        if (f + 1 < a.nf) cx_load_field_async<T, N, NB>(F, valid, g0, a.in[f + 1]);
-        cp_commit();
-        C2<T> *spec = a.spec[f];
-        cx_store<T, N, NB>(X, valid, [&](int t, C2<T> v) {
-            if (filt_col_live(t % N, a.dead0, a.dead1)) spec[g0 + t] = v;
-        });
-        cp_wait<0>();
-        __syncthreads();
-        src = F;
-    }
-}
-
-template <typename T, int N>
-__global__ void HQT_CT_BOUNDS k_y_filt_c(YFiltArgs<T> a) {
-    constexpr int TX = ct_lines_y(N, 6, sizeof(C2<T>));
-    constexpr int NB = 3 * TX;  // up to three fields of TX columns
-    const int x0 = blockIdx.x * TX;
-    const int valid = min(TX, a.nx - x0);
-    const long long zoff = (long long)blockIdx.y * a.ny * a.nx + x0;
-    constexpr int R = 0, A = N, B = N + NB * N;
-    bool live = false;
-    for (int b = 0; b < valid; ++b) live = live || filt_col_live(x0 + b, a.dead0, a.dead1);
-    if (!live) return;  // every column filtered out
-    ct_load_roots<T, N>(R, a.roots);
-    pdl_wait();
-    {
-        const CtView<T, N> s = ctv<T, N>(A);
-        for (int t = threadIdx.x; t < N * NB; t += ct_threads<T, N, NB>()) {
-            const int bb = t % NB, y = t / NB;
-            const int f = bb / TX, b = bb % TX;
-            s[t] = (f < a.nf && b < valid) ? a.spec[f][zoff + (long long)y * a.nx + b]
-                                           : mk2<T>(T(0), T(0));
-        }
-    }
-    __syncthreads();
-    const int X = ct_fft<T, N, NB, -1>(A, B, R);
-    {
-        const CtView<T, N> s = ctv<T, N>(X);
-        for (int t = threadIdx.x; t < N * NB; t += ct_threads<T, N, NB>()) {
-            const int bb = t % NB, ky = t / NB;
-            const int kx = x0 + min(bb % TX, valid - 1);
-            const int kxm = (a.nx - kx) % a.nx, kym = (N - ky) % N;
-            const T wgt = T(0.5) * (a.mx[kx] * a.my[ky] + a.mx[kxm] * a.my[kym]) * a.scale;
-            s[t] = wgt * s[t];
-        }
-    }
-    __syncthreads();
-    const int r = ct_fft<T, N, NB, +1>(X, (X == A) ? B : A, R);
-    const CtView<T, N> s = ctv<T, N>(r);
-    for (int t = threadIdx.x; t < N * NB; t += ct_threads<T, N, NB>()) {
-        const int bb = t % NB, y = t / NB;
-        const int f = bb / TX, b = bb % TX;
-        if (f < a.nf && b < valid) a.spec[f][zoff + (long long)y * a.nx + b] = s[t];
-    }
-}
-
-template <typename T, int N>
-__global__ void HQT_CT_BOUNDS k_x_filt_inv_c(XFiltInvArgs<T> a) {
-    constexpr int NB = ct_lines(N, 2, sizeof(C2<T>));
-    const int L0 = blockIdx.x * NB;
-    const int valid = min(NB, a.nlines - L0);
-    constexpr int R = 0, A = N, B = N + NB * N;
-    const long long g0 = (long long)L0 * N;
-    ct_load_roots<T, N>(R, a.roots);
-    pdl_wait();
-    __shared__ int bad;
-    if (threadIdx.x == 0) bad = 0;
-    int mybad = 0;
-    // spectrum f by cp.async, the weight-zeroed columns as zero; spectrum
-    // f + 1 comes into the buffer the transform of field f left free while
-    // field f is stored
-    auto fetch = [&](int buf, int f) {
-        const CtView<T, N> s = ctv<T, N>(buf);
-        const C2<T> *spec = a.spec[f];
-        for (int t = threadIdx.x; t < N * NB; t += ct_threads<T, N, NB>()) {
-            const int b = t / N, e = t - b * N;
-            C2<T> &d = s[e * NB + b];
-            if (b < valid && filt_col_live(e, a.dead0, a.dead1))
-                cp_async<sizeof(C2<T>)>(&d, spec + g0 + t);
-            else
-                d = mk2<T>(T(0), T(0));
-        }
-    };
-    fetch(A, 0);
-    cp_commit();
-    cp_wait<0>();
-    __syncthreads();
-    int src = A;
-    for (int f = 0; f < a.nf; ++f) {
-        const int X = ct_fft<T, N, NB, +1>(src, src == A ? B : A, R);
-        const int F = (X == A) ? B : A;
-        if (f + 1 < a.nf) fetch(F, f + 1);
-        cp_commit();
-        cx_store<T, N, NB>(X, valid, [&](int t, C2<T> v) {
-            if (!(isfinite(v.x) && isfinite(v.y))) mybad = 1;
-            store_field(a.out[f], g0 + t, v);
-        });
-        cp_wait<0>();
-        __syncthreads();
-        src = F;
-    }
-    if (a.st) {
-        if (mybad) bad = 1;
-        __syncthreads();
-        if (threadIdx.x == 0 && bad)
-            atomicMin(reinterpret_cast<unsigned long long *>(&a.st->first_bad_step),
-                      (unsigned long long)(a.st->step + 1));
     }
 }
 

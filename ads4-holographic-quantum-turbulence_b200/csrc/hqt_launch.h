@@ -58,12 +58,23 @@ cudaError_t launch_y_rhs_f(const YRhsArgs<float> &a, dim3 grid, size_t smem, cud
 cudaError_t launch_x_d1_f(const XD1Args<float> &a, int grid, size_t smem, cudaStream_t s);
 cudaError_t launch_y_d1_f(const YD1Args<float> &a, dim3 grid, size_t smem, cudaStream_t s);
 
-// Compile-time line lengths (hqt_c<N>.cu): kinds of pass kernel.
+// Kinds of line pass.
 enum CtKind {
-    CT_X_RHS, CT_Y_RHS, CT_X_D1, CT_Y_D1, CT_FX_FWD, CT_FY, CT_FX_INV,
+    CT_X_RHS, CT_Y_RHS, CT_X_D1, CT_Y_D1, CT_FX_FWD, CT_FY, CT_FX_INV, CT_Y_FWD,
     // FP32 line passes of the mixed-precision stage (args of type <float>)
     CT_X_RHS_F, CT_Y_RHS_F, CT_X_D1_F, CT_Y_D1_F
 };
+// FP64 in-place line passes (hqt_line_passes.cuh) of a compile-time length
+// (hqt_c<N>.cu); nsl: z slices
+template <int N> cudaError_t ct_init64(int max_smem);
+template <int N> cudaError_t ct_launch_x64(int kind, const void *args, cudaStream_t s);
+template <int N> cudaError_t ct_launch_y64(int kind, const void *args, int nsl, cudaStream_t s);
+// ... and of a length with a runtime plan (lplan).
+cudaError_t line_rt_init_x(int max_smem);
+cudaError_t line_rt_init_y(int max_smem);
+cudaError_t line_rt_launch_x(int kind, const void *args, cudaStream_t s);
+cudaError_t line_rt_launch_y(int kind, const void *args, int nsl, cudaStream_t s);
+// FP32 Stockham passes of a compile-time length
 template <int N> cudaError_t ct_init(const double *tab_cos, const double *tab_sin, int ntab,
                                      const double *big_cos, const double *big_sin, int nbig,
                                      int max_smem);
@@ -72,6 +83,7 @@ cudaError_t ct_launch(int kind, const void *args, dim3 grid, size_t smem, cudaSt
 
 // Line lengths with a prime-factor tensor-core engine (hqt_pfa.cuh): 301 = 7*43.
 constexpr bool pfa_length(int n) { return n == 301; }
+cudaError_t pfa_init_301();
 // Launch pass `kind` (CT_X_RHS, ...) on it: lines of kPfaLines per one-warp
 // block.  `nlines`: lines of an x pass; z slices of a y pass.
 cudaError_t pfa_launch_301(int kind, const void *args, int nlines, cudaStream_t s);
@@ -96,8 +108,10 @@ cudaError_t z_misc(const ZColArgs<double> &a, const ZHost &h, int grid, int thre
 // Compile-time column lengths compiled into the library; a run uses the
 // smallest >= nz.
 #define HQT_NZP_LIST(X) X(8) X(12) X(16) X(17) X(21) X(25) X(33)
-// Line lengths with compile-time transforms; other lengths use hqt_fft.cuh.
-#define HQT_CN_LIST(X) X(33) X(64) X(128) X(192) X(256) X(301) X(512) X(1024)
+// Line lengths with compile-time passes: FP64 in place (HQT_LN_LIST), FP32
+// also 301 = 7*43.
+#define HQT_LN_LIST(X) X(33) X(64) X(128) X(192) X(256) X(512) X(1024)
+#define HQT_CN_LIST(X) HQT_LN_LIST(X) X(301)
 
 namespace hqt {
 #define HQT_ZDECL(N)                                                                       \
@@ -121,4 +135,10 @@ HQT_NZP_LIST(HQT_ZDECL)
     template <> cudaError_t ct_launch<N>(int, const void *, dim3, size_t, cudaStream_t);
 HQT_CN_LIST(HQT_CDECL)
 #undef HQT_CDECL
+#define HQT_LDECL(N)                                                                       \
+    template <> cudaError_t ct_init64<N>(int);                                             \
+    template <> cudaError_t ct_launch_x64<N>(int, const void *, cudaStream_t);             \
+    template <> cudaError_t ct_launch_y64<N>(int, const void *, int, cudaStream_t);
+HQT_LN_LIST(HQT_LDECL)
+#undef HQT_LDECL
 }  // namespace hqt

@@ -1,0 +1,634 @@
+// hqt_line.cuh -- in-place mixed-radix line transforms: forward decimation in
+// frequency, inverse decimation in time, on NB lines held in shared memory.
+//
+// The passes of a line of n = R0 R1 .. R(m-1) points work on blocks of
+// L_p = n/(R0..R(p-1)) elements with stride s_p = L_p/R_p: butterfly (blk, j)
+// takes elements blk L_p + j + r s_p (r < R_p), transforms over r in
+// registers, multiplies by w_{L_p}^{j k} and writes back where it read.  The
+// spectrum is left in digit-reversed order; the inverse runs the same
+// butterflies backwards with conjugate twiddles and ends in natural order, so
+// nothing is ever reordered.  What follows from that, against a ping-pong
+// (Stockham) transform:
+//   - the first pass reads global memory into registers and the last inverse
+//     pass writes global memory from registers: no staging passes;
+//   - the last forward pass, the multiplier of a derivative (or the filter's
+//     weight) and the first inverse pass are one pass: a thread holds the
+//     spectrum of its butterfly and writes one product per derivative;
+//   - one buffer per line and derivative instead of three, no twiddle table
+//     in shared memory, a barrier per pass.
+// A first and a second derivative of a three-pass line move 12 line lengths
+// through shared memory (25 in the Stockham form): W | RW | R WW | RW RW | R R.
+// Twiddles come from a table packed per pass as [k][j], so that consecutive
+// butterflies read consecutive entries (through L1).
+//
+// Shared-memory layout: element e of line b at (e << nbl) + b, with an XOR of
+// e's low bits where n is a multiple of 8 (the strided rows of the last
+// forward pass otherwise fall on the same banks); threads run over b first, so
+// a warp touches 2^nbl lines by 32 >> nbl consecutive butterflies.
+//
+// The plan is a compile-time constant (SGeo) for the lengths of HQT_CN_LIST
+// and a kernel argument (RGeo, divisions by multiply-high) for every other
+// length whose prime factors are at most 13.
+#pragma once
+#include <type_traits>
+
+#include "hqt_args.h"
+#include "hqt_dev.cuh"
+
+namespace hqt {
+
+// cos(2 pi k / R) of the radices' real-pair forms, to 20 digits (folded to immediates
+// once k is known).
+__host__ __device__ constexpr double lf_cos(int R, int k) {
+    switch (32 * R + k) {
+        case 97: return -0.5;
+        case 98: return -0.5;
+        case 161: return 0.3090169943749474241;
+        case 162: return -0.8090169943749474241;
+        case 163: return -0.8090169943749474241;
+        case 164: return 0.3090169943749474241;
+        case 225: return 0.62348980185873353053;
+        case 226: return -0.22252093395631440429;
+        case 227: return -0.90096886790241912624;
+        case 228: return -0.90096886790241912624;
+        case 229: return -0.22252093395631440429;
+        case 230: return 0.62348980185873353053;
+        case 257: return 0.7071067811865475244;
+        case 258: return 0.0;
+        case 259: return -0.7071067811865475244;
+        case 260: return -1.0;
+        case 261: return -0.7071067811865475244;
+        case 262: return 0.0;
+        case 263: return 0.7071067811865475244;
+        case 289: return 0.7660444431189780352;
+        case 290: return 0.17364817766693034885;
+        case 291: return -0.5;
+        case 292: return -0.93969262078590838405;
+        case 293: return -0.93969262078590838405;
+        case 294: return -0.5;
+        case 295: return 0.17364817766693034885;
+        case 296: return 0.7660444431189780352;
+        case 353: return 0.84125353283118116886;
+        case 354: return 0.41541501300188642553;
+        case 355: return -0.14231483827328514044;
+        case 356: return -0.65486073394528506406;
+        case 357: return -0.95949297361449738989;
+        case 358: return -0.95949297361449738989;
+        case 359: return -0.65486073394528506406;
+        case 360: return -0.14231483827328514044;
+        case 361: return 0.41541501300188642553;
+        case 362: return 0.84125353283118116886;
+        case 417: return 0.8854560256532098959;
+        case 418: return 0.56806474673115580251;
+        case 419: return 0.12053668025532305335;
+        case 420: return -0.35460488704253562597;
+        case 421: return -0.74851074817110109863;
+        case 422: return -0.97094181742605202716;
+        case 423: return -0.97094181742605202716;
+        case 424: return -0.74851074817110109863;
+        case 425: return -0.35460488704253562597;
+        case 426: return 0.12053668025532305335;
+        case 427: return 0.56806474673115580251;
+        case 428: return 0.8854560256532098959;
+        case 513: return 0.92387953251128675613;
+        case 514: return 0.7071067811865475244;
+        case 515: return 0.38268343236508977173;
+        case 516: return 0.0;
+        case 517: return -0.38268343236508977173;
+        case 518: return -0.7071067811865475244;
+        case 519: return -0.92387953251128675613;
+        case 520: return -1.0;
+        case 521: return -0.92387953251128675613;
+        case 522: return -0.7071067811865475244;
+        case 523: return -0.38268343236508977173;
+        case 524: return 0.0;
+        case 525: return 0.38268343236508977173;
+        case 526: return 0.7071067811865475244;
+        case 527: return 0.92387953251128675613;
+        default: return 1.0;
+    }
+}
+__host__ __device__ constexpr double lf_sin(int R, int k) {
+    switch (32 * R + k) {
+        case 97: return 0.86602540378443864676;
+        case 98: return -0.86602540378443864676;
+        case 161: return 0.95105651629515357212;
+        case 162: return 0.58778525229247312917;
+        case 163: return -0.58778525229247312917;
+        case 164: return -0.95105651629515357212;
+        case 225: return 0.78183148246802980871;
+        case 226: return 0.97492791218182360702;
+        case 227: return 0.43388373911755812048;
+        case 228: return -0.43388373911755812048;
+        case 229: return -0.97492791218182360702;
+        case 230: return -0.78183148246802980871;
+        case 257: return 0.7071067811865475244;
+        case 258: return 1.0;
+        case 259: return 0.7071067811865475244;
+        case 260: return 0.0;
+        case 261: return -0.7071067811865475244;
+        case 262: return -1.0;
+        case 263: return -0.7071067811865475244;
+        case 289: return 0.64278760968653932632;
+        case 290: return 0.98480775301220805937;
+        case 291: return 0.86602540378443864676;
+        case 292: return 0.34202014332566873304;
+        case 293: return -0.34202014332566873304;
+        case 294: return -0.86602540378443864676;
+        case 295: return -0.98480775301220805937;
+        case 296: return -0.64278760968653932632;
+        case 353: return 0.54064081745559758211;
+        case 354: return 0.90963199535451837141;
+        case 355: return 0.98982144188093273238;
+        case 356: return 0.75574957435425828377;
+        case 357: return 0.28173255684142969771;
+        case 358: return -0.28173255684142969771;
+        case 359: return -0.75574957435425828377;
+        case 360: return -0.98982144188093273238;
+        case 361: return -0.90963199535451837141;
+        case 362: return -0.54064081745559758211;
+        case 417: return 0.46472317204376854566;
+        case 418: return 0.82298386589365639458;
+        case 419: return 0.9927088740980539928;
+        case 420: return 0.93501624268541482344;
+        case 421: return 0.66312265824079520238;
+        case 422: return 0.23931566428755776715;
+        case 423: return -0.23931566428755776715;
+        case 424: return -0.66312265824079520238;
+        case 425: return -0.93501624268541482344;
+        case 426: return -0.9927088740980539928;
+        case 427: return -0.82298386589365639458;
+        case 428: return -0.46472317204376854566;
+        case 513: return 0.38268343236508977173;
+        case 514: return 0.7071067811865475244;
+        case 515: return 0.92387953251128675613;
+        case 516: return 1.0;
+        case 517: return 0.92387953251128675613;
+        case 518: return 0.7071067811865475244;
+        case 519: return 0.38268343236508977173;
+        case 520: return 0.0;
+        case 521: return -0.38268343236508977173;
+        case 522: return -0.7071067811865475244;
+        case 523: return -0.92387953251128675613;
+        case 524: return -1.0;
+        case 525: return -0.92387953251128675613;
+        case 526: return -0.7071067811865475244;
+        case 527: return -0.38268343236508977173;
+        default: return 0.0;
+    }
+}
+
+template <typename T> __device__ __forceinline__ C2<T> lf_cmul(C2<T> a, C2<T> w) {
+    return mk2<T>(a.x * w.x - a.y * w.y, a.x * w.y + a.y * w.x);
+}
+template <typename T> __device__ __forceinline__ C2<T> lf_cmulc(C2<T> a, C2<T> w) {  // a conj(w)
+    return mk2<T>(a.x * w.x + a.y * w.y, a.y * w.x - a.x * w.y);
+}
+
+// ---- R-point DFTs in registers, natural order in and out ------------------
+template <typename T, int R, int SIGN> struct LDft;
+template <typename T, int R, int SIGN> __device__ __forceinline__ void ldft(C2<T> (&v)[R]) {
+    LDft<T, R, SIGN>::run(v);
+}
+// a * e^{SIGN 2 pi i k/R}
+template <typename T, int R, int SIGN> __device__ __forceinline__ C2<T> lrot(C2<T> a, int k) {
+    const T c = (T)lf_cos(R, k), s = (T)(SIGN * lf_sin(R, k));
+    return mk2<T>(a.x * c - a.y * s, a.x * s + a.y * c);
+}
+template <typename T, int SIGN> __device__ __forceinline__ C2<T> lmuli(C2<T> a) {  // SIGN i a
+    return SIGN < 0 ? mk2<T>(a.y, -a.x) : mk2<T>(-a.y, a.x);
+}
+
+template <typename T, int SIGN> struct LDft<T, 2, SIGN> {
+    static __device__ __forceinline__ void run(C2<T> (&v)[2]) {
+        const C2<T> a = v[0], b = v[1];
+        v[0] = a + b;
+        v[1] = a - b;
+    }
+};
+template <typename T, int SIGN> struct LDft<T, 4, SIGN> {
+    static __device__ __forceinline__ void run(C2<T> (&v)[4]) {
+        const C2<T> a = v[0] + v[2], b = v[0] - v[2], c = v[1] + v[3];
+        const C2<T> d = lmuli<T, SIGN>(v[1] - v[3]);
+        v[0] = a + c;
+        v[1] = b + d;
+        v[2] = a - c;
+        v[3] = b - d;
+    }
+};
+// R = 2 H for power-of-two H: two H-point DFTs of the even and odd elements
+template <typename T, int R, int SIGN> struct LDftPow2 {
+    static __device__ __forceinline__ void run(C2<T> (&v)[R]) {
+        constexpr int H = R / 2;
+        C2<T> e[H], o[H];
+#pragma unroll
+        for (int i = 0; i < H; ++i) {
+            e[i] = v[2 * i];
+            o[i] = v[2 * i + 1];
+        }
+        ldft<T, H, SIGN>(e);
+        ldft<T, H, SIGN>(o);
+#pragma unroll
+        for (int k = 0; k < H; ++k) {
+            C2<T> t;
+            if (k == 0) {
+                t = o[0];
+            } else if (4 * k == R) {
+                t = lmuli<T, SIGN>(o[k]);
+            } else if (8 * k == R || 8 * k == 3 * R) {
+                // +-(1 + SIGN i)/sqrt(2) forms: two adds, two products
+                const T h = (T)0.70710678118654752440;
+                const C2<T> q = lmuli<T, SIGN>(o[k]);
+                t = 8 * k == R ? mk2<T>(h * (o[k].x + q.x), h * (o[k].y + q.y))
+                               : mk2<T>(h * (q.x - o[k].x), h * (q.y - o[k].y));
+            } else {
+                t = lrot<T, R, SIGN>(o[k], k);
+            }
+            v[k] = e[k] + t;
+            v[k + H] = e[k] - t;
+        }
+    }
+};
+template <typename T, int SIGN> struct LDft<T, 8, SIGN> : LDftPow2<T, 8, SIGN> {};
+template <typename T, int SIGN> struct LDft<T, 16, SIGN> : LDftPow2<T, 16, SIGN> {};
+// odd prime R in the real-pair form: a_j = x_j + x_{R-j}, b_j = x_j - x_{R-j}
+template <typename T, int R, int SIGN> struct LDftOdd {
+    static __device__ __forceinline__ void run(C2<T> (&v)[R]) {
+        constexpr int M = (R - 1) / 2;
+        C2<T> a[M + 1], b[M + 1];
+#pragma unroll
+        for (int j = 1; j <= M; ++j) {
+            a[j] = v[j] + v[R - j];
+            b[j] = v[j] - v[R - j];
+        }
+        const C2<T> x0 = v[0];
+#pragma unroll
+        for (int j = 1; j <= M; ++j) v[0] = v[0] + a[j];
+#pragma unroll
+        for (int k = 1; k <= M; ++k) {
+            C2<T> p = x0, q = mk2<T>(T(0), T(0));
+#pragma unroll
+            for (int j = 1; j <= M; ++j) {
+                const T c = (T)lf_cos(R, (j * k) % R), s = (T)lf_sin(R, (j * k) % R);
+                p = mk2<T>(fma(a[j].x, c, p.x), fma(a[j].y, c, p.y));
+                q = mk2<T>(fma(b[j].x, s, q.x), fma(b[j].y, s, q.y));
+            }
+            q = lmuli<T, SIGN>(q);
+            v[k] = p + q;
+            v[R - k] = p - q;
+        }
+    }
+};
+template <typename T, int SIGN> struct LDft<T, 3, SIGN> : LDftOdd<T, 3, SIGN> {};
+template <typename T, int SIGN> struct LDft<T, 5, SIGN> : LDftOdd<T, 5, SIGN> {};
+template <typename T, int SIGN> struct LDft<T, 7, SIGN> : LDftOdd<T, 7, SIGN> {};
+template <typename T, int SIGN> struct LDft<T, 11, SIGN> : LDftOdd<T, 11, SIGN> {};
+template <typename T, int SIGN> struct LDft<T, 13, SIGN> : LDftOdd<T, 13, SIGN> {};
+template <typename T, int SIGN> struct LDft<T, 9, SIGN> {
+    static __device__ __forceinline__ void run(C2<T> (&v)[9]) {
+        C2<T> u[3][3];
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+            C2<T> w[3] = {v[i], v[i + 3], v[i + 6]};
+            ldft<T, 3, SIGN>(w);
+#pragma unroll
+            for (int k = 0; k < 3; ++k) u[k][i] = i * k == 0 ? w[k] : lrot<T, 9, SIGN>(w[k], i * k);
+        }
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            ldft<T, 3, SIGN>(u[k]);
+#pragma unroll
+            for (int m = 0; m < 3; ++m) v[k + 3 * m] = u[k][m];
+        }
+    }
+};
+__host__ __device__ constexpr int lf_modinv(int a, int m) {
+    for (int x = 1; x < m; ++x)
+        if ((a * x) % m == 1) return x;
+    return 1;
+}
+// R = P Q with gcd(P, Q) = 1: P- and Q-point DFTs without twiddles
+template <typename T, int P, int Q, int SIGN> struct LDftPrimeFactor {
+    static __device__ __forceinline__ void run(C2<T> (&v)[P * Q]) {
+        constexpr int R = P * Q, QI = lf_modinv(Q % P, P), PI = lf_modinv(P % Q, Q);
+        C2<T> u[P][Q];
+#pragma unroll
+        for (int a = 0; a < P; ++a) {
+#pragma unroll
+            for (int b = 0; b < Q; ++b) u[a][b] = v[(Q * a + P * b) % R];
+            ldft<T, Q, SIGN>(u[a]);
+        }
+#pragma unroll
+        for (int b = 0; b < Q; ++b) {
+            C2<T> w[P];
+#pragma unroll
+            for (int a = 0; a < P; ++a) w[a] = u[a][b];
+            ldft<T, P, SIGN>(w);
+#pragma unroll
+            for (int a = 0; a < P; ++a) v[(Q * QI * a + P * PI * b) % R] = w[a];
+        }
+    }
+};
+template <typename T, int SIGN> struct LDft<T, 6, SIGN> : LDftPrimeFactor<T, 2, 3, SIGN> {};
+template <typename T, int SIGN> struct LDft<T, 10, SIGN> : LDftPrimeFactor<T, 2, 5, SIGN> {};
+template <typename T, int SIGN> struct LDft<T, 12, SIGN> : LDftPrimeFactor<T, 4, 3, SIGN> {};
+
+// ---- the transform --------------------------------------------------------
+// NT threads of the block work on the lines; A and B are its two buffers.
+template <typename T, class G> struct LineEng {
+    using C = C2<T>;
+    // a runtime plan stays in the kernel's parameters (its dynamic indexing
+    // would put a copy on the stack)
+    std::conditional_t<G::kStatic, G, const RGeo &> g;
+    C *A, *B;
+    const C *tw;
+    const int *freq, *posn;  // RGeo only: digit reversal of blocks and modes
+
+    __device__ __forceinline__ LineEng(const LineTab<T> &t)
+        : g(t.g), A(sptr<T>(0)), B(sptr<T>(0) + (g.n() << g.nbl())), tw(t.tw), freq(t.freq),
+          posn(t.pos) {}
+
+    // bank swizzle of row e (rows stay inside their group of 8)
+    __device__ __forceinline__ int row(int e) const {
+        const int m = g.template swz<T>();
+        if (G::kStatic && m == 0) return e << g.nbl();
+        return (e ^ (((e >> 3) ^ (e >> 6) ^ (e >> 9)) & m)) << g.nbl();
+    }
+    __device__ __forceinline__ static int div(unsigned x, int s, unsigned mg) {
+        if constexpr (G::kStatic) return (int)x / s;
+        return s == 1 ? (int)x : (int)__umulhi(x, mg);
+    }
+    // f(b, jj) for every butterfly jj < n/R of every line b
+    template <int R, typename F> __device__ __forceinline__ void each(F f) const {
+        const int cnt = (g.n() / R) << g.nbl();
+#pragma unroll 1
+        for (int t = threadIdx.x; t < cnt; t += g.threads())
+            f(t & ((1 << g.nbl()) - 1), t >> g.nbl());
+    }
+    // f(integral_constant<int, R>, stride, magic, twiddle offset) of pass p
+    template <int P, typename F> __device__ __forceinline__ void at_static(F f) const {
+        constexpr LPlan pl = lplan(G::N);
+        constexpr int R = pl.R[P], s = pl.s[P], o = pl.tw[P];
+        f(std::integral_constant<int, R>{}, s, 0u, o);
+    }
+    template <typename F> __device__ __forceinline__ void at(int p, F f) const {
+        const int s = g.s(p), o = g.tw(p);
+        const unsigned mg = g.mg(p);
+        switch (g.R(p)) {
+#define HQT_LR(RR) \
+    case RR: f(std::integral_constant<int, RR>{}, s, mg, o); break;
+            HQT_LR(2) HQT_LR(3) HQT_LR(4) HQT_LR(5) HQT_LR(6) HQT_LR(7) HQT_LR(8) HQT_LR(9)
+            HQT_LR(10) HQT_LR(11) HQT_LR(12) HQT_LR(13)
+#undef HQT_LR
+        }
+    }
+    // pass `P` of the plan: first, last or any of the ones between
+    template <typename F> __device__ __forceinline__ void at_first(F f) const {
+        if constexpr (G::kStatic)
+            at_static<0>(f);
+        else
+            at(0, f);
+    }
+    template <typename F> __device__ __forceinline__ void at_last(F f) const {
+        if constexpr (G::kStatic)
+            at_static<G::np() - 1>(f);
+        else
+            at(g.np() - 1, f);
+    }
+    // the passes between, in order (+1) or backwards (-1), a barrier after each
+    template <int DIR, int P = 1, typename F> __device__ __forceinline__ void at_mid(F f) const {
+        if constexpr (G::kStatic) {
+            if constexpr (P < G::np() - 1) {
+                at_static<(DIR > 0 ? P : G::np() - 1 - P)>(f);
+                __syncthreads();
+                at_mid<DIR, P + 1>(f);
+            }
+        } else {
+            const int np = g.np();
+#pragma unroll 1
+            for (int i = 1; i < np - 1; ++i) {
+                at(DIR > 0 ? i : np - 1 - i, f);
+                __syncthreads();
+            }
+        }
+    }
+
+    // butterfly of one pass in place: forward (with twiddles) or inverse
+    template <int R, int SIGN>
+    __device__ __forceinline__ void step(C *X, int s, unsigned mg, int o) const {
+        each<R>([&](int b, int jj) {
+            const int blk = div(jj, s, mg), j = jj - blk * s, e0 = blk * s * R + j;
+            C v[R];
+#pragma unroll
+            for (int r = 0; r < R; ++r) v[r] = X[row(e0 + r * s) + b];
+            if (SIGN > 0) {
+#pragma unroll
+                for (int r = 1; r < R; ++r)
+                    v[r] = lf_cmulc<T>(v[r], __ldg(tw + o + (r - 1) * s + j));
+            }
+            ldft<T, R, SIGN>(v);
+            if (SIGN < 0) {
+#pragma unroll
+                for (int r = 1; r < R; ++r)
+                    v[r] = lf_cmul<T>(v[r], __ldg(tw + o + (r - 1) * s + j));
+            }
+#pragma unroll
+            for (int r = 0; r < R; ++r) X[row(e0 + r * s) + b] = v[r];
+        });
+    }
+
+    // first forward pass from ld(b, e) into X; then the middle passes
+    template <typename Ld> __device__ __forceinline__ void first(C *X, Ld ld) const {
+        at_first([&](auto rc, int s, unsigned, int o) {
+            constexpr int R = decltype(rc)::value;
+            each<R>([&](int b, int j) {
+                C v[R];
+#pragma unroll
+                for (int r = 0; r < R; ++r) v[r] = ld(b, j + r * s);
+                ldft<T, R, -1>(v);
+#pragma unroll
+                for (int r = 1; r < R; ++r)
+                    v[r] = lf_cmul<T>(v[r], __ldg(tw + o + (r - 1) * s + j));
+#pragma unroll
+                for (int r = 0; r < R; ++r) X[row(j + r * s) + b] = v[r];
+            });
+        });
+    }
+    // middle passes of nx buffers (A, then B); starts and ends at a barrier
+    __device__ __forceinline__ void forward_mid(int nx) const {
+        __syncthreads();
+        at_mid<1>([&](auto rc, int s, unsigned mg, int o) {
+#pragma unroll 1
+            for (int x = 0; x < nx; ++x) step<decltype(rc)::value, -1>(x ? B : A, s, mg, o);
+        });
+    }
+    __device__ __forceinline__ void inverse_mid(int nx) const {
+        __syncthreads();
+        at_mid<-1>([&](auto rc, int s, unsigned mg, int o) {
+#pragma unroll 1
+            for (int x = 0; x < nx; ++x) step<decltype(rc)::value, 1>(x ? B : A, s, mg, o);
+        });
+    }
+    template <int P> __device__ __forceinline__ static int mode0_static(int rem, int mult) {
+        constexpr LPlan pl = lplan(G::N);
+        if constexpr (P < pl.np - 1) {
+            constexpr int w = pl.s[P] / pl.R[pl.np - 1], R = pl.R[P];
+            return (rem / w) * mult + mode0_static<P + 1>(rem % w, mult * R);
+        }
+        return 0;
+    }
+    template <int P> __device__ __forceinline__ static int pos_static(int k) {
+        constexpr LPlan pl = lplan(G::N);
+        if constexpr (P < pl.np) {
+            constexpr int R = pl.R[P], s = pl.s[P];
+            return (k % R) * s + pos_static<P + 1>(k / R);
+        }
+        return 0;
+    }
+    // mode number of output km of the last pass's butterfly blk: base + km n/R
+    __device__ __forceinline__ int mode0(int blk) const {
+        if constexpr (G::kStatic) {
+            return mode0_static<0>(blk, 1);
+        } else {
+            return __ldg(freq + blk);
+        }
+    }
+    // row of mode k
+    __device__ __forceinline__ int pos(int k) const {
+        if constexpr (G::kStatic) {
+            return pos_static<0>(k);
+        } else {
+            return __ldg(posn + k);
+        }
+    }
+    __device__ __forceinline__ T wave(int k) const {  // signed, Nyquist 0
+        const int k2 = 2 * k, n = g.n();
+        return (T)(k2 < n ? k : (k2 > n ? k - n : 0));
+    }
+    // Last forward pass of X, f(v, b, k0, step) on the spectrum of a butterfly
+    // (v[i] = mode k0 + i step), which writes what it wants with put().
+    template <int R> __device__ __forceinline__ void put(C *X, int b, int blk, C (&v)[R]) const {
+        ldft<T, R, 1>(v);
+#pragma unroll
+        for (int r = 0; r < R; ++r) X[row(blk * R + r) + b] = v[r];
+    }
+    template <typename F> __device__ __forceinline__ void middle(const C *X, F f) const {
+        at_last([&](auto rc, int, unsigned, int) {
+            constexpr int R = decltype(rc)::value;
+            const int st = g.n() / R;
+            each<R>([&](int b, int blk) {
+                C v[R];
+#pragma unroll
+                for (int r = 0; r < R; ++r) v[r] = X[row(blk * R + r) + b];
+                ldft<T, R, -1>(v);
+                f(v, b, blk, mode0(blk), st);
+            });
+        });
+    }
+    // A <- d A, B <- d^2 A (spectra times i s1 k and s2 k^2), after forward_mid
+    __device__ __forceinline__ void middle_deriv12(T s1, T s2) const {
+        middle(A, [&](auto &v, int b, int blk, int k0, int st) {
+            constexpr int R = sizeof(v) / sizeof(C);
+            C u[R];
+#pragma unroll
+            for (int i = 0; i < R; ++i) {
+                const T m = s1 * wave(k0 + i * st);
+                u[i] = mk2<T>(-m * v[i].y, m * v[i].x);
+            }
+            put<R>(A, b, blk, u);
+#pragma unroll
+            for (int i = 0; i < R; ++i) {
+                const T k = wave(k0 + i * st), m = s2 * k * k;
+                v[i] = mk2<T>(m * v[i].x, m * v[i].y);
+            }
+            put<R>(B, b, blk, v);
+        });
+    }
+    __device__ __forceinline__ void middle_deriv1(C *X, T s1) const {
+        middle(X, [&](auto &v, int b, int blk, int k0, int st) {
+            constexpr int R = sizeof(v) / sizeof(C);
+#pragma unroll
+            for (int i = 0; i < R; ++i) {
+                const T m = s1 * wave(k0 + i * st);
+                v[i] = mk2<T>(-m * v[i].y, m * v[i].x);
+            }
+            put<R>(X, b, blk, v);
+        });
+    }
+    // X <- (s1 k - s2 k^2) X
+    __device__ __forceinline__ void middle_deriv_mix(C *X, T s1, T s2) const {
+        middle(X, [&](auto &v, int b, int blk, int k0, int st) {
+            constexpr int R = sizeof(v) / sizeof(C);
+#pragma unroll
+            for (int i = 0; i < R; ++i) {
+                const T k = wave(k0 + i * st), m = s1 * k - s2 * k * k;
+                v[i] = mk2<T>(m * v[i].x, m * v[i].y);
+            }
+            put<R>(X, b, blk, v);
+        });
+    }
+    // last inverse pass of X: st(b, e, v) for every element
+    template <typename St> __device__ __forceinline__ void last(const C *X, St st) const {
+        last(X, [](int, int) { return 0; }, [&](int b, int e, C v, int) { st(b, e, v); });
+    }
+    // ... with x = get(b, e) read for up to 8 elements ahead of their stores (a
+    // read after a store could not move ahead of it)
+    template <typename Get, typename St>
+    __device__ __forceinline__ void last(const C *X, Get get, St st) const {
+        at_first([&](auto rc, int s, unsigned, int o) {
+            constexpr int R = decltype(rc)::value, H = R > 8 ? 4 : R;
+            each<R>([&](int b, int j) {
+                C v[R];
+#pragma unroll
+                for (int r = 0; r < R; ++r) v[r] = X[row(j + r * s) + b];
+#pragma unroll
+                for (int r = 1; r < R; ++r)
+                    v[r] = lf_cmulc<T>(v[r], __ldg(tw + o + (r - 1) * s + j));
+                ldft<T, R, 1>(v);
+#pragma unroll
+                for (int r0 = 0; r0 < R; r0 += H) {
+                    decltype(get(0, 0)) x[H];
+#pragma unroll
+                    for (int r = 0; r < H; ++r)
+                        if (r0 + r < R) x[r] = get(b, j + (r0 + r) * s);
+#pragma unroll
+                    for (int r = 0; r < H; ++r)
+                        if (r0 + r < R) st(b, j + (r0 + r) * s, v[r0 + r], x[r]);
+                }
+            });
+        });
+    }
+    // f(b, k) over all modes of all lines, b fastest
+    template <typename F> __device__ __forceinline__ void modes(F f) const {
+        const int cnt = g.n() << g.nbl();
+#pragma unroll 4
+        for (int t = threadIdx.x; t < cnt; t += g.threads())
+            f(t & ((1 << g.nbl()) - 1), t >> g.nbl());
+    }
+    // forward, spectrum left in A by rows pos(k); starts after first(A, ..)
+    __device__ __forceinline__ void forward_rest() const {
+        forward_mid(1);
+        middle(A, [&](auto &v, int b, int blk, int, int) {
+            constexpr int R = sizeof(v) / sizeof(C);
+#pragma unroll
+            for (int r = 0; r < R; ++r) A[row(blk * R + r) + b] = v[r];
+        });
+        __syncthreads();
+    }
+    // inverse of a spectrum in A up to (not including) last(A, ..)
+    __device__ __forceinline__ void inverse_begin() const {
+        __syncthreads();
+        at_last([&](auto rc, int, unsigned, int) {
+            constexpr int R = decltype(rc)::value;
+            each<R>([&](int b, int blk) {
+                C v[R];
+#pragma unroll
+                for (int r = 0; r < R; ++r) v[r] = A[row(blk * R + r) + b];
+                put<R>(A, b, blk, v);
+            });
+        });
+        inverse_mid(1);
+    }
+};
+
+}  // namespace hqt

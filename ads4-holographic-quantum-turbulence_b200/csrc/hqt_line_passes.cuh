@@ -1,0 +1,343 @@
+// hqt_line_passes.cuh -- the spectral passes of one RK stage and of the
+// filter (what each computes: hqt_passes.cuh) on the in-place line transforms
+// of hqt_line.cuh.  G is the geometry, compile-time (SGeo) or a kernel
+// argument (RGeo).
+//
+// Bound: each pass streams its fields through HBM once (x_rhs 88, y_rhs 112
+// bytes a site in FP64); next come the FP64 units (about 30 operations an
+// element and transform) and shared memory.  Two buffers of a block's lines
+// take at most about 66 KB, so three blocks share an SM and one block's loads
+// and stores run behind another's butterflies.
+#pragma once
+#include "hqt_line.cuh"
+#include "hqt_passes.cuh"
+
+namespace hqt {
+
+// The rhs passes get 128 registers a thread (512 threads per SM): an FP64
+// radix-8 butterfly with its spectrum and one product fits without spills.
+// The others hold one spectrum and get 80 (768 threads); with a runtime plan
+// all get 128, for the radices 9..13.
+#define HQT_L_BOUNDS(G) __launch_bounds__(G::kMaxThreads, 512 / G::kMaxThreads)
+#define HQT_L_BOUNDS1(G) \
+    __launch_bounds__(G::kMaxThreads, (G::kStatic && G::kMaxThreads < 512 ? 768 : 512) / G::kMaxThreads)
+
+template <typename T> __device__ __forceinline__ C2<T> lzero() { return mk2<T>(T(0), T(0)); }
+
+template <typename T, class G>
+__global__ void HQT_L_BOUNDS(G) k_lx_rhs(const __grid_constant__ XRhsArgs<T> a) {
+    const LineEng<T, G> w(a.lt);
+    const int n = w.g.n(), L0 = blockIdx.x << w.g.nbl(), valid = a.nlines - L0;
+    const long long g0 = (long long)L0 * n;
+    pdl_wait();
+    auto at = [&](int b, int e) { return g0 + (long long)b * n + e; };
+    // Psi, then C = A_x + i A_y: first and second derivative
+#pragma unroll 1
+    for (int f = 0; f < 2; ++f) {
+        w.first(w.A, [&](int b, int e) {
+            if (b >= valid) return lzero<T>();
+            const long long g = at(b, e);
+            return f == 0 ? a.psi[g] : mk2<T>(a.ax[g], a.ay[g]);
+        });
+        w.forward_mid(1);
+        w.middle_deriv12(a.s1, a.s2);
+        w.inverse_mid(2);
+        C2<T> *d1 = f == 0 ? a.dxpsi : a.E;
+        w.last(w.A, [&](int b, int e, C2<T> v) {
+            if (b < valid) d1[at(b, e)] = v;
+        });
+        w.last(w.B, [&](int b, int e, C2<T> v) {
+            if (b >= valid) return;
+            if (f == 0)
+                a.dxxpsi[at(b, e)] = v;
+            else
+                a.dxxay[at(b, e)] = v.y;
+        });
+    }
+}
+
+// The gauge fields travel as two complex lines whose y derivatives are the
+// outputs (no split of pair spectra):
+//   W1 = E_x + i A_y:  div A = E_x + Im(d_y W1),  d_x B = d_xx A_y - Re(d_y W1);
+//   W2 = A_x + i E_y:  d_y B = Im(d_y W2) - Re(d_yy W2)
+//      = Re(IFFT((s1 k - s2 k^2) W2^)), one real multiplier.
+template <typename T, class G>
+__global__ void HQT_L_BOUNDS(G) k_ly_rhs(const __grid_constant__ YRhsArgs<T> a) {
+    const LineEng<T, G> w(a.lt);
+    const int x0 = blockIdx.x << w.g.nbl(), valid = a.nx - x0;
+    const long long zoff = (long long)blockIdx.y * a.ny * a.nx + x0;
+    pdl_wait();
+    auto at = [&](int b, int e) { return zoff + (long long)e * a.nx + b; };
+#pragma unroll 1
+    for (int f = 0; f < 2; ++f) {
+        if (f == 0) {
+            w.first(w.A, [&](int b, int e) { return b < valid ? a.psi[at(b, e)] : lzero<T>(); });
+        } else {
+            w.first(w.A, [&](int b, int e) {
+                if (b >= valid) return lzero<T>();
+                const long long g = at(b, e);
+                return mk2<T>(a.E[g].x, a.ay[g]);
+            });
+            w.first(w.B, [&](int b, int e) {
+                if (b >= valid) return lzero<T>();
+                const long long g = at(b, e);
+                return mk2<T>(a.ax[g], a.E[g].y);
+            });
+        }
+        w.forward_mid(1 + f);
+        if (f == 0) {
+            w.middle_deriv12(a.s1, a.s2);
+        } else {
+            w.middle_deriv1(w.A, a.s1);
+            w.middle_deriv_mix(w.B, a.s1, a.s2);
+        }
+        w.inverse_mid(2);
+        if (f == 0) {
+            w.last(w.A, [&](int b, int e, C2<T> v) {
+                if (b < valid) a.dypsi[at(b, e)] = v;
+            });
+            w.last(w.B, [&](int b, int e, C2<T> v) {
+                if (b < valid) a.dyypsi[at(b, e)] = v;
+            });
+        } else {
+            w.last(
+                w.A,
+                [&](int b, int e) {
+                    if (b >= valid) return lzero<T>();
+                    const long long g = at(b, e);
+                    return mk2<T>(a.E[g].x, a.dxxay[g]);
+                },
+                [&](int b, int e, C2<T> v, C2<T> x) {
+                    if (b >= valid) return;
+                    const long long g = at(b, e);
+                    a.divA[g] = x.x + v.y;
+                    a.dxB[g] = x.y - v.x;
+                });
+            w.last(w.B, [&](int b, int e, C2<T> v) {
+                if (b < valid) a.dyB[at(b, e)] = v.x;
+            });
+        }
+    }
+}
+
+template <typename T, class G>
+__global__ void HQT_L_BOUNDS1(G) k_lx_d1(const __grid_constant__ XD1Args<T> a) {
+    const LineEng<T, G> w(a.lt);
+    const int n = w.g.n(), L0 = blockIdx.x << w.g.nbl(), valid = a.nlines - L0;
+    const long long g0 = (long long)L0 * n;
+    pdl_wait();
+    auto at = [&](int b, int e) { return g0 + (long long)b * n + e; };
+    w.first(w.A, [&](int b, int e) {
+        return b < valid ? load_field(a.in, at(b, e)) : lzero<T>();
+    });
+    w.forward_mid(1);
+    w.middle_deriv1(w.A, a.s1);
+    w.inverse_mid(1);
+    w.last(w.A, [&](int b, int e, C2<T> v) {
+        if (b < valid) store_field(a.out, at(b, e), v);
+    });
+}
+
+template <typename T, class G>
+__global__ void HQT_L_BOUNDS1(G) k_ly_d1(const __grid_constant__ YD1Args<T> a) {
+    const LineEng<T, G> w(a.lt);
+    const int x0 = blockIdx.x << w.g.nbl(), valid = a.nx - x0;
+    const long long zoff = (long long)blockIdx.y * a.ny * a.nx + x0;
+    pdl_wait();
+    auto at = [&](int b, int e) { return zoff + (long long)e * a.nx + b; };
+    w.first(w.A, [&](int b, int e) {
+        return b < valid ? load_field(a.in, at(b, e)) : lzero<T>();
+    });
+    w.forward_mid(1);
+    w.middle_deriv1(w.A, a.s1);
+    w.inverse_mid(1);
+    w.last(
+        w.A, [&](int b, int e) { return a.add_re && b < valid ? a.add_re[at(b, e)] : T(0); },
+        [&](int b, int e, C2<T> v, T x) {
+            v.x += x;
+            if (b < valid) store_field(a.out, at(b, e), v);
+        });
+}
+
+// First derivative of a real field into a real field, two real lines per
+// complex line (real_field_d1): complex line b carries real lines 2b and 2b+1.
+template <typename T, class G>
+__global__ void HQT_L_BOUNDS1(G) k_lx_d1r(const __grid_constant__ XD1Args<T> a) {
+    const LineEng<T, G> w(a.lt);
+    const int n = w.g.n(), L0 = blockIdx.x << (w.g.nbl() + 1), nr = a.nlines - L0;
+    const T *src = a.in.re + (long long)L0 * n;
+    T *dst = a.out.re + (long long)L0 * n;
+    pdl_wait();
+    w.first(w.A, [&](int b, int e) {
+        const long long g = 2ll * b * n + e;
+        return mk2<T>(2 * b < nr ? src[g] : T(0), 2 * b + 1 < nr ? src[g + n] : T(0));
+    });
+    w.forward_mid(1);
+    w.middle_deriv1(w.A, a.s1);
+    w.inverse_mid(1);
+    w.last(w.A, [&](int b, int e, C2<T> v) {
+        const long long g = 2ll * b * n + e;
+        if (2 * b < nr) dst[g] = v.x;
+        if (2 * b + 1 < nr) dst[g + n] = v.y;
+    });
+}
+
+template <typename T, class G>
+__global__ void HQT_L_BOUNDS1(G) k_ly_d1r(const __grid_constant__ YD1Args<T> a) {
+    const LineEng<T, G> w(a.lt);
+    const int x0 = blockIdx.x << (w.g.nbl() + 1), nr = a.nx - x0;
+    const long long zoff = (long long)blockIdx.y * a.ny * a.nx + x0;
+    pdl_wait();
+    auto pair = [&](const T *p, int b, int e) {
+        const long long g = zoff + (long long)e * a.nx + 2 * b;
+        return mk2<T>(2 * b < nr ? p[g] : T(0), 2 * b + 1 < nr ? p[g + 1] : T(0));
+    };
+    w.first(w.A, [&](int b, int e) { return pair(a.in.re, b, e); });
+    w.forward_mid(1);
+    w.middle_deriv1(w.A, a.s1);
+    w.inverse_mid(1);
+    w.last(
+        w.A, [&](int b, int e) { return a.add_re ? pair(a.add_re, b, e) : lzero<T>(); },
+        [&](int b, int e, C2<T> v, C2<T> x) {
+            const long long g = zoff + (long long)e * a.nx + 2 * b;
+            if (2 * b < nr) a.out.re[g] = v.x + x.x;
+            if (2 * b + 1 < nr) a.out.re[g + 1] = v.y + x.y;
+        });
+}
+
+// Filter, x forward: spectra in natural order, the weight-zeroed columns left
+// unwritten.
+template <typename T, class G>
+__global__ void HQT_L_BOUNDS1(G) k_lx_filt_fwd(const __grid_constant__ XFiltFwdArgs<T> a) {
+    const LineEng<T, G> w(a.lt);
+    const int n = w.g.n(), L0 = blockIdx.x << w.g.nbl(), valid = a.nlines - L0;
+    const long long g0 = (long long)L0 * n;
+    pdl_wait();
+    const int wnd = a.st ? a.st->winding : 0;
+    auto at = [&](int b, int e) { return g0 + (long long)b * n + e; };
+    // winding phase -2 pi y w / ny of this thread's line (a thread keeps its
+    // line: the lines per block divide the block)
+    double sn = 0.0, cs = 1.0;
+    if (wnd != 0) {
+        const int y = (L0 + (threadIdx.x & ((1 << w.g.nbl()) - 1))) % a.ny;
+        const long long q = ((long long)y * wnd) % a.ny;
+        sincospi(-2.0 * (double)q / (double)a.ny, &sn, &cs);
+    }
+#pragma unroll 1
+    for (int f = 0; f < a.nf; ++f) {
+        // one load expression per kind of field, without branches an element:
+        // the loads of a butterfly are in flight together
+        const FieldIn<T> in = a.in[f];
+        if (in.c) {
+            const bool turn = f == 0 && wnd != 0;
+            const T c = turn ? (T)cs : T(1), s = turn ? (T)sn : T(0);
+            w.first(w.A, [&](int b, int e) {
+                const C2<T> v = b < valid ? in.c[at(b, e)] : lzero<T>();
+                return turn ? mk2<T>(v.x * c - v.y * s, v.x * s + v.y * c) : v;
+            });
+        } else {
+            const bool pair = in.im != nullptr;
+            const T *im = pair ? in.im : in.re;
+            const bool turn = f == 0 && wnd != 0;
+            const T c = turn ? (T)cs : T(1), s = turn ? (T)sn : T(0);
+            w.first(w.A, [&](int b, int e) {
+                if (b >= valid) return lzero<T>();
+                const long long g = at(b, e);
+                C2<T> v = mk2<T>(in.re[g], im[g]);
+                if (!pair) v.y = T(0);
+                return turn ? mk2<T>(v.x * c - v.y * s, v.x * s + v.y * c) : v;
+            });
+        }
+        w.forward_rest();
+        C2<T> *spec = a.spec[f];
+        w.modes([&](int b, int k) {
+            if (b < valid && filt_col_live(k, a.dead0, a.dead1))
+                spec[at(b, k)] = w.A[w.row(w.pos(k)) + b];
+        });
+        __syncthreads();  // the next field's first pass writes other threads' rows
+    }
+}
+
+// Filter, y: forward, weight, inverse; blockIdx.z = field
+template <typename T, class G>
+__global__ void HQT_L_BOUNDS1(G) k_ly_filt(const __grid_constant__ YFiltArgs<T> a) {
+    const LineEng<T, G> w(a.lt);
+    const int n = w.g.n(), NB = 1 << w.g.nbl();
+    const int x0 = blockIdx.x * NB, valid = min(NB, a.nx - x0);
+    const long long zoff = (long long)blockIdx.y * a.ny * a.nx + x0;
+    bool live = false;
+    for (int b = 0; b < valid; ++b) live = live || filt_col_live(x0 + b, a.dead0, a.dead1);
+    if (!live) return;  // every column filtered out
+    pdl_wait();
+    C2<T> *spec = a.spec[blockIdx.z];
+    auto at = [&](int b, int e) { return zoff + (long long)e * a.nx + b; };
+    w.first(w.A, [&](int b, int e) { return b < valid ? spec[at(b, e)] : lzero<T>(); });
+    w.forward_mid(1);
+    w.middle(w.A, [&](auto &v, int b, int blk, int k0, int st) {
+        constexpr int R = sizeof(v) / sizeof(C2<T>);
+        const int kx = x0 + min(b, valid - 1), kxm = kx == 0 ? 0 : a.nx - kx;
+        const T m0 = __ldg(a.mx + kx), m1 = __ldg(a.mx + kxm);
+#pragma unroll
+        for (int i = 0; i < R; ++i) {
+            const int ky = k0 + i * st, kym = ky == 0 ? 0 : n - ky;
+            const T wgt = T(0.5) * (m0 * __ldg(a.my + ky) + m1 * __ldg(a.my + kym)) * a.scale;
+            v[i] = wgt * v[i];
+        }
+        w.template put<R>(w.A, b, blk, v);
+    });
+    w.inverse_mid(1);
+    w.last(w.A, [&](int b, int e, C2<T> v) {
+        if (b < valid) spec[at(b, e)] = v;
+    });
+}
+
+// Filter, x inverse; a non-finite value sets the status' first bad step
+template <typename T, class G>
+__global__ void HQT_L_BOUNDS1(G) k_lx_filt_inv(const __grid_constant__ XFiltInvArgs<T> a) {
+    const LineEng<T, G> w(a.lt);
+    const int n = w.g.n(), L0 = blockIdx.x << w.g.nbl(), valid = a.nlines - L0;
+    const long long g0 = (long long)L0 * n;
+    pdl_wait();
+    int bad = 0;
+    auto at = [&](int b, int e) { return g0 + (long long)b * n + e; };
+#pragma unroll 1
+    for (int f = 0; f < a.nf; ++f) {
+        const C2<T> *spec = a.spec[f];
+        w.modes([&](int b, int k) {
+            w.A[w.row(w.pos(k)) + b] =
+                b < valid && filt_col_live(k, a.dead0, a.dead1) ? spec[at(b, k)] : lzero<T>();
+        });
+        w.inverse_begin();
+        const FieldOut<T> out = a.out[f];
+        w.last(w.A, [&](int b, int e, C2<T> v) {
+            if (!(isfinite(v.x) && isfinite(v.y))) bad = 1;
+            if (b < valid) store_field(out, at(b, e), v);
+        });
+        __syncthreads();  // the next field's load writes other threads' rows
+    }
+    if (a.st && __syncthreads_or(bad) && threadIdx.x == 0)
+        atomicMin(reinterpret_cast<unsigned long long *>(&a.st->first_bad_step),
+                  (unsigned long long)(a.st->step + 1));
+}
+
+// Forward transform along y of nf complex fields, natural order (spectrum)
+template <typename T, class G>
+__global__ void HQT_L_BOUNDS1(G) k_ly_fwd(const __grid_constant__ YFiltArgs<T> a) {
+    const LineEng<T, G> w(a.lt);
+    const int x0 = blockIdx.x << w.g.nbl(), valid = a.nx - x0;
+    const long long zoff = (long long)blockIdx.y * a.ny * a.nx + x0;
+    pdl_wait();
+    auto at = [&](int b, int e) { return zoff + (long long)e * a.nx + b; };
+#pragma unroll 1
+    for (int f = 0; f < a.nf; ++f) {
+        C2<T> *spec = a.spec[f];
+        w.first(w.A, [&](int b, int e) { return b < valid ? spec[at(b, e)] : lzero<T>(); });
+        w.forward_rest();
+        w.modes([&](int b, int k) {
+            if (b < valid) spec[at(b, k)] = w.A[w.row(w.pos(k)) + b];
+        });
+        __syncthreads();
+    }
+}
+
+}  // namespace hqt

@@ -181,6 +181,30 @@ void make_big_tables(std::vector<double> &c, std::vector<double> &s) {
         }
 }
 
+void make_line_tables(const LPlan &p, const std::vector<double2> &roots,
+                      std::vector<double2> &tw, std::vector<int> &freq, std::vector<int> &pos) {
+    tw.assign((size_t)p.ntw + 1, double2{1.0, 0.0});
+    for (int i = 0; i + 1 < p.np; ++i) {
+        const int s = p.s[i], R = p.R[i], step = p.n / (R * s);
+        for (int k = 1; k < R; ++k)
+            for (int j = 0; j < s; ++j)
+                tw[(size_t)p.tw[i] + (size_t)(k - 1) * s + j] =
+                    roots[(size_t)((long long)j * k * step % p.n)];
+    }
+    pos.assign(p.n, 0);
+    freq.assign(p.n, 0);
+    const int Rm = p.R[p.np - 1];
+    for (int k = 0; k < p.n; ++k) {
+        int e = 0, rem = k;
+        for (int i = 0; i < p.np; ++i) {
+            e += (rem % p.R[i]) * p.s[i];
+            rem /= p.R[i];
+        }
+        pos[k] = e;
+        if (e % Rm == 0) freq[e / Rm] = k;
+    }
+}
+
 static int matlab_round_pos(double v) { return (int)std::floor(v + 0.5); }
 
 void filter_band(int n, int &lo, int &hi) {

@@ -3,6 +3,7 @@
 #include <vector>
 
 #include "hqt_common.cuh"
+#include "hqt_lineplan.h"
 
 namespace hqt {
 
@@ -29,6 +30,12 @@ void make_radix_tables(std::vector<double> &c, std::vector<double> &s);
 
 // cos/sin tables of the large odd primes of the compile-time transforms.
 void make_big_tables(std::vector<double> &c, std::vector<double> &s);
+
+// Tables of an in-place plan from the roots of its length: packed twiddles,
+// freq[blk] = lowest mode of butterfly blk of the last pass, pos[k] = row of
+// mode k.
+void make_line_tables(const LPlan &p, const std::vector<double2> &roots,
+                      std::vector<double2> &tw, std::vector<int> &freq, std::vector<int> &pos);
 
 // MATLAB round of the filter band edges: 1-based indices lo..hi of the
 // zeroed modes (tevol_driven_cluster.m:27-30).
