@@ -22,9 +22,12 @@
 #include <string>
 #include <vector>
 
+#include <cudaTypedefs.h>
+
 #include "hqt.h"
 #include "hqt_diag.cuh"
 #include "hqt_launch.h"
+#include "hqt_zdims.h"
 #include "hqt_ops_host.h"
 
 namespace hqt {
@@ -73,24 +76,29 @@ struct hqt_ctx {
     // stage input and accumulators
     // stage inputs, double-buffered: stages 2 and 4 read Y[0], stage 3 reads Y[1]
     double2 *ypsi2[2] = {nullptr, nullptr}, *kpsi = nullptr;
-    double *yax2[2] = {nullptr, nullptr}, *yay2[2] = {nullptr, nullptr};
-    double2 *kA = nullptr;  // (A_x, A_y) accumulator, interleaved
+    double2 *yA2[2] = {nullptr, nullptr};
+    double2 *kA = nullptr;
+    // (A_x, A_y) and (A_t, d_z A_t) of the current state, interleaved: what a
+    // step reads and writes; the filter (or k_unpack_state) writes the
+    // caller's real arrays beside them
+    double2 *zA = nullptr, *atd = nullptr;
     double *krho = nullptr;
     // derivatives
     double2 *dxpsi = nullptr, *dxxpsi = nullptr, *E = nullptr, *dypsi = nullptr,
             *dyypsi = nullptr;
-    double *dxxay = nullptr, *divA = nullptr, *dxB = nullptr, *dyB = nullptr;
-    double *dxat = nullptr, *dyat = nullptr, *dat = nullptr, *dxax = nullptr;
+    double *dxxay = nullptr, *divA = nullptr, *dxax = nullptr;
+    double2 *B = nullptr;    // (d_y B, d_x B)
+    double2 *dAt = nullptr;  // (d_x A_t, d_y A_t)
     // mixed precision: FP32 stage inputs ([0], [1]; [2] = copy of the state)
     // and FP32 derivative fields of the line passes
     bool mixed = false;
     float2 *ypsi32[3] = {nullptr, nullptr, nullptr};
-    float *yax32[3] = {nullptr, nullptr, nullptr}, *yay32[3] = {nullptr, nullptr, nullptr};
+    float2 *yA32[3] = {nullptr, nullptr, nullptr};
     float *at32 = nullptr;
     float2 *dxpsi32 = nullptr, *dxx32 = nullptr, *dyy32 = nullptr, *E32 = nullptr,
            *dypsi32 = nullptr;
-    float *dxxay32 = nullptr, *divA32 = nullptr, *dxB32 = nullptr, *dyB32 = nullptr;
-    float *dxat32 = nullptr, *dyat32 = nullptr;
+    float *dxxay32 = nullptr, *divA32 = nullptr;
+    float2 *B32 = nullptr, *dAt32 = nullptr;
     double *slice_mean = nullptr;                           // 5 per z-slice
     double *slice_partial = nullptr;                        // 5 per (z, chunk)
     double2 *O = nullptr;
@@ -103,6 +111,9 @@ struct hqt_ctx {
     double2 *obs_partial = nullptr;  // compensated observable sums per block
     double *obs_out = nullptr;       // Q, E_kin, N_O
     DevStatus *st = nullptr;
+    // radial stage: operand tables (z_tables) and the tensor-map encoder
+    double *zfrag = nullptr, *ztab = nullptr;
+    PFN_cuTensorMapEncodeTiled_v12000 tmap_encode = nullptr;
     // launch geometry
     int NBx_rhs = 1, NBx_2 = 1, TXy_rhs = 1, TXy_2 = 1, TXy_filt = 1;
     bool cx = false, cy = false;  // compile-time line passes along x / y
@@ -177,12 +188,12 @@ int fail(hqt_ctx *c, int code, const std::string &msg) {
 // kernel kinds reported by hqt_profile_report
 enum Kind {
     K_X_RHS, K_Y_RHS, K_ZSTAGE, K_X_D1, K_Y_D1, K_ZCONS, K_ZMISC, K_WIND, K_FILT_X_FWD,
-    K_FILT_Y, K_FILT_X_INV, K_PHASE, K_STEP_END, K_COUNT, K_RHO, K_CONVERT, K_NKINDS
+    K_FILT_Y, K_FILT_X_INV, K_PHASE, K_STEP_END, K_COUNT, K_RHO, K_CONVERT, K_PACK, K_NKINDS
 };
 const char *const kKindName[K_NKINDS] = {
     "x_rhs", "y_rhs", "zstage", "x_d1", "y_d1", "zcons", "zcol_misc", "winding",
     "filter_x_fwd", "filter_y", "filter_x_inv", "phase_multiply", "step_end",
-    "count_vortices", "rho_gather_scatter", "state_to_f32"};
+    "count_vortices", "rho_gather_scatter", "state_to_f32", "pack_pairs"};
 
 struct Prof {
     hqt_ctx *c;
@@ -302,10 +313,8 @@ int pick_lines(int n, int nbuf, int cap) {
 
 ZHost zhost(const hqt_ctx *c) { return ZHost{c->nz, c->Lz.data(), c->Lz1.data(), c->zz.data()}; }
 
-size_t smem_z(int NZP) { return sizeof(double) * 2 * (size_t)NZP * kThreadsZ; }
-
 // ---------------------------------------------------------------- launches
-int launch_x_rhs(hqt_ctx *c, const double2 *psi, const double *ax, const double *ay) {
+int launch_x_rhs(hqt_ctx *c, const double2 *psi, const double2 *A) {
     XRhsArgs<double> a{};
     a.plan = c->planx;
     a.roots = c->rootsx;
@@ -316,8 +325,7 @@ int launch_x_rhs(hqt_ctx *c, const double2 *psi, const double *ax, const double 
     a.s1 = two_pi / c->p.Lx / c->nx;
     a.s2 = -(two_pi / c->p.Lx) * (two_pi / c->p.Lx) / c->nx;
     a.psi = psi;
-    a.ax = ax;
-    a.ay = ay;
+    a.A = A;
     a.dxpsi = c->dxpsi;
     a.dxxpsi = c->dxxpsi;
     a.E = c->E;
@@ -333,7 +341,7 @@ int launch_x_rhs(hqt_ctx *c, const double2 *psi, const double *ax, const double 
     return HQT_OK;
 }
 
-int launch_y_rhs(hqt_ctx *c, const double2 *psi, const double *ax, const double *ay) {
+int launch_y_rhs(hqt_ctx *c, const double2 *psi, const double2 *A) {
     YRhsArgs<double> a{};
     a.plan = c->plany;
     a.roots = c->rootsy;
@@ -345,15 +353,13 @@ int launch_y_rhs(hqt_ctx *c, const double2 *psi, const double *ax, const double 
     a.s1 = two_pi / c->p.Ly / c->ny;
     a.s2 = -(two_pi / c->p.Ly) * (two_pi / c->p.Ly) / c->ny;
     a.psi = psi;
-    a.ax = ax;
-    a.ay = ay;
+    a.A = A;
     a.E = c->E;
     a.dxxay = c->dxxay;
     a.dypsi = c->dypsi;
     a.dyypsi = c->dyypsi;
     a.divA = c->divA;
-    a.dxB = c->dxB;
-    a.dyB = c->dyB;
+    a.B = c->B;
     dim3 grid((c->nx + a.TX - 1) / a.TX, c->nz);
     Prof pr(c, K_Y_RHS);
     if (c->py) {
@@ -412,7 +418,7 @@ int launch_y_d1(hqt_ctx *c, FieldIn<double> in, const double *add_re, FieldOut<d
 }
 
 // ---- FP32 stage passes (mixed precision) ----
-int launch_x_rhs32(hqt_ctx *c, const float2 *psi, const float *ax, const float *ay) {
+int launch_x_rhs32(hqt_ctx *c, const float2 *psi, const float2 *A) {
     XRhsArgs<float> a{};
     a.plan = c->planx;
     a.roots = nullptr;
@@ -423,8 +429,7 @@ int launch_x_rhs32(hqt_ctx *c, const float2 *psi, const float *ax, const float *
     a.s2 = (float)(-(two_pi / c->p.Lx) * (two_pi / c->p.Lx) / c->nx);
     a.roots = reinterpret_cast<const float2 *>(c->rootsx32);
     a.psi = psi;
-    a.ax = ax;
-    a.ay = ay;
+    a.A = A;
     a.dxpsi = c->dxpsi32;
     a.dxxpsi = c->dxx32;
     a.E = c->E32;
@@ -445,7 +450,7 @@ int launch_x_rhs32(hqt_ctx *c, const float2 *psi, const float *ax, const float *
     return HQT_OK;
 }
 
-int launch_y_rhs32(hqt_ctx *c, const float2 *psi, const float *ax, const float *ay) {
+int launch_y_rhs32(hqt_ctx *c, const float2 *psi, const float2 *A) {
     YRhsArgs<float> a{};
     a.plan = c->plany;
     a.roots = reinterpret_cast<const float2 *>(c->rootsy32);
@@ -456,15 +461,13 @@ int launch_y_rhs32(hqt_ctx *c, const float2 *psi, const float *ax, const float *
     a.s1 = (float)(two_pi / c->p.Ly / c->ny);
     a.s2 = (float)(-(two_pi / c->p.Ly) * (two_pi / c->p.Ly) / c->ny);
     a.psi = psi;
-    a.ax = ax;
-    a.ay = ay;
+    a.A = A;
     a.E = c->E32;
     a.dxxay = c->dxxay32;
     a.dypsi = c->dypsi32;
     a.dyypsi = c->dyy32;
     a.divA = c->divA32;
-    a.dxB = c->dxB32;
-    a.dyB = c->dyB32;
+    a.B = c->B32;
     Prof pr(c, K_Y_RHS);
     if (c->py) {
         CK(pfa_launch_301(CT_Y_RHS_F, &a, c->nz, c->stream));
@@ -481,7 +484,9 @@ int launch_y_rhs32(hqt_ctx *c, const float2 *psi, const float *ax, const float *
     return HQT_OK;
 }
 
-int launch_d1_32(hqt_ctx *c, bool along_x, const float *in, float *out) {
+// first derivative of a real field into part (0: x, 1: y) of pairs
+int launch_d1_32(hqt_ctx *c, bool along_x, const float *in, float2 *pairs) {
+    float *out = reinterpret_cast<float *>(pairs) + (along_x ? 0 : 1);
     const double two_pi = 2.0 * 3.14159265358979323846;
     if (along_x) {
         XD1Args<float> a{};
@@ -491,7 +496,7 @@ int launch_d1_32(hqt_ctx *c, bool along_x, const float *in, float *out) {
         a.nlines = c->ny * c->nz;
         a.s1 = (float)(two_pi / c->p.Lx / c->nx);
         a.in = FieldIn<float>{nullptr, in, nullptr};
-        a.out = FieldOut<float>{nullptr, out, nullptr};
+        a.out = FieldOut<float>{nullptr, out, nullptr, 2};
         Prof pr(c, K_X_D1);
         if (c->px) {
             CK(pfa_launch_301(CT_X_D1_F, &a, a.nlines, c->stream));
@@ -515,7 +520,7 @@ int launch_d1_32(hqt_ctx *c, bool along_x, const float *in, float *out) {
     a.ny = c->ny;
     a.s1 = (float)(two_pi / c->p.Ly / c->ny);
     a.in = FieldIn<float>{nullptr, in, nullptr};
-    a.out = FieldOut<float>{nullptr, out, nullptr};
+    a.out = FieldOut<float>{nullptr, out, nullptr, 2};
     Prof pr(c, K_Y_D1);
     if (c->py) {
         CK(pfa_launch_301(CT_Y_D1_F, &a, c->nz, c->stream));
@@ -619,8 +624,7 @@ int launch_filter(hqt_ctx *c, int nf, const FieldIn<double> *in, const FieldOut<
                 for (int k = 0; k < 2; ++k) a.slot[f][k] = kMeanSlot[f][k];
             a.c32[0] = c->ypsi32[2];
             a.re32[1] = c->at32;
-            a.re32[2] = c->yax32[2];
-            a.im32[2] = c->yay32[2];
+            a.c32[2] = c->yA32[2];
         }
         const int grid = (a.nlines + a.NB - 1) / a.NB;
         Prof pr(c, K_FILT_X_INV);
@@ -635,29 +639,53 @@ int launch_filter(hqt_ctx *c, int nf, const FieldIn<double> *in, const FieldOut<
     return HQT_OK;
 }
 
-template <int MODE> int launch_zstage(hqt_ctx *c, const ZStageArgs<double, double> &a) {
-    const int grid = (int)((c->plane + kThreadsZ - 1) / kThreadsZ);
-    const ZHost h = zhost(c);
-    Prof pr(c, K_ZSTAGE);
-    switch (c->NZP) {
-#define HQT_Z(N)                                                                      \
-    case N:                                                                           \
-        CK(z_stage<N>(MODE, a, h, grid, kThreadsZ, smem_z(N), c->stream));            \
-        return HQT_OK;
-        HQT_NZP_LIST(HQT_Z)
-#undef HQT_Z
-    }
-    return fail(c, HQT_EUNSUPPORTED, "unsupported nz");
+// Tensor map of a field [nz][plane] of `comps` values of type T per site: boxes of
+// `width` sites x nz levels.  The level rows must be a multiple of 16 bytes apart.
+template <typename T>
+int zs_map(hqt_ctx *c, CUtensorMap *m, const void *base, int comps, int width) {
+    const cuuint64_t dims[2] = {(cuuint64_t)comps * c->plane, (cuuint64_t)c->nz};
+    const cuuint64_t strides[1] = {(cuuint64_t)comps * sizeof(T) * c->plane};
+    const cuuint32_t box[2] = {(cuuint32_t)(width * comps), (cuuint32_t)c->nz}, es[2] = {1, 1};
+    const CUresult r = c->tmap_encode(
+        m, sizeof(T) == 8 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT64 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2,
+        const_cast<void *>(base), dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
+        CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+        CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS) return fail(c, HQT_ECUDA, "tensor map");
+    return HQT_OK;
 }
 
-int launch_zstage_mixed(hqt_ctx *c, int mode, const ZStageArgs<double, double, float> &a) {
-    const int grid = (int)((c->plane + kThreadsZ - 1) / kThreadsZ);
-    const ZHost h = zhost(c);
+// One radial stage (mode 0: right-hand side only); fills in the arguments common
+// to all and the tensor maps of the pointers that are set.
+template <typename TD> int launch_zstage(hqt_ctx *c, int mode, ZStageArgs<TD> a) {
+    a.nz = c->nz;
+    a.plane = c->plane;
+    a.h = c->p.dt;
+    a.frag = c->zfrag;
+    a.ztab = c->ztab;
+    a.fault = &c->st->fault;
+    a.copy_pairs = c->plane * sizeof(C2<TD>) % 16 != 0;
+    a.copy_real = c->plane * sizeof(TD) % 16 != 0;
+    struct {
+        CUtensorMap *m;
+        const void *p;
+    } full[] = {{&a.mPS, a.ypsi}, {&a.mAXY, a.yA},   {&a.mATD, a.atd}, {&a.mZA, a.zA},
+                {&a.mKA, a.kA},   {&a.mZP, a.zpsi}, {&a.mKP, a.kpsi}},
+      pairs[] = {{&a.mDX, a.dxpsi}, {&a.mDY, a.dypsi}, {&a.mDT, a.dAt},
+                 {&a.mB, a.B},      {&a.mXX, a.dxxpsi}, {&a.mYY, a.dyypsi}};
+    for (auto &f : full)
+        if (f.p) RC(zs_map<double>(c, f.m, f.p, 2, zs_row_td<double>() / 16));
+    if (!a.copy_pairs)
+        for (auto &f : pairs) RC(zs_map<TD>(c, f.m, f.p, 2, zs_row_td<TD>() / (int)sizeof(C2<TD>)));
+    if (!a.copy_real) RC(zs_map<TD>(c, &a.mDIV, a.divA, 1, zs_row_r<TD>() / (int)sizeof(TD)));
     Prof pr(c, K_ZSTAGE);
     switch (c->NZP) {
-#define HQT_Z(N)                                                                       \
-    case N:                                                                            \
-        CK(z_stage_mixed<N>(mode, a, h, grid, kThreadsZ, smem_z(N), c->stream));       \
+#define HQT_Z(N)                                                       \
+    case N:                                                            \
+        if constexpr (std::is_same<TD, double>::value)                 \
+            CK(z_stage<N>(mode, a, c->stream));                        \
+        else                                                           \
+            CK(z_stage_mixed<N>(mode, a, c->stream));                  \
         return HQT_OK;
         HQT_NZP_LIST(HQT_Z)
 #undef HQT_Z
@@ -672,10 +700,8 @@ int launch_zcons(hqt_ctx *c) {
     a.mu = c->p.mu;
     a.vy = c->p.vy;
     a.psi = c->cpsi;
-    a.ax = c->cax;
-    a.ay = c->cay;
-    a.at = c->cat;
-    a.dat = c->dat;
+    a.A = c->zA;
+    a.atd = c->atd;
     a.divA = c->divA;
     a.rho = c->rho;
     a.O = c->O;
@@ -691,12 +717,12 @@ int launch_zcons(hqt_ctx *c) {
     return fail(c, HQT_EUNSUPPORTED, "unsupported nz");
 }
 
-int launch_zcol_misc(hqt_ctx *c, const double *at, double *dat, const double2 *psi, double2 *O) {
+int launch_zcol_misc(hqt_ctx *c, const double *at, double2 *atd, const double2 *psi, double2 *O) {
     ZColArgs<double> a{};
     a.nz = c->nz;
     a.plane = c->plane;
     a.at = at;
-    a.dat = dat;
+    a.atd = atd;
     a.psi = psi;
     a.O = O;
     const int grid = (int)((c->plane + kThreadsZ - 1) / kThreadsZ);
@@ -739,8 +765,7 @@ int enqueue_convert(hqt_ctx *c) {
                   c->slice_partial, c->nz, c->plane, c->slice_mean);
     CK(cudaGetLastError());
     (void)klaunch(k_state_to_f32, dim3(592), dim3(256), 0, c->stream, c->cpsi, c->cat, c->cax,
-                  c->cay, c->plane, c->vol, c->slice_mean, c->ypsi32[2], c->at32, c->yax32[2],
-                  c->yay32[2]);
+                  c->cay, c->plane, c->vol, c->slice_mean, c->ypsi32[2], c->at32, c->yA32[2]);
     CK(cudaGetLastError());
     return HQT_OK;
 }
@@ -768,60 +793,47 @@ int join_side(hqt_ctx *c) {
 
 int enqueue_stages_mixed(hqt_ctx *c) {
     double2 *psi = c->cpsi;
-    double *at = c->cat, *ax = c->cax, *ay = c->cay;
     // with fused_convert the previous step's filter (or prestep) left them
     if (!c->fused_convert) RC(enqueue_convert(c));
     // the A_t derivatives beside stage 1's line passes
     RC(on_side(c, [&]() -> int {
-        RC(launch_d1_32(c, true, c->at32, c->dxat32));
-        return launch_d1_32(c, false, c->at32, c->dyat32);
+        RC(launch_d1_32(c, true, c->at32, c->dAt32));
+        return launch_d1_32(c, false, c->at32, c->dAt32);
     }));
     for (int s = 1; s <= 4; ++s) {
         const int yi = (s == 3) ? 1 : 0, ni = (s == 2) ? 1 : 0;
         const int y32 = (s == 1) ? 2 : yi;
         const double2 *ypsi = (s == 1) ? psi : c->ypsi2[yi];
-        const double *yax = (s == 1) ? ax : c->yax2[yi];
-        const double *yay = (s == 1) ? ay : c->yay2[yi];
-        RC(launch_x_rhs32(c, c->ypsi32[y32], c->yax32[y32], c->yay32[y32]));
-        RC(launch_y_rhs32(c, c->ypsi32[y32], c->yax32[y32], c->yay32[y32]));
-        ZStageArgs<double, double, float> a{};
-        a.nz = c->nz;
-        a.plane = c->plane;
-        a.h = c->p.dt;
+        const double2 *yA = (s == 1) ? c->zA : c->yA2[yi];
+        RC(launch_x_rhs32(c, c->ypsi32[y32], c->yA32[y32]));
+        RC(launch_y_rhs32(c, c->ypsi32[y32], c->yA32[y32]));
+        ZStageArgs<float> a{};
         a.ypsi = ypsi;
-        a.yax = yax;
-        a.yay = yay;
-        a.at = at;
-        a.dat = c->dat;
-        a.dxat = c->dxat32;
-        a.dyat = c->dyat32;
+        a.yA = yA;
+        a.atd = c->atd;
+        a.dAt = c->dAt32;
         a.dxpsi = c->dxpsi32;
         a.dypsi = c->dypsi32;
         a.dxxpsi = c->dxx32;
         a.dyypsi = c->dyy32;
         a.divA = c->divA32;
-        a.dxB = c->dxB32;
-        a.dyB = c->dyB32;
+        a.B = c->B32;
         a.zpsi = psi;
-        a.zax = ax;
-        a.zay = ay;
+        a.zA = c->zA;
         a.zrho = c->rho;
         a.kpsi = c->kpsi;
         a.kA = c->kA;
         a.krho = c->krho;
         a.npsi = c->ypsi2[ni];
-        a.nax = c->yax2[ni];
-        a.nay = c->yay2[ni];
+        a.nA = c->yA2[ni];
         a.npsi_d = c->ypsi32[ni];
-        a.nax_d = c->yax32[ni];
-        a.nay_d = c->yay32[ni];
+        a.nA_d = c->yA32[ni];
         a.wpsi = psi;
-        a.wax = ax;
-        a.way = ay;
+        a.wA = c->zA;
         a.wrho = c->rho;
         a.slice_mean = c->slice_mean;
         if (s == 1) RC(join_side(c));
-        RC(launch_zstage_mixed(c, s, a));
+        RC(launch_zstage<float>(c, s, a));
     }
     return HQT_OK;
 }
@@ -844,75 +856,66 @@ int enqueue_step(hqt_ctx *c) {
     // beside stage 1's line passes (which do not read them)
     RC(on_side(c, [&]() -> int {
         RC(launch_x_d1(c, FieldIn<double>{nullptr, at, nullptr},
-                       FieldOut<double>{nullptr, c->dxat, nullptr}));
+                       FieldOut<double>{nullptr, &c->dAt->x, nullptr, 2}));
         return launch_y_d1(c, FieldIn<double>{nullptr, at, nullptr}, nullptr,
-                           FieldOut<double>{nullptr, c->dyat, nullptr});
+                           FieldOut<double>{nullptr, &c->dAt->y, nullptr, 2});
     }));
     for (int s = 1; s <= 4; ++s) {
         // stage s reads Y[(s-2)&1] (the state itself at s = 1) and writes the
         // next stage input to the other buffer
         const int yi = (s == 3) ? 1 : 0, ni = (s == 2) ? 1 : 0;
         const double2 *ypsi = (s == 1) ? psi : c->ypsi2[yi];
-        const double *yax = (s == 1) ? ax : c->yax2[yi];
-        const double *yay = (s == 1) ? ay : c->yay2[yi];
-        RC(launch_x_rhs(c, ypsi, yax, yay));
-        RC(launch_y_rhs(c, ypsi, yax, yay));
-        ZStageArgs<double, double> a{};
-        a.nz = c->nz;
-        a.plane = c->plane;
-        a.h = c->p.dt;
+        const double2 *yA = (s == 1) ? c->zA : c->yA2[yi];
+        RC(launch_x_rhs(c, ypsi, yA));
+        RC(launch_y_rhs(c, ypsi, yA));
+        ZStageArgs<double> a{};
         a.ypsi = ypsi;
-        a.yax = yax;
-        a.yay = yay;
-        a.at = at;
-        a.dat = c->dat;
-        a.dxat = c->dxat;
-        a.dyat = c->dyat;
+        a.yA = yA;
+        a.atd = c->atd;
+        a.dAt = c->dAt;
         a.dxpsi = c->dxpsi;
         a.dypsi = c->dypsi;
         a.dxxpsi = c->dxxpsi;
         a.dyypsi = c->dyypsi;
         a.divA = c->divA;
-        a.dxB = c->dxB;
-        a.dyB = c->dyB;
+        a.B = c->B;
         a.zpsi = psi;
-        a.zax = ax;
-        a.zay = ay;
+        a.zA = c->zA;
         a.zrho = c->rho;
         a.kpsi = c->kpsi;
         a.kA = c->kA;
         a.krho = c->krho;
         a.npsi = c->ypsi2[ni];
-        a.nax = c->yax2[ni];
-        a.nay = c->yay2[ni];
+        a.nA = c->yA2[ni];
         a.wpsi = psi;
-        a.wax = ax;
-        a.way = ay;
+        a.wA = c->zA;
         a.wrho = c->rho;
         if (s == 1) RC(join_side(c));
-        switch (s) {
-            case 1: RC(launch_zstage<1>(c, a)); break;
-            case 2: RC(launch_zstage<2>(c, a)); break;
-            case 3: RC(launch_zstage<3>(c, a)); break;
-            default: RC(launch_zstage<4>(c, a)); break;
-        }
+        RC(launch_zstage<double>(c, s, a));
     }
     }
     // constraint: div A of the combined fields, then A_t, BCs, O
-    RC(launch_x_d1(c, FieldIn<double>{nullptr, ax, nullptr},
+    RC(launch_x_d1(c, FieldIn<double>{nullptr, &c->zA->x, nullptr, 2},
                    FieldOut<double>{nullptr, c->dxax, nullptr}));
-    RC(launch_y_d1(c, FieldIn<double>{nullptr, ay, nullptr}, c->dxax,
+    RC(launch_y_d1(c, FieldIn<double>{nullptr, &c->zA->y, nullptr, 2}, c->dxax,
                    FieldOut<double>{nullptr, c->divA, nullptr}));
     RC(launch_zcons(c));
     if (c->p.remove_winding) RC(launch_winding(c, c->O, nullptr));
     if (c->p.apply_filter) {
-        FieldIn<double> in[3] = {{psi, nullptr, nullptr}, {nullptr, at, c->dat}, {nullptr, ax, ay}};
-        FieldOut<double> out[3] = {{psi, nullptr, nullptr}, {nullptr, at, c->dat}, {nullptr, ax, ay}};
+        FieldIn<double> in[3] = {
+            {psi, nullptr, nullptr}, {c->atd, nullptr, nullptr}, {c->zA, nullptr, nullptr}};
+        FieldOut<double> out[3] = {{psi, nullptr, nullptr}, {c->atd, at, nullptr}, {c->zA, ax, ay}};
         RC(launch_filter(c, 3, in, out, c->p.remove_winding != 0, true, c->fused_convert));
-    } else if (c->p.remove_winding) {
-        Prof pr(c, K_PHASE);
-        (void)klaunch(k_phase_multiply, dim3(592), dim3(256), 0, c->stream, psi, c->nx, c->ny,
-                      c->vol, c->st);
+    } else {
+        if (c->p.remove_winding) {
+            Prof pr(c, K_PHASE);
+            (void)klaunch(k_phase_multiply, dim3(592), dim3(256), 0, c->stream, psi, c->nx, c->ny,
+                          c->vol, c->st);
+            CK(cudaGetLastError());
+        }
+        Prof pr(c, K_PACK);
+        (void)klaunch(k_unpack_state, dim3(592), dim3(256), 0, c->stream, c->zA, c->atd, c->vol,
+                      ax, ay, at);
         CK(cudaGetLastError());
     }
     {
@@ -996,10 +999,7 @@ long long launches_per_step(hqt_ctx *c) {
     // guard, 2 d1 passes of A_t, 4 x (x, y, z), 2 d1 passes of A, zcons, step end
     long long n = 1 + 2 + 4 * 3 + 2 + 1 + 1 + (c->mixed && !c->fused_convert ? 3 : 0);
     if (c->p.remove_winding) n += 2;
-    if (c->p.apply_filter)
-        n += 3;
-    else if (c->p.remove_winding)
-        n += 1;
+    n += c->p.apply_filter ? 3 : 1 + (c->p.remove_winding ? 1 : 0);
     return n;
 }
 
@@ -1020,11 +1020,16 @@ int count_vortices_dev(hqt_ctx *c, const double2 *O, int32_t *n, int32_t *np, in
 }
 
 // Advance the current state nsteps steps.
-// Work on the incoming state before the first step of a call: d_z A_t and,
-// with fused_convert, the FP32 stage-1 copies (later steps get both from the
+// Work on the incoming state before the first step of a call: d_z A_t, the
+// interleaved pairs and, with fused_convert, the FP32 stage-1 copies (later steps get both from the
 // previous step's constraint and filter).
 int prestep(hqt_ctx *c) {
-    RC(launch_zcol_misc(c, c->cat, c->dat, nullptr, nullptr));
+    RC(launch_zcol_misc(c, c->cat, c->atd, nullptr, nullptr));
+    {
+        Prof pr(c, K_PACK);
+        k_pack_pair<<<592, 256, 0, c->stream>>>(c->cax, c->cay, c->vol, c->zA);
+        CK(cudaGetLastError());
+    }
     if (c->fused_convert) RC(enqueue_convert(c));
     return HQT_OK;
 }
@@ -1038,6 +1043,7 @@ int run_steps(hqt_ctx *c, int64_t nsteps, hqt_diag *diag) {
     const long long step0 = h0.step;
     h0.first_bad_step = LLONG_MAX;
     h0.winding = 0;
+    h0.fault = 0;
     CK(cudaMemcpyAsync(c->st, &h0, sizeof(DevStatus), cudaMemcpyHostToDevice, c->stream));
     RC(prestep(c));
     if (!c->prof_on) RC(build_graph(c));
@@ -1078,6 +1084,7 @@ int run_steps(hqt_ctx *c, int64_t nsteps, hqt_diag *diag) {
             DevStatus h{};
             CK(cudaMemcpyAsync(&h, c->st, sizeof(DevStatus), cudaMemcpyDeviceToHost, c->stream));
             CK(cudaStreamSynchronize(c->stream));
+            if (h.fault) return fail(c, HQT_ECUDA, "the radial stage's copies did not arrive");
             if (h.first_bad_step != LLONG_MAX) {
                 bad = true;
                 if (diag) diag->nonfinite_step = h.first_bad_step - step0;
@@ -1441,8 +1448,9 @@ int vortex_compact(hqt_ctx *c, const signed char *q, bool any, int *list0, int *
 // find_vortices (src/diagnostics/find_vortices.m:1-28) of O [nx, ny]
 int find_vortices_dev(hqt_ctx *c, const double2 *O, double threshold, int radius, int capacity,
                       double *vort, double *avort, int32_t *n_out) {
-    signed char *q = reinterpret_cast<signed char *>(c->dxB);
-    int *list0 = reinterpret_cast<int *>(c->dyB), *list1 = list0 + c->plane;
+    // scratch: the two halves of B
+    signed char *q = reinterpret_cast<signed char *>(c->B);
+    int *list0 = reinterpret_cast<int *>(&c->B->x + c->vol), *list1 = list0 + c->plane;
     k_vort_charge<0><<<kPartials, 256, 0, c->stream>>>(O, c->nx, c->ny, q);
     CK(cudaGetLastError());
     int nv = 0, na = 0;
@@ -1478,8 +1486,9 @@ int structure_factor_dev(hqt_ctx *c, const double2 *Phi, double Lx, double Ly, i
                          double *Sc, double *Sn, int32_t *nbins_out, double *spacing) {
     const int n0 = c->nx, n1 = c->ny;  // Ny, Nx of the routine
     const double dx = Lx / n1, dy = Ly / n0;
-    signed char *q = reinterpret_cast<signed char *>(c->dxB);
-    int *list0 = reinterpret_cast<int *>(c->dyB), *list1 = list0 + c->plane;
+    // scratch: the two halves of B
+    signed char *q = reinterpret_cast<signed char *>(c->B);
+    int *list0 = reinterpret_cast<int *>(&c->B->x + c->vol), *list1 = list0 + c->plane;
     k_vort_charge<1><<<kPartials, 256, 0, c->stream>>>(Phi, n0, n1, q);
     CK(cudaGetLastError());
     int nv = 0, unused = 0;
@@ -1699,11 +1708,12 @@ int hqt_create(const hqt_params *params, int device, hqt_ctx **out) {
     A(&c->rho, sizeof(double) * P2);
     for (int b = 0; b < 2; ++b) {
         A(&c->ypsi2[b], sizeof(double2) * V);
-        A(&c->yax2[b], sizeof(double) * V);
-        A(&c->yay2[b], sizeof(double) * V);
+        A(&c->yA2[b], sizeof(double2) * V);
     }
     A(&c->kpsi, sizeof(double2) * V);
     A(&c->kA, sizeof(double2) * V);
+    A(&c->zA, sizeof(double2) * V);
+    A(&c->atd, sizeof(double2) * V);
     A(&c->krho, sizeof(double) * P2);
     A(&c->dxpsi, sizeof(double2) * V);
     A(&c->dxxpsi, sizeof(double2) * V);
@@ -1712,18 +1722,14 @@ int hqt_create(const hqt_params *params, int device, hqt_ctx **out) {
     A(&c->dyypsi, sizeof(double2) * V);
     A(&c->dxxay, sizeof(double) * V);
     A(&c->divA, sizeof(double) * V);
-    A(&c->dxB, sizeof(double) * V);
-    A(&c->dyB, sizeof(double) * V);
-    A(&c->dxat, sizeof(double) * V);
-    A(&c->dyat, sizeof(double) * V);
-    A(&c->dat, sizeof(double) * V);
+    A(&c->B, sizeof(double2) * V);
+    A(&c->dAt, sizeof(double2) * V);
     A(&c->dxax, sizeof(double) * V);
     A(&c->O, sizeof(double2) * P2);
     if (c->mixed) {
         for (int b = 0; b < 3; ++b) {
             A(&c->ypsi32[b], sizeof(float2) * V);
-            A(&c->yax32[b], sizeof(float) * V);
-            A(&c->yay32[b], sizeof(float) * V);
+            A(&c->yA32[b], sizeof(float2) * V);
         }
         A(&c->at32, sizeof(float) * V);
         A(&c->dxpsi32, sizeof(float2) * V);
@@ -1733,10 +1739,8 @@ int hqt_create(const hqt_params *params, int device, hqt_ctx **out) {
         A(&c->dypsi32, sizeof(float2) * V);
         A(&c->dxxay32, sizeof(float) * V);
         A(&c->divA32, sizeof(float) * V);
-        A(&c->dxB32, sizeof(float) * V);
-        A(&c->dyB32, sizeof(float) * V);
-        A(&c->dxat32, sizeof(float) * V);
-        A(&c->dyat32, sizeof(float) * V);
+        A(&c->B32, sizeof(float2) * V);
+        A(&c->dAt32, sizeof(float2) * V);
         A(&c->slice_mean, sizeof(double) * 5 * p.nz);
         A(&c->slice_partial, sizeof(double) * 5 * kSliceChunks * p.nz);
     }
@@ -1808,6 +1812,34 @@ int hqt_create(const hqt_params *params, int device, hqt_ctx **out) {
                 return bail(HQT_ECUDA);
             }
         }
+    }
+    // operand tables and tensor maps of the radial stage
+    {
+        std::vector<double> frag, tab;
+        switch (c->NZP) {
+#define HQT_Z(N)                                   \
+    case N:                                        \
+        z_tables<N>(zhost(c), frag, tab);          \
+        break;
+            HQT_NZP_LIST(HQT_Z)
+#undef HQT_Z
+        }
+        A(&c->zfrag, sizeof(double) * frag.size());
+        A(&c->ztab, sizeof(double) * tab.size());
+        if (rc != HQT_OK) return bail(rc);
+        void *fn = nullptr;
+        cudaDriverEntryPointQueryResult q{};
+        if (cudaMemcpy(c->zfrag, frag.data(), sizeof(double) * frag.size(),
+                       cudaMemcpyHostToDevice) ||
+            cudaMemcpy(c->ztab, tab.data(), sizeof(double) * tab.size(), cudaMemcpyHostToDevice) ||
+            cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &fn, 12000,
+                                             cudaEnableDefault, &q) ||
+            q != cudaDriverEntryPointSuccess) {
+            cudaGetLastError();
+            c->err = "radial-stage set-up failed";
+            return bail(HQT_ECUDA);
+        }
+        c->tmap_encode = reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(fn);
     }
     // launch geometry and shared-memory opt-in
     c->NBx_rhs = pick_lines(p.nx, 3, 32);
@@ -2054,36 +2086,39 @@ int hqt_rhs_device(hqt_ctx *c, const void *dZ1, const void *dZ2, const void *dZ3
     DeviceGuard guard(c->device);
     const double2 *psi = (const double2 *)dZ1;
     const double *at = (const double *)dZ2, *ax = (const double *)dZ3, *ay = (const double *)dZ4;
-    RC(launch_x_d1(c, FieldIn<double>{nullptr, at, nullptr}, FieldOut<double>{nullptr, c->dxat, nullptr}));
+    // (the pairs are scratch here: a run of steps packs its own)
+    {
+        Prof pr(c, K_PACK);
+        k_pack_pair<<<592, 256, 0, c->stream>>>(ax, ay, c->vol, c->zA);
+        CK(cudaGetLastError());
+    }
+    RC(launch_x_d1(c, FieldIn<double>{nullptr, at, nullptr},
+                   FieldOut<double>{nullptr, &c->dAt->x, nullptr, 2}));
     RC(launch_y_d1(c, FieldIn<double>{nullptr, at, nullptr}, nullptr,
-                   FieldOut<double>{nullptr, c->dyat, nullptr}));
-    RC(launch_zcol_misc(c, at, c->dat, nullptr, nullptr));
-    RC(launch_x_rhs(c, psi, ax, ay));
-    RC(launch_y_rhs(c, psi, ax, ay));
-    ZStageArgs<double, double> a{};
-    a.nz = c->nz;
-    a.plane = c->plane;
-    a.h = c->p.dt;
+                   FieldOut<double>{nullptr, &c->dAt->y, nullptr, 2}));
+    RC(launch_zcol_misc(c, at, c->atd, nullptr, nullptr));
+    RC(launch_x_rhs(c, psi, c->zA));
+    RC(launch_y_rhs(c, psi, c->zA));
+    ZStageArgs<double> a{};
     a.ypsi = psi;
-    a.yax = ax;
-    a.yay = ay;
-    a.at = at;
-    a.dat = c->dat;
-    a.dxat = c->dxat;
-    a.dyat = c->dyat;
+    a.yA = c->zA;
+    a.atd = c->atd;
+    a.dAt = c->dAt;
     a.dxpsi = c->dxpsi;
     a.dypsi = c->dypsi;
     a.dxxpsi = c->dxxpsi;
     a.dyypsi = c->dyypsi;
     a.divA = c->divA;
-    a.dxB = c->dxB;
-    a.dyB = c->dyB;
+    a.B = c->B;
     a.f1 = (double2 *)dF1;
     a.f3 = (double *)dF3;
     a.f4 = (double *)dF4;
     a.f2b = (double *)dF2b;
-    RC(launch_zstage<0>(c, a));
+    RC(launch_zstage<double>(c, 0, a));
+    int fault = 0;
+    CK(cudaMemcpyAsync(&fault, &c->st->fault, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
     CK(cudaStreamSynchronize(c->stream));
+    if (fault) return fail(c, HQT_ECUDA, "the radial stage's copies did not arrive");
     return HQT_OK;
 }
 
@@ -2371,6 +2406,7 @@ int hqt_ensemble_step_device(hqt_ensemble *e, void *const *dZ1, void *const *dZ2
             step0[i] = h0.step;
             h0.first_bad_step = LLONG_MAX;
             h0.winding = 0;
+            h0.fault = 0;
             CK(cudaMemcpyAsync(c->st, &h0, sizeof(DevStatus), cudaMemcpyHostToDevice, c->stream));
             {
                 Prof pr(c, K_RHO);
@@ -2407,6 +2443,9 @@ int hqt_ensemble_step_device(hqt_ensemble *e, void *const *dZ1, void *const *dZ2
                 EK(cudaMemcpyAsync(&hs[i], e->m[i]->st, sizeof(DevStatus),
                                    cudaMemcpyDeviceToHost, e->stream));
             EK(cudaStreamSynchronize(e->stream));
+            for (size_t i = 0; i < n; ++i)
+                if (hs[i].fault)
+                    return efail(e, HQT_ECUDA, "the radial stage's copies did not arrive");
             for (size_t i = 0; i < n; ++i)
                 if (hs[i].first_bad_step != LLONG_MAX) {
                     bad = true;

@@ -1,5 +1,7 @@
 // hqt_args.h -- kernel argument blocks (plain structs, host and device).
 #pragma once
+#include <cuda.h>
+
 #include "hqt_common.cuh"
 #include "hqt_lineplan.h"
 
@@ -9,14 +11,18 @@ constexpr int kMaxFilt = 4;
 
 template <typename T> struct FieldIn {
     const C2<T> *c;  // interleaved complex source, or
-    const T *re;     // split real / imaginary sources (im may be null)
+    const T *re;     // split real / imaginary sources (im may be null),
     const T *im;
+    int st = 1;  // elements st apart (2: one part of an interleaved pair; only
+                 // for a real field, im null)
 };
 
 template <typename T> struct FieldOut {
-    C2<T> *c;
-    T *re;
+    C2<T> *c;  // interleaved, and/or
+    T *re;     // split parts (each may be null),
     T *im;
+    int st = 1;  // elements st apart (2: one part of an interleaved pair; only
+                 // for a real field, c and im null)
 };
 
 // A first derivative of one real field into one real field: the line
@@ -34,7 +40,7 @@ template <typename T> struct XRhsArgs {
     int NB, nlines;
     T s1, s2;
     const C2<T> *psi;
-    const T *ax, *ay;
+    const C2<T> *A;  // (A_x, A_y)
     C2<T> *dxpsi, *dxxpsi, *E;
     T *dxxay;
 };
@@ -46,11 +52,12 @@ template <typename T> struct YRhsArgs {
     int TX, nx, ny;
     T s1, s2;
     const C2<T> *psi;
-    const T *ax, *ay;
+    const C2<T> *A;  // (A_x, A_y)
     const C2<T> *E;  // d_x A_x + i d_x A_y
     const T *dxxay;
     C2<T> *dypsi, *dyypsi;  // (the radial stage forms lap Psi = d_xx Psi + d_yy Psi)
-    T *divA, *dxB, *dyB;
+    T *divA;
+    C2<T> *B;  // (d_y B, d_x B)
 };
 
 template <typename T> struct XD1Args {
@@ -114,13 +121,12 @@ template <typename T> struct XFiltInvArgs {
     FieldOut<T> out[kMaxFilt];
     DevStatus *st;  // non-finite check when non-null
     // optional FP32 copies minus the slice means (slice_mean[5*z + slot]):
-    // interleaved c32[f], or re32[f] / im32[f]; z = line / ny
+    // interleaved c32[f], or re32[f]; z = line / ny
     const T *slice_mean = nullptr;
     int slot[kMaxFilt][2] = {};
     int ny = 0;
     C2<float> *c32[kMaxFilt] = {};
     float *re32[kMaxFilt] = {};
-    float *im32[kMaxFilt] = {};
     int dead0 = 1, dead1 = 0;  // spectral columns dead0 <= kx <= dead1 read as zero
 };
 
@@ -132,38 +138,43 @@ template <typename T, int NZP> struct ZOps {
     T lzb[NZP];  // boundary row Lz(nz, :)
 };
 
-// T: stage-input and arithmetic type, TS: state / accumulator type,
-// TD: type of the horizontal-derivative fields written by the line passes.
-template <typename T, typename TS, typename TD = T> struct ZStageArgs {
+// Radial stage (hqt_zstage.cuh).  TD: type of the horizontal-derivative fields
+// written by the line passes; all else is FP64.  Pairs of real fields are
+// interleaved.  Inputs come by the tensor maps, or by the pointers where a
+// field's level rows are not 16 bytes apart modulo 16 (copy_pairs: the TD pairs,
+// copy_real: div A).
+template <typename TD> struct ZStageArgs {
+    CUtensorMap mPS, mAXY;        // stage input Psi, (A_x, A_y)
+    CUtensorMap mDX, mDY;         // d_x Psi, d_y Psi
+    CUtensorMap mDT, mB;          // (d_x A_t, d_y A_t), (d_y B, d_x B)
+    CUtensorMap mZA, mKA;         // state and RK accumulator of (A_x, A_y)
+    CUtensorMap mATD;             // (A_t, d_z A_t)
+    CUtensorMap mXX, mYY, mDIV;   // d_xx Psi, d_yy Psi (their sum is lap Psi), div A
+    CUtensorMap mZP, mKP;         // state and RK accumulator of Psi
     int nz;
+    int copy_pairs, copy_real;
     long long plane;  // nx*ny
-    TS h;
-    // stage inputs
-    const C2<T> *ypsi;
-    const T *yax, *yay;
-    const T *at, *dat;
-    const TD *dxat, *dyat;
-    const C2<TD> *dxpsi, *dypsi, *dxxpsi, *dyypsi;  // lap Psi = dxxpsi + dyypsi
-    const TD *divA, *dxB, *dyB;
-    // RK state and accumulators (type TS)
-    const C2<TS> *zpsi;
-    const TS *zax, *zay, *zrho;
-    C2<TS> *kpsi;
-    C2<TS> *kA;  // (A_x, A_y) accumulator, interleaved: staged by 16-byte copies
-    TS *krho;
-    C2<T> *npsi;  // next stage input
-    T *nax, *nay;
-    C2<TD> *npsi_d;  // its copy in the derivative type (mixed precision; may be null)
-    TD *nax_d, *nay_d;
-    // per z-slice plane means (psi re, psi im, A_t, A_x, A_y), subtracted from
-    // the copies above: the line passes only differentiate, and the smaller
-    // magnitude rounds to FP32 with a smaller error
-    const TS *slice_mean;
-    C2<TS> *wpsi;  // new state (stage 4)
-    TS *wax, *way, *wrho;
-    // right-hand-side outputs (MODE 0)
-    C2<T> *f1;
-    T *f3, *f4, *f2b;
+    double h;
+    const double *frag;  // operator fragments per lane (make_zstage_tables)
+    const double *ztab;  // z, 1 - z^3, Lz(nz,:), NZP each
+    const double2 *ypsi, *yA, *atd;
+    const C2<TD> *dxpsi, *dypsi, *dAt, *B, *dxxpsi, *dyypsi;
+    const TD *divA;
+    const double2 *zpsi, *zA;
+    const double *zrho;
+    double2 *kpsi, *kA;
+    double *krho;
+    double2 *npsi, *nA;       // next stage input
+    C2<TD> *npsi_d, *nA_d;    // its copy in the derivative type (TD float only),
+    // minus the plane means of its z slice (psi re, psi im, A_t, A_x, A_y): the
+    // line passes only differentiate, and the smaller magnitude rounds to FP32
+    // with a smaller error
+    const double *slice_mean;
+    double2 *wpsi, *wA;       // new state (stage 4)
+    double *wrho;
+    double2 *f1;              // right-hand-side outputs (MODE 0)
+    double *f3, *f4, *f2b;
+    int *fault;               // set when a copy did not arrive
 };
 
 template <typename T> struct ZConsArgs {
@@ -171,7 +182,8 @@ template <typename T> struct ZConsArgs {
     long long plane;
     T mu, vy;
     C2<T> *psi;
-    T *ax, *ay, *at, *dat;
+    C2<T> *A;    // (A_x, A_y): boundary row
+    C2<T> *atd;  // (A_t, d_z A_t)
     const T *divA;
     const T *rho;  // 2-D
     C2<T> *O;      // 2-D boundary order parameter (may be null)
@@ -181,7 +193,7 @@ template <typename T> struct ZColArgs {
     int nz;
     long long plane;
     const T *at;
-    T *dat;
+    C2<T> *atd;  // (A_t, d_z A_t) of at
     const C2<T> *psi;
     C2<T> *O;
 };

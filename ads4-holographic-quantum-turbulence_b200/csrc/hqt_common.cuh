@@ -157,6 +157,7 @@ struct DevStatus {
     long long first_bad_step;  // first step (1-based) with a non-finite value, or LLONG_MAX
     int winding;               // winding removed at the most recent step
     int n_records;             // vortex-count records written
+    int fault;                 // a kernel gave up waiting for its copies
 };
 
 }  // namespace hqt

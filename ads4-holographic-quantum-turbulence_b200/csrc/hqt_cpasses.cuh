@@ -31,21 +31,18 @@ __device__ __forceinline__ void cx_store(int buf, int valid, F put) {
         if (b < valid) put(t, s[e * NB + b]);
     }
 }
-// (re, im) of two real fields into the x-line layout of cx_load by cp.async
-// (zero past `valid`); the caller commits and waits
+// a complex field into the x-line layout of cx_load by cp.async (zero past
+// `valid`); the caller commits and waits
 template <typename T, int N, int NB>
-__device__ __forceinline__ void cx_load_pair_async(int buf, int valid, long long g0, const T *re,
-                                                   const T *im) {
+__device__ __forceinline__ void cx_load_async(int buf, int valid, long long g0, const C2<T> *src) {
     const CtView<T, N> s = ctv<T, N>(buf);
     for (int t = threadIdx.x; t < N * NB; t += ct_threads<T, N, NB>()) {
         const int b = t / N, e = t - b * N;
         C2<T> &d = s[e * NB + b];
-        if (b < valid) {
-            cp_async<sizeof(T)>(&d.x, re + g0 + t);
-            cp_async<sizeof(T)>(&d.y, im + g0 + t);
-        } else {
+        if (b < valid)
+            cp_async<sizeof(C2<T>)>(&d, src + g0 + t);
+        else
             d = mk2<T>(T(0), T(0));
-        }
     }
 }
 // y lines: NB adjacent columns of one z slice; element (y, b) at y*NB + b
@@ -65,8 +62,8 @@ __device__ __forceinline__ void cy_store(int buf, int valid, int nx, long long z
         if (b < valid) put(zoff + (long long)y * nx + b, s[t]);
     }
 }
-// cy_load by cp.async of a complex field, or of the pair (re, im) of two
-// real fields (zero past `valid`); the caller commits and waits
+// cy_load by cp.async of a complex field (zero past `valid`); the caller
+// commits and waits
 template <typename T, int N, int NB>
 __device__ __forceinline__ void cy_load_async(int buf, int valid, int nx, long long zoff,
                                               const C2<T> *src) {
@@ -77,22 +74,6 @@ __device__ __forceinline__ void cy_load_async(int buf, int valid, int nx, long l
             cp_async<sizeof(C2<T>)>(&s[t], src + zoff + (long long)y * nx + b);
         else
             s[t] = mk2<T>(T(0), T(0));
-    }
-}
-template <typename T, int N, int NB>
-__device__ __forceinline__ void cy_load_pair_async(int buf, int valid, int nx, long long zoff,
-                                                   const T *re, const T *im) {
-    const CtView<T, N> s = ctv<T, N>(buf);
-    for (int t = threadIdx.x; t < N * NB; t += ct_threads<T, N, NB>()) {
-        const int y = t / NB, b = t - y * NB;
-        C2<T> &d = s[t];
-        if (b < valid) {
-            const long long g = zoff + (long long)y * nx + b;
-            cp_async<sizeof(T)>(&d.x, re + g);
-            cp_async<sizeof(T)>(&d.y, im + g);
-        } else {
-            d = mk2<T>(T(0), T(0));
-        }
     }
 }
 // cy_store whose put(g, v, x) also takes x = get(g), a global value of the
@@ -142,7 +123,7 @@ __global__ void HQT_CT_BOUNDS k_x_rhs_c(XRhsArgs<T> a) {
     __syncthreads();
     // r1's buffer is free: C = A_x + i A_y comes into it while d_xx Psi is
     // transformed and stored
-    cx_load_pair_async<T, N, NB>(r1, valid, g0, a.ax, a.ay);
+    cx_load_async<T, N, NB>(r1, valid, g0, a.A);
     cp_commit();
     const int fr = (r1 == Y) ? C : Y;
     const int r2 = ct_fft<T, N, NB, +1>(X, fr, R);
@@ -185,7 +166,7 @@ __global__ void HQT_CT_BOUNDS k_y_rhs_c(YRhsArgs<T> a) {
     // C = A_x + i A_y and E = d_x C, each transformed, then paired.  C comes
     // into r1's buffer (free now) while d_yy Psi is transformed and stored,
     // E into a third buffer while C is transformed.
-    cy_load_pair_async<T, N, NB>(r1, valid, a.nx, zoff, a.ax, a.ay);
+    cy_load_async<T, N, NB>(r1, valid, a.nx, zoff, a.A);
     cp_commit();
     const int fr = (r1 == Y) ? C : Y;
     const int r2 = ct_fft<T, N, NB, +1>(X, fr, R);
@@ -240,9 +221,9 @@ __global__ void HQT_CT_BOUNDS k_y_rhs_c(YRhsArgs<T> a) {
             P1, valid, a.nx, zoff, [&](long long g) { return mk2<T>(a.E[g].x, a.dxxay[g]); },
             [&](long long g, C2<T> v, C2<T> x) {
                 a.divA[g] = x.x + v.x;
-                a.dxB[g] = x.y + v.y;
+                a.B[g].y = x.y + v.y;
             });
-        cy_store<T, N, NB>(P2, valid, a.nx, zoff, [&](long long g, C2<T> v) { a.dyB[g] = v.x; });
+        cy_store<T, N, NB>(P2, valid, a.nx, zoff, [&](long long g, C2<T> v) { a.B[g].x = v.x; });
     }
 }
 
@@ -302,7 +283,8 @@ __global__ void HQT_CT_BOUNDS k_x_d1r_c(XD1Args<T> a) {
     const int valid = (nr + 1) / 2;
     constexpr int R = 0, A = N, B = N + NB * N;
     const T *src = a.in.re + (long long)L0 * N;
-    T *dst = a.out.re + (long long)L0 * N;
+    const int so = a.out.st;
+    T *dst = a.out.re + (long long)L0 * N * so;
     ct_load_roots<T, N>(R, a.roots);
     pdl_wait();
     cx_load<T, N, NB>(A, valid, [&](int t) {
@@ -319,8 +301,8 @@ __global__ void HQT_CT_BOUNDS k_x_d1r_c(XD1Args<T> a) {
     cx_store<T, N, NB>(r, valid, [&](int t, C2<T> v) {
         const int j = t / N, e = t - j * N;
         const int r0 = 2 * j, r1 = r0 + 1;
-        if (r0 < nr) dst[(long long)r0 * N + e] = v.x;
-        if (r1 < nr) dst[(long long)r1 * N + e] = v.y;
+        if (r0 < nr) dst[((long long)r0 * N + e) * so] = v.x;
+        if (r1 < nr) dst[((long long)r1 * N + e) * so] = v.y;
     });
 }
 
@@ -368,8 +350,8 @@ __global__ void HQT_CT_BOUNDS k_y_d1r_c(YD1Args<T> a) {
             const int r0 = 2 * j, r1 = r0 + 1;
             const long long gy = zoff + (long long)y * a.nx;
             const C2<T> v = sr[t];
-            if (r0 < nr) a.out.re[gy + r0] = v.x + x[i].x;
-            if (r1 < nr) a.out.re[gy + r1] = v.y + x[i].y;
+            if (r0 < nr) a.out.re[(gy + r0) * a.out.st] = v.x + x[i].x;
+            if (r1 < nr) a.out.re[(gy + r1) * a.out.st] = v.y + x[i].y;
         }
     }
 }

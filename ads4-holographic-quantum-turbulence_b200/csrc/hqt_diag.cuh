@@ -157,8 +157,7 @@ __global__ void k_slice_finalize(const double *partial, int nz, long long plane,
 // (mixed precision).
 __global__ void k_state_to_f32(const double2 *psi, const double *at, const double *ax,
                                const double *ay, long long plane, long long vol,
-                               const double *mean, float2 *psi32, float *at32, float *ax32,
-                               float *ay32) {
+                               const double *mean, float2 *psi32, float *at32, float2 *A32) {
     pdl_wait();
     for (long long s = (long long)blockIdx.x * blockDim.x + threadIdx.x; s < vol;
          s += (long long)gridDim.x * blockDim.x) {
@@ -166,8 +165,26 @@ __global__ void k_state_to_f32(const double2 *psi, const double *at, const doubl
         const double2 p = psi[s];
         psi32[s] = make_float2((float)(p.x - m[0]), (float)(p.y - m[1]));
         at32[s] = (float)(at[s] - m[2]);
-        ax32[s] = (float)(ax[s] - m[3]);
-        ay32[s] = (float)(ay[s] - m[4]);
+        A32[s] = make_float2((float)(ax[s] - m[3]), (float)(ay[s] - m[4]));
+    }
+}
+
+// (A_x, A_y) interleaved, the layout in which a step keeps them: 16-byte
+// loads in the line and column passes.  And back, with A_t from (A_t, d_z A_t).
+__global__ void k_pack_pair(const double *x, const double *y, long long n, double2 *p) {
+    for (long long s = (long long)blockIdx.x * blockDim.x + threadIdx.x; s < n;
+         s += (long long)gridDim.x * blockDim.x)
+        p[s] = make_double2(x[s], y[s]);
+}
+__global__ void k_unpack_state(const double2 *A, const double2 *atd, long long n, double *ax,
+                               double *ay, double *at) {
+    pdl_wait();
+    for (long long s = (long long)blockIdx.x * blockDim.x + threadIdx.x; s < n;
+         s += (long long)gridDim.x * blockDim.x) {
+        const double2 v = A[s];
+        ax[s] = v.x;
+        ay[s] = v.y;
+        at[s] = atd[s].x;
     }
 }
 

@@ -3,6 +3,7 @@
 #include <cuda_runtime.h>
 
 #include <utility>
+#include <vector>
 
 #include "hqt_args.h"
 
@@ -92,11 +93,9 @@ cudaError_t pfa_launch_301(int kind, const void *args, int nlines, cudaStream_t 
 // mode 0: right-hand side only, 1..4: RK stage.
 template <int N> cudaError_t z_init(int max_smem);
 template <int N>
-cudaError_t z_stage(int mode, const ZStageArgs<double, double> &a, const ZHost &h, int grid,
-                    int threads, size_t smem, cudaStream_t s);
-template <int N>
-cudaError_t z_stage_mixed(int mode, const ZStageArgs<double, double, float> &a, const ZHost &h,
-                          int grid, int threads, size_t smem, cudaStream_t s);
+void z_tables(const ZHost &h, std::vector<double> &frag, std::vector<double> &tab);
+template <int N> cudaError_t z_stage(int mode, const ZStageArgs<double> &a, cudaStream_t s);
+template <int N> cudaError_t z_stage_mixed(int mode, const ZStageArgs<float> &a, cudaStream_t s);
 template <int N>
 cudaError_t z_cons(const ZConsArgs<double> &a, const ZHost &h, cudaStream_t s);
 template <int N>
@@ -117,11 +116,9 @@ namespace hqt {
 #define HQT_ZDECL(N)                                                                       \
     template <> cudaError_t z_init<N>(int);                                                \
     template <>                                                                            \
-    cudaError_t z_stage<N>(int, const ZStageArgs<double, double> &, const ZHost &, int, int, \
-                           size_t, cudaStream_t);                                          \
-    template <>                                                                            \
-    cudaError_t z_stage_mixed<N>(int, const ZStageArgs<double, double, float> &,            \
-                                 const ZHost &, int, int, size_t, cudaStream_t);           \
+    void z_tables<N>(const ZHost &, std::vector<double> &, std::vector<double> &);         \
+    template <> cudaError_t z_stage<N>(int, const ZStageArgs<double> &, cudaStream_t);     \
+    template <> cudaError_t z_stage_mixed<N>(int, const ZStageArgs<float> &, cudaStream_t); \
     template <>                                                                            \
     cudaError_t z_cons<N>(const ZConsArgs<double> &, const ZHost &, cudaStream_t);             \
     template <>                                                                            \

@@ -37,7 +37,7 @@ __global__ void HQT_L_BOUNDS(G) k_lx_rhs(const __grid_constant__ XRhsArgs<T> a) 
         w.first(w.A, [&](int b, int e) {
             if (b >= valid) return lzero<T>();
             const long long g = at(b, e);
-            return f == 0 ? a.psi[g] : mk2<T>(a.ax[g], a.ay[g]);
+            return f == 0 ? a.psi[g] : a.A[g];
         });
         w.forward_mid(1);
         w.middle_deriv12(a.s1, a.s2);
@@ -76,12 +76,12 @@ __global__ void HQT_L_BOUNDS(G) k_ly_rhs(const __grid_constant__ YRhsArgs<T> a) 
             w.first(w.A, [&](int b, int e) {
                 if (b >= valid) return lzero<T>();
                 const long long g = at(b, e);
-                return mk2<T>(a.E[g].x, a.ay[g]);
+                return mk2<T>(a.E[g].x, a.A[g].y);
             });
             w.first(w.B, [&](int b, int e) {
                 if (b >= valid) return lzero<T>();
                 const long long g = at(b, e);
-                return mk2<T>(a.ax[g], a.E[g].y);
+                return mk2<T>(a.A[g].x, a.E[g].y);
             });
         }
         w.forward_mid(1 + f);
@@ -111,10 +111,10 @@ __global__ void HQT_L_BOUNDS(G) k_ly_rhs(const __grid_constant__ YRhsArgs<T> a) 
                     if (b >= valid) return;
                     const long long g = at(b, e);
                     a.divA[g] = x.x + v.y;
-                    a.dxB[g] = x.y - v.x;
+                    a.B[g].y = x.y - v.x;
                 });
             w.last(w.B, [&](int b, int e, C2<T> v) {
-                if (b < valid) a.dyB[at(b, e)] = v.x;
+                if (b < valid) a.B[at(b, e)].x = v.x;
             });
         }
     }
@@ -165,20 +165,21 @@ template <typename T, class G>
 __global__ void HQT_L_BOUNDS1(G) k_lx_d1r(const __grid_constant__ XD1Args<T> a) {
     const LineEng<T, G> w(a.lt);
     const int n = w.g.n(), L0 = blockIdx.x << (w.g.nbl() + 1), nr = a.nlines - L0;
-    const T *src = a.in.re + (long long)L0 * n;
-    T *dst = a.out.re + (long long)L0 * n;
+    const int si = a.in.st, so = a.out.st;
+    const T *src = a.in.re + (long long)L0 * n * si;
+    T *dst = a.out.re + (long long)L0 * n * so;
     pdl_wait();
     w.first(w.A, [&](int b, int e) {
         const long long g = 2ll * b * n + e;
-        return mk2<T>(2 * b < nr ? src[g] : T(0), 2 * b + 1 < nr ? src[g + n] : T(0));
+        return mk2<T>(2 * b < nr ? src[g * si] : T(0), 2 * b + 1 < nr ? src[(g + n) * si] : T(0));
     });
     w.forward_mid(1);
     w.middle_deriv1(w.A, a.s1);
     w.inverse_mid(1);
     w.last(w.A, [&](int b, int e, C2<T> v) {
         const long long g = 2ll * b * n + e;
-        if (2 * b < nr) dst[g] = v.x;
-        if (2 * b + 1 < nr) dst[g + n] = v.y;
+        if (2 * b < nr) dst[g * so] = v.x;
+        if (2 * b + 1 < nr) dst[(g + n) * so] = v.y;
     });
 }
 
@@ -188,20 +189,21 @@ __global__ void HQT_L_BOUNDS1(G) k_ly_d1r(const __grid_constant__ YD1Args<T> a) 
     const int x0 = blockIdx.x << (w.g.nbl() + 1), nr = a.nx - x0;
     const long long zoff = (long long)blockIdx.y * a.ny * a.nx + x0;
     pdl_wait();
-    auto pair = [&](const T *p, int b, int e) {
-        const long long g = zoff + (long long)e * a.nx + 2 * b;
-        return mk2<T>(2 * b < nr ? p[g] : T(0), 2 * b + 1 < nr ? p[g + 1] : T(0));
+    auto pair = [&](const T *p, int st, int b, int e) {
+        const long long g = (zoff + (long long)e * a.nx + 2 * b) * st;
+        return mk2<T>(2 * b < nr ? p[g] : T(0), 2 * b + 1 < nr ? p[g + st] : T(0));
     };
-    w.first(w.A, [&](int b, int e) { return pair(a.in.re, b, e); });
+    w.first(w.A, [&](int b, int e) { return pair(a.in.re, a.in.st, b, e); });
     w.forward_mid(1);
     w.middle_deriv1(w.A, a.s1);
     w.inverse_mid(1);
     w.last(
-        w.A, [&](int b, int e) { return a.add_re ? pair(a.add_re, b, e) : lzero<T>(); },
+        w.A, [&](int b, int e) { return a.add_re ? pair(a.add_re, 1, b, e) : lzero<T>(); },
         [&](int b, int e, C2<T> v, C2<T> x) {
-            const long long g = zoff + (long long)e * a.nx + 2 * b;
+            const int st = a.out.st;
+            const long long g = (zoff + (long long)e * a.nx + 2 * b) * st;
             if (2 * b < nr) a.out.re[g] = v.x + x.x;
-            if (2 * b + 1 < nr) a.out.re[g + 1] = v.y + x.y;
+            if (2 * b + 1 < nr) a.out.re[g + st] = v.y + x.y;
         });
 }
 

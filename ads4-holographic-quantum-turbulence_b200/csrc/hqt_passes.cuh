@@ -38,17 +38,14 @@ __device__ __forceinline__ int wavenum(int k, int n) {
 template <typename T>
 __device__ __forceinline__ C2<T> load_field(const FieldIn<T> &f, long long idx) {
     if (f.c) return f.c[idx];
-    return mk2<T>(f.re[idx], f.im ? f.im[idx] : T(0));
+    return mk2<T>(f.re[idx * f.st], f.im ? f.im[idx] : T(0));
 }
 
 template <typename T>
 __device__ __forceinline__ void store_field(const FieldOut<T> &f, long long idx,
                                             C2<T> v) {
-    if (f.c) {
-        f.c[idx] = v;
-        return;
-    }
-    if (f.re) f.re[idx] = v.x;
+    if (f.c) f.c[idx] = v;
+    if (f.re) f.re[idx * f.st] = v.x;
     if (f.im) f.im[idx] = v.y;
 }
 
@@ -175,7 +172,7 @@ template <typename T> __global__ void HQT_FFT_BOUNDS k_x_rhs(XRhsArgs<T> a) {
     xl_store<T>(r2, n, nb, [&](int t, C2<T> v) { a.dxxpsi[g0 + t] = v; });
     __syncthreads();
     // ---- A_x + i A_y ----
-    xl_load<T>(A, n, nb, [&](int t) { return mk2<T>(a.ax[g0 + t], a.ay[g0 + t]); });
+    xl_load<T>(A, n, nb, [&](int t) { return a.A[g0 + t]; });
     __syncthreads();
     X = fft_run<T>(A, B, R, a.plan, nb, -1);
     Y = (X == A) ? B : A;
@@ -226,7 +223,7 @@ template <typename T> __global__ void HQT_FFT_BOUNDS k_y_rhs(YRhsArgs<T> a) {
         for (int t = threadIdx.x; t < tot; t += blockDim.x) {
             const int y = t / nb, b = t - y * nb;
             const long long g = zoff + (long long)y * a.nx + b;
-            s[y * nb2 + b] = mk2<T>(a.ax[g], a.ay[g]);
+            s[y * nb2 + b] = a.A[g];
             s[y * nb2 + nb + b] = a.E[g];
         }
     }
@@ -279,8 +276,7 @@ template <typename T> __global__ void HQT_FFT_BOUNDS k_y_rhs(YRhsArgs<T> a) {
                 const C2<T> p1 = s[y * nb2 + b];
                 const C2<T> p2 = s[y * nb2 + nb + b];
                 a.divA[g] = x.x + p1.x;
-                a.dxB[g] = x.y + p1.y;
-                a.dyB[g] = p2.x;
+                a.B[g] = mk2<T>(p2.x, x.y + p1.y);
             });
     }
 }

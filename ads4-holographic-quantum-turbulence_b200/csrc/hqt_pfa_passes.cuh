@@ -89,7 +89,7 @@ template <typename T, int P, int Q> struct PfaLines {
                     cp_async<sizeof(T)>(dst.re + i, &f.c[g].x);
                     cp_async<sizeof(T)>(dst.im + i, &f.c[g].y);
                 } else {
-                    cp_async<sizeof(T)>(dst.re + i, f.re + g);
+                    cp_async<sizeof(T)>(dst.re + i, f.re + g * f.st);
                     if (f.im)
                         cp_async<sizeof(T)>(dst.im + i, f.im + g);
                     else
@@ -161,8 +161,8 @@ __global__ void __launch_bounds__(32) k_x_rhs_pfa(const __grid_constant__ XRhsAr
     __syncwarp();
     deriv(O2{});
     // C = A_x + i A_y loads while the inverse runs
-    L.fetch(L.b0, [&](int ln, int n) { return &a.ax[gi(ln, n)]; },
-            [&](int ln, int n) { return &a.ay[gi(ln, n)]; });
+    L.fetch(L.b0, [&](int ln, int n) { return &a.A[gi(ln, n)].x; },
+            [&](int ln, int n) { return &a.A[gi(ln, n)].y; });
     cp_commit();
     inverse();
     L.each([&](int ln, int n, int i) { a.dxxpsi[gi(ln, n)] = mk2<T>(L.b1.re[i], L.b1.im[i]); });
@@ -228,11 +228,11 @@ __global__ void __launch_bounds__(32) k_y_rhs_pfa(const __grid_constant__ YRhsAr
     // form (W1 = E_x + i A_y, W2 = A_x + i E_y, below).
     constexpr bool kF64 = std::is_same<T, double>::value;
     if constexpr (kF64)
-        L.fetch(L.b0, [&](int ln, int n) { return &a.ax[gi(ln, n)]; },
-                [&](int ln, int n) { return &a.ay[gi(ln, n)]; });
+        L.fetch(L.b0, [&](int ln, int n) { return &a.A[gi(ln, n)].x; },
+                [&](int ln, int n) { return &a.A[gi(ln, n)].y; });
     else
         L.fetch(L.b0, [&](int ln, int n) { return &a.E[gi(ln, n)].x; },
-                [&](int ln, int n) { return &a.ay[gi(ln, n)]; });
+                [&](int ln, int n) { return &a.A[gi(ln, n)].y; });
     cp_commit();
     inverse(L.b1);
     L.each([&](int ln, int n, int i) { a.dyypsi[gi(ln, n)] = mk2<T>(L.b1.re[i], L.b1.im[i]); });
@@ -241,7 +241,7 @@ __global__ void __launch_bounds__(32) k_y_rhs_pfa(const __grid_constant__ YRhsAr
         L.fetch(L.b1, [&](int ln, int n) { return &a.E[gi(ln, n)].x; },
                 [&](int ln, int n) { return &a.E[gi(ln, n)].y; });
     else
-        L.fetch(L.b1, [&](int ln, int n) { return &a.ax[gi(ln, n)]; },
+        L.fetch(L.b1, [&](int ln, int n) { return &a.A[gi(ln, n)].x; },
                 [&](int ln, int n) { return &a.E[gi(ln, n)].y; });
     cp_commit();
     cp_wait<1>();
@@ -335,7 +335,7 @@ __global__ void __launch_bounds__(32) k_y_rhs_pfa(const __grid_constant__ YRhsAr
         }
         __syncwarp();
         inverse(L.b1);
-        L.each([&](int ln, int n, int i) { a.dyB[gi(ln, n)] = L.b1.re[i]; });
+        L.each([&](int ln, int n, int i) { a.B[gi(ln, n)].x = L.b1.re[i]; });
         __syncwarp();
         L.fetch(L.b1, [&](int ln, int n) { return &a.E[gi(ln, n)].x; },
                 [&](int ln, int n) { return &a.dxxay[gi(ln, n)]; });
@@ -345,7 +345,7 @@ __global__ void __launch_bounds__(32) k_y_rhs_pfa(const __grid_constant__ YRhsAr
         __syncwarp();
         L.each([&](int ln, int n, int i) {
             a.divA[gi(ln, n)] = L.b1.re[i] + L.b0.re[i];
-            a.dxB[gi(ln, n)] = L.b1.im[i] + L.b0.im[i];
+            a.B[gi(ln, n)].y = L.b1.im[i] + L.b0.im[i];
         });
     } else {
         // The gauge fields as two complex lines whose y derivatives give the
@@ -363,7 +363,7 @@ __global__ void __launch_bounds__(32) k_y_rhs_pfa(const __grid_constant__ YRhsAr
         });
         __syncwarp();
         inverse(L.b1);
-        L.each([&](int ln, int n, int i) { a.dyB[gi(ln, n)] = L.b1.re[i]; });
+        L.each([&](int ln, int n, int i) { a.B[gi(ln, n)].x = L.b1.re[i]; });
         __syncwarp();
         L.fetch(L.b1, [&](int ln, int n) { return &a.E[gi(ln, n)].x; },
                 [&](int ln, int n) { return &a.dxxay[gi(ln, n)]; });
@@ -373,18 +373,15 @@ __global__ void __launch_bounds__(32) k_y_rhs_pfa(const __grid_constant__ YRhsAr
         __syncwarp();
         L.each([&](int ln, int n, int i) {
             a.divA[gi(ln, n)] = L.b1.re[i] + L.b0.im[i];
-            a.dxB[gi(ln, n)] = L.b1.im[i] - L.b0.re[i];
+            a.B[gi(ln, n)].y = L.b1.im[i] - L.b0.re[i];
         });
     }
 }
 
 template <typename T>
 __device__ __forceinline__ void pfa_store_field(const FieldOut<T> &f, long long idx, T re, T im) {
-    if (f.c) {
-        f.c[idx] = mk2<T>(re, im);
-        return;
-    }
-    if (f.re) f.re[idx] = re;
+    if (f.c) f.c[idx] = mk2<T>(re, im);
+    if (f.re) f.re[idx * f.st] = re;
     if (f.im) f.im[idx] = im;
 }
 
@@ -463,14 +460,15 @@ __global__ void __launch_bounds__(32) k_x_d1r_pfa(const __grid_constant__ XD1Arg
     const int R0 = blockIdx.x * kPfaRealLines;
     const int nr = min(kPfaRealLines, a.nlines - R0);  // real lines inside the grid
     const L_t L((nr + 1) / 2);
-    const T *src = a.in.re + (long long)R0 * N;
-    T *dst = a.out.re + (long long)R0 * N;
+    const int si = a.in.st, so = a.out.st;
+    const T *src = a.in.re + (long long)R0 * N * si;
+    T *dst = a.out.re + (long long)R0 * N * so;
     for (int e = L.lane; e < L_t::LN; e += 32) {
         const int ln = e % kPfaLines, n = e / kPfaLines, i = L_t::pos(ln, n);
         const int r0 = 2 * ln, r1 = r0 + 1;
-        if (r0 < nr) cp_async<sizeof(T)>(L.b0.re + i, src + (long long)r0 * N + n);
+        if (r0 < nr) cp_async<sizeof(T)>(L.b0.re + i, src + ((long long)r0 * N + n) * si);
         else L.b0.re[i] = T(0);
-        if (r1 < nr) cp_async<sizeof(T)>(L.b0.im + i, src + (long long)r1 * N + n);
+        if (r1 < nr) cp_async<sizeof(T)>(L.b0.im + i, src + ((long long)r1 * N + n) * si);
         else L.b0.im[i] = T(0);
     }
     cp_commit();
@@ -485,8 +483,8 @@ __global__ void __launch_bounds__(32) k_x_d1r_pfa(const __grid_constant__ XD1Arg
     for (int e = L.lane; e < L_t::LN; e += 32) {
         const int ln = e % kPfaLines, n = e / kPfaLines, i = L_t::pos(ln, n);
         const int r0 = 2 * ln, r1 = r0 + 1;
-        if (r0 < nr) dst[(long long)r0 * N + n] = L.b1.re[i];
-        if (r1 < nr) dst[(long long)r1 * N + n] = L.b1.im[i];
+        if (r0 < nr) dst[((long long)r0 * N + n) * so] = L.b1.re[i];
+        if (r1 < nr) dst[((long long)r1 * N + n) * so] = L.b1.im[i];
     }
 }
 
@@ -506,9 +504,9 @@ __global__ void __launch_bounds__(32) k_y_d1r_pfa(const __grid_constant__ YD1Arg
     for (int e = L.lane; e < L_t::LN; e += 32) {
         const int ln = e % kPfaLines, n = e / kPfaLines, i = L_t::pos(ln, n);
         const int r0 = 2 * ln, r1 = r0 + 1;
-        if (r0 < nr) cp_async<sizeof(T)>(L.b0.re + i, a.in.re + gi(r0, n));
+        if (r0 < nr) cp_async<sizeof(T)>(L.b0.re + i, a.in.re + gi(r0, n) * a.in.st);
         else L.b0.re[i] = T(0);
-        if (r1 < nr) cp_async<sizeof(T)>(L.b0.im + i, a.in.re + gi(r1, n));
+        if (r1 < nr) cp_async<sizeof(T)>(L.b0.im + i, a.in.re + gi(r1, n) * a.in.st);
         else L.b0.im[i] = T(0);
     }
     cp_commit();
@@ -525,11 +523,11 @@ __global__ void __launch_bounds__(32) k_y_d1r_pfa(const __grid_constant__ YD1Arg
         const int r0 = 2 * ln, r1 = r0 + 1;
         if (r0 < nr) {
             const long long g = gi(r0, n);
-            a.out.re[g] = L.b1.re[i] + (a.add_re ? a.add_re[g] : T(0));
+            a.out.re[g * a.out.st] = L.b1.re[i] + (a.add_re ? a.add_re[g] : T(0));
         }
         if (r1 < nr) {
             const long long g = gi(r1, n);
-            a.out.re[g] = L.b1.im[i] + (a.add_re ? a.add_re[g] : T(0));
+            a.out.re[g * a.out.st] = L.b1.im[i] + (a.add_re ? a.add_re[g] : T(0));
         }
     }
 }
@@ -697,7 +695,7 @@ __global__ void __launch_bounds__(32) k_x_filt_inv_pfa(const __grid_constant__ X
         cp_commit();
         w.template stage_a<+1>(L.b1, L_t::in_place(L.b1));
         __syncwarp();
-        const bool f32 = a.slice_mean && (a.c32[f] || a.re32[f] || a.im32[f]);
+        const bool f32 = a.slice_mean && (a.c32[f] || a.re32[f]);
         if (!f32) {
             L.each([&](int ln, int n, int i) {
                 const double re = L.b1.re[i], im = L.b1.im[i];
@@ -716,7 +714,7 @@ __global__ void __launch_bounds__(32) k_x_filt_inv_pfa(const __grid_constant__ X
                 mi[ln] = a.slot[f][1] >= 0 ? m[a.slot[f][1]] : 0.0;
             }
             C2<float> *c32 = a.c32[f];
-            float *re32 = a.re32[f], *im32 = a.im32[f];
+            float *re32 = a.re32[f];
             L.each([&](int ln, int n, int i) {
                 const double re = L.b1.re[i], im = L.b1.im[i];
                 if (!(isfinite(re) && isfinite(im))) bad = true;
@@ -724,12 +722,8 @@ __global__ void __launch_bounds__(32) k_x_filt_inv_pfa(const __grid_constant__ X
                 pfa_store_field(a.out[f], g, re, im);
                 const double m0 = ln == 0 ? mr[0] : mr[kPfaLines - 1];
                 const double m1 = ln == 0 ? mi[0] : mi[kPfaLines - 1];
-                if (c32) {
-                    c32[g] = make_float2((float)(re - m0), (float)(im - m1));
-                } else {
-                    if (re32) re32[g] = (float)(re - m0);
-                    if (im32) im32[g] = (float)(im - m1);
-                }
+                if (c32) c32[g] = make_float2((float)(re - m0), (float)(im - m1));
+                if (re32) re32[g] = (float)(re - m0);
             });
         }
         __syncwarp();

@@ -2,10 +2,12 @@
 // HQT_ZN (each hqt_z<N>.cu defines HQT_ZN and includes this file).
 #include <cstring>
 #include <type_traits>
+#include <vector>
 
 #include "hqt_launch.h"
 #include "hqt_zcol.cuh"
 #include "hqt_zfused.cuh"
+#include "hqt_zstage.cuh"
 
 #ifndef HQT_ZN
 #error "define HQT_ZN"
@@ -38,86 +40,99 @@ template <> cudaError_t z_init<HQT_ZN>(int max_smem) {
             e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      max_smem - (int)fa.sharedSizeBytes);
     };
-    opt((const void *)k_zstage<double, double, double, HQT_ZN, 0>);
-    opt((const void *)k_zstage<double, double, double, HQT_ZN, 1>);
-    opt((const void *)k_zstage<double, double, double, HQT_ZN, 2>);
-    opt((const void *)k_zstage<double, double, double, HQT_ZN, 3>);
-    opt((const void *)k_zstage<double, double, double, HQT_ZN, 4>);
-    opt((const void *)k_zstage<double, double, float, HQT_ZN, 1>);
-    opt((const void *)k_zstage<double, double, float, HQT_ZN, 2>);
-    opt((const void *)k_zstage<double, double, float, HQT_ZN, 3>);
-    opt((const void *)k_zstage<double, double, float, HQT_ZN, 4>);
+    opt((const void *)k_zstage<double, HQT_ZN, 0>);
+    opt((const void *)k_zstage<double, HQT_ZN, 1>);
+    opt((const void *)k_zstage<double, HQT_ZN, 2>);
+    opt((const void *)k_zstage<double, HQT_ZN, 3>);
+    opt((const void *)k_zstage<double, HQT_ZN, 4>);
+    opt((const void *)k_zstage<float, HQT_ZN, 1>);
+    opt((const void *)k_zstage<float, HQT_ZN, 2>);
+    opt((const void *)k_zstage<float, HQT_ZN, 3>);
+    opt((const void *)k_zstage<float, HQT_ZN, 4>);
     opt((const void *)k_zcons_tc<HQT_ZN>);
     return e;
 }
 
-// One fused launch per stage (hqt_zfused.cuh): persistent blocks of kZWarps
-// warps, as many as fit on the device at once, each looping over tiles of
-// kZTile columns.
-template <typename TD, int M> static int z_stage_grid(long long plane) {
+// Operand tables of the radial stage: the fragments per lane ([frag][lane]) of
+// Le, Lo (the half-size products of Lz, hqt_zstage.cuh) and Lz1, and z,
+// 1 - z^3, Lz(nz,:) padded to HQT_ZN.  Lz enters through its centro-antisymmetric
+// part (Lz(i,j) - Lz(n'-i,n'-j))/2, from which it differs by rounding (the
+// diagonal is a sum).
+template <>
+void z_tables<HQT_ZN>(const ZHost &h, std::vector<double> &frag, std::vector<double> &tab) {
+    using D = ZsDims<HQT_ZN>;
+    const int nz = h.nz, n1 = nz - 1, hf = (nz + 1) / 2;
+    auto L = [&](int i, int j) {
+        return 0.5 * (h.Lz[(size_t)i * nz + j] - h.Lz[(size_t)(n1 - i) * nz + (n1 - j)]);
+    };
+    frag.clear();
+    auto put = [&](int mt, int kt, auto f) {
+        for (int m = 0; m < mt; ++m)
+            for (int s = 0; s < kt; ++s)
+                for (int lane = 0; lane < 32; ++lane)
+                    frag.push_back(f(8 * m + zs_row(lane >> 2), 4 * s + (lane & 3)));
+    };
+    put(D::MP, D::KE, [&](int i, int j) {
+        if (i >= nz / 2 || j >= hf) return 0.0;
+        return j == n1 - j ? 0.5 * L(i, j) : 0.5 * (L(i, j) + L(i, n1 - j));
+    });
+    put(D::MH, D::KO, [&](int i, int j) {
+        if (i >= hf || j >= nz / 2) return 0.0;
+        return 0.5 * (L(i, j) - L(i, n1 - j));
+    });
+    put(D::M1, D::K1, [&](int i, int j) {
+        return i < n1 && j < n1 ? h.Lz1[(size_t)i * n1 + j] : 0.0;
+    });
+    tab.assign(3 * HQT_ZN, 0.0);
+    for (int i = 0; i < nz; ++i) {
+        tab[i] = h.zz[i];
+        tab[HQT_ZN + i] = 1.0 - h.zz[i] * h.zz[i] * h.zz[i];
+        tab[2 * HQT_ZN + i] = h.Lz[(size_t)n1 * nz + i];
+    }
+}
+
+// One launch per stage (hqt_zstage.cuh): persistent blocks, as many as fit on
+// the device at once, each looping over tiles of kZsCols columns.
+template <typename TD, int M>
+static cudaError_t z_stage_mode(const ZStageArgs<TD> &a, cudaStream_t s) {
+    constexpr int smem = ZsLay<TD, HQT_ZN, M>::bytes;
     static int per_sm = 0, nsm = 0;
     if (per_sm == 0) {
         int dev = 0;
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-            &per_sm, k_zstage<double, double, TD, HQT_ZN, M>, kZThreads,
-            zf_smem_bytes<double, double, TD, HQT_ZN>());
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_zstage<TD, HQT_ZN, M>, kZsThreads,
+                                                      smem);
         if (per_sm < 1) per_sm = 1;
     }
-    const long long tiles = (plane + kZTile - 1) / kZTile;
+    const long long tiles = (a.plane + kZsCols - 1) / kZsCols;
     const long long full = (long long)per_sm * (nsm > 0 ? nsm : 1);
-    return (int)(tiles < full ? tiles : full);
-}
-
-template <typename TD>
-static cudaError_t z_stage_fused_v(int mode, const ZStageArgs<double, double, TD> &a,
-                                   const ZOps<double, HQT_ZN> &op, cudaStream_t s) {
-    constexpr size_t smem = zf_smem_bytes<double, double, TD, HQT_ZN>();
-    switch (mode) {
-#define HQT_ZS(M)                                                                            \
-    case M:                                                                                  \
-        (void)klaunch(k_zstage<double, double, TD, HQT_ZN, M>,                               \
-                      dim3(z_stage_grid<TD, M>(a.plane)), dim3(kZThreads), smem, s, a, op); \
-        break;
-        HQT_ZS(1)
-        HQT_ZS(2)
-        HQT_ZS(3)
-        HQT_ZS(4)
-#undef HQT_ZS
-        default:
-            return cudaErrorInvalidValue;
-    }
+    (void)klaunch(k_zstage<TD, HQT_ZN, M>, dim3((int)(tiles < full ? tiles : full)),
+                  dim3(kZsThreads), smem, s, a);
     return cudaGetLastError();
 }
 
-template <typename TD>
-static cudaError_t z_stage_fused(int mode, const ZStageArgs<double, double, TD> &a,
-                                 const ZHost &h, cudaStream_t s) {
-    const ZOps<double, HQT_ZN> op = make_zops(h);
-    if (mode == 0) {
-        if constexpr (std::is_same<TD, double>::value) {
-            constexpr size_t smem = zf_smem_bytes<double, double, double, HQT_ZN>();
-            (void)klaunch(k_zstage<double, double, double, HQT_ZN, 0>,
-                          dim3(z_stage_grid<double, 0>(a.plane)), dim3(kZThreads), smem, s, a,
-                          op);
-            return cudaGetLastError();
-        }
-        return cudaErrorInvalidValue;
+template <>
+cudaError_t z_stage<HQT_ZN>(int mode, const ZStageArgs<double> &a, cudaStream_t s) {
+    switch (mode) {
+        case 0: return z_stage_mode<double, 0>(a, s);
+        case 1: return z_stage_mode<double, 1>(a, s);
+        case 2: return z_stage_mode<double, 2>(a, s);
+        case 3: return z_stage_mode<double, 3>(a, s);
+        case 4: return z_stage_mode<double, 4>(a, s);
     }
-    return z_stage_fused_v<TD>(mode, a, op, s);
+    return cudaErrorInvalidValue;
 }
 
 template <>
-cudaError_t z_stage<HQT_ZN>(int mode, const ZStageArgs<double, double> &a, const ZHost &h,
-                            int, int, size_t, cudaStream_t s) {
-    return z_stage_fused<double>(mode, a, h, s);
-}
-
-template <>
-cudaError_t z_stage_mixed<HQT_ZN>(int mode, const ZStageArgs<double, double, float> &a,
-                                  const ZHost &h, int, int, size_t, cudaStream_t s) {
-    return z_stage_fused<float>(mode, a, h, s);
+cudaError_t z_stage_mixed<HQT_ZN>(int mode, const ZStageArgs<float> &a, cudaStream_t s) {
+    switch (mode) {
+        case 1: return z_stage_mode<float, 1>(a, s);
+        case 2: return z_stage_mode<float, 2>(a, s);
+        case 3: return z_stage_mode<float, 3>(a, s);
+        case 4: return z_stage_mode<float, 4>(a, s);
+    }
+    return cudaErrorInvalidValue;
 }
 
 template <>

@@ -39,7 +39,7 @@ __global__ void __launch_bounds__(128, 4) k_zcol_misc(ZColArgs<T> a, ZOps<T, NZP
                 T s = T(0);
 #pragma unroll
                 for (int j = 0; j < NZP; ++j) s = fma(op.Lz[i][j], v[j], s);
-                a.dat[(long long)i * P + site] = s;
+                a.atd[(long long)i * P + site] = mk2<T>(v[i], s);
             }
         }
     }

@@ -1,0 +1,40 @@
+// hqt_zdims.h -- sizes and operand tables of the radial stage (hqt_zstage.cuh),
+// shared by host and device.
+#pragma once
+#include "hqt_common.cuh"
+
+namespace hqt {
+
+constexpr int kZsCols = 16;  // columns of a tile
+// Row pitches in shared memory (= widths of the TMA boxes) in bytes: kZsRow of an FP64 pair field,
+// zs_row_td of a pair of type TD, zs_row_r of a real field of type TD.
+constexpr int kZsRow = (kZsCols + 1) * 16;
+template <typename TD> __host__ __device__ constexpr int zs_row_td() {
+    return sizeof(TD) == 8 ? kZsRow : (kZsCols + 2) * 8;
+}
+template <typename TD> __host__ __device__ constexpr int zs_row_r() {
+    return sizeof(TD) == 8 ? (kZsCols + 2) * 8 : (kZsCols + 4) * 4;
+}
+
+// Row g of an mma tile stands for level 8m + zs_row(g) (bits 0 and 1 swapped).
+__host__ __device__ constexpr int zs_row(int g) { return (g & 4) | ((g & 1) << 1) | ((g >> 1) & 1); }
+
+template <int NZP> struct ZsDims {
+    static constexpr int HE = (NZP + 1) / 2, HO = NZP / 2;  // even, odd halves
+    static constexpr int MH = (HE + 7) / 8, MP = (HO + 7) / 8;
+    static constexpr int KE = (HE + 3) / 4, KO = (HO + 3) / 4;
+    static constexpr int M1 = (NZP - 1 + 7) / 8, K1 = (NZP - 1 + 3) / 4;
+    static constexpr int VR = NZP > 4 * K1 ? NZP : 4 * K1;  // rows of a scratch field
+    static constexpr int nfrag = MP * KE + MH * KO + M1 * K1;
+    // state and accumulator are read straight from global memory instead of staged
+#ifndef HQT_ZDIR
+#define HQT_ZDIR (NZP > 25)
+#endif
+#ifndef HQT_ZMB
+#define HQT_ZMB 2
+#endif
+    static constexpr bool direct = HQT_ZDIR;
+    static constexpr int min_blocks = HQT_ZMB;
+};
+
+}  // namespace hqt
