@@ -7,13 +7,22 @@
 // every n1 followed by a P-point DFT along n1 for every k2, with no twiddle
 // factors.
 //   stage A (Q-point): the real-pair fold a_t = x_t + x_{Q-t},
-//     b_t = x_t - x_{Q-t} is formed while loading the operand fragments; two
-//     products with the (M+1) x (M+1) cosine and sine matrices (M = (Q-1)/2)
-//     give P_k, Q_k and X_k = P_k -+ i Q_k, X_{Q-k} = P_k +- i Q_k.  In FP64
-//     the products run as mma.sync m8n8k4 f64; in FP32 (the mixed-precision
-//     step) as mma.sync m16n8k8 tf32 in the 3xTF32 form
-//     A_hi B_hi + A_hi B_lo + A_lo B_hi (hi = the TF32 rounding, lo = the
-//     TF32 rounding of the rest), accumulated in FP32.
+//     b_t = x_t - x_{Q-t} is formed while loading the operand fragments; products
+//     with cosine and sine matrices give P_k, Q_k and X_k = P_k -+ i Q_k,
+//     X_{Q-k} = P_k +- i Q_k.
+//     FP64 (mma.sync m8n8k4 f64), Q = 43: in the order of powers of 3 (Rader:
+//     3 generates the residues of 43) the 21 x 21 cosine matrix depends on the sum
+//     of its indices modulo 21 only, the sine matrix too up to signs.  With
+//     index r + 7p (p = 0..2) the sums over p are cyclic convolutions of three
+//     terms, whose constant part takes one 7 x 7 product with
+//     s_r = x_0 + x_1 + x_2 and whose rest takes one 14 x 14 product with
+//     x_0 - x_2, x_1 - x_2 for the outputs p = 0, 1 (the three rests add to zero,
+//     which gives p = 2).  Padded to the mma that is 10 products of 8 x 8 x 4 per
+//     operand tile instead of 18 for the whole 22 x 22, and 20 fragments in
+//     registers instead of 36.
+//     FP32 (the mixed-precision step): the whole matrices, as mma.sync m16n8k8
+//     tf32 in the 3xTF32 form A_hi B_hi + A_hi B_lo + A_lo B_hi (hi = the TF32
+//     rounding, lo = the TF32 rounding of the rest), accumulated in FP32.
 //   stage B (P-point, P <= 8): on the CUDA cores, a lane per column, in the
 //     real-pair form; as a padded tensor-core product it cost several times
 //     the arithmetic.  A spectral derivative runs forward stage B, its
@@ -51,18 +60,52 @@ template <int P_, int Q_> struct PfaDims {
     static constexpr int NTA = (2 * U + 7) / 8;  // ... times (re, im), 8 per tile
     static constexpr int CB = kPfaLines * Q;     // stage-B columns: (line, k2)
     static constexpr int QIP = pfa_modinv(Q_ % P_, P_), PIQ = pfa_modinv(P_ % Q_, Q_);
-    // FP64 stage A: m8n8k4 tiles over rows k = 0..M and reduction t = 0..M
-    static constexpr int MTA = (M + 1 + 7) / 8, KSA = (M + 1 + 3) / 4;
-    static constexpr int NFRAG = 2 * MTA * KSA;  // cos, sin
+    // FP64 stage A: m8n8k4 tiles of the constant part (1 x 2 reduction steps) and
+    // of the rest (2 x 4), cos and sin
+    static constexpr int NFRAG = 2 * (2 + 8);
     // FP32 stage A: m16n8k8 tiles; per lane 4 registers per tile, hi and lo
     static constexpr int MT32 = (M + 1 + 15) / 16, KS32 = (M + 1 + 7) / 8;
     static constexpr int NFRAG32 = 2 * 2 * MT32 * KS32 * 4;  // cos/sin x hi/lo
-    static_assert(2 * P_ <= 16 && MTA * 8 <= 24, "P <= 8 and Q <= 47");
+    static_assert(2 * P_ <= 16 && Q_ == 43, "P <= 8; Q = 43 (powers of 3, 21 = 3 * 7)");
 };
 
-// Shared-memory planes of one buffer: re/im of [u][t], u = line*P + n1.
-template <typename T> struct PfaBuf {
-    T *re, *im;
+// Storage of the Q entries of a column u in shared memory.  FP32: in order, Q
+// apart.  FP64: entry 3^i mod 43 at position i, entry 0 at 42, columns 44 apart:
+// stage A's operand rows and results (powers r + 7p, and r + 7p + 21 for the
+// negative) are then runs of adjacent elements at fixed offsets, and its accesses
+// nearly free of bank conflicts (per 43-point stage of two lines 264 wavefronts
+// instead of 431, of 192 without any).
+template <typename T, int P, int Q> struct PfaStore {
+    static constexpr bool kPow = std::is_same<T, double>::value;
+    static constexpr int PITCH = kPow ? 44 : Q;
+    static constexpr int SIZE = kPfaLines * P * PITCH;  // complex elements of a buffer
+};
+
+// One buffer in shared memory: values of [u][t], u = line*P + n1.  FP64:
+// interleaved (16-byte copies, reads and writes); FP32: split planes.
+template <typename T> struct PfaBuf;
+template <> struct PfaBuf<double> {
+    double2 *c;
+    __device__ __forceinline__ double *re(int i) const { return &c[i].x; }
+    __device__ __forceinline__ double *im(int i) const { return &c[i].y; }
+    __device__ __forceinline__ double2 get(int i) const { return c[i]; }
+    __device__ __forceinline__ void put(int i, double x, double y) const { c[i] = make_double2(x, y); }
+    // cp.async of a complex value
+    __device__ __forceinline__ void copy(int i, const double2 *src) const { cp_async<16>(c + i, src); }
+};
+template <> struct PfaBuf<float> {
+    float *r, *m;
+    __device__ __forceinline__ float *re(int i) const { return r + i; }
+    __device__ __forceinline__ float *im(int i) const { return m + i; }
+    __device__ __forceinline__ float2 get(int i) const { return make_float2(r[i], m[i]); }
+    __device__ __forceinline__ void put(int i, float x, float y) const {
+        r[i] = x;
+        m[i] = y;
+    }
+    __device__ __forceinline__ void copy(int i, const float2 *src) const {
+        cp_async<4>(r + i, &src->x);
+        cp_async<4>(m + i, &src->y);
+    }
 };
 
 // d += a * b on one 8x8x4 FP64 tensor-core tile
@@ -85,39 +128,48 @@ __device__ __forceinline__ unsigned pfa_tf32(float x) {
     return r;
 }
 
-// Combine P_k, Q_k of row k into X_k and X_{Q-k} (SIGN -1 forward).
-template <int SIGN, int Q, typename T, typename Put>
-__device__ __forceinline__ void pfa_unfold(int u, int k, T pr, T pi, T qr, T qi, Put put) {
-    if (k == 0) {
-        put(u, 0, pr, pi);
-    } else if (SIGN < 0) {
+// Combine P_k, Q_k into X_k (at k) and X_{Q-k} (at kn) (SIGN -1 forward).
+template <int SIGN, typename T, typename Put>
+__device__ __forceinline__ void pfa_unfold(int u, int k, int kn, T pr, T pi, T qr, T qi, Put put) {
+    if (SIGN < 0) {
         put(u, k, pr + qi, pi - qr);
-        put(u, Q - k, pr - qi, pi + qr);
+        put(u, kn, pr - qi, pi + qr);
     } else {
         put(u, k, pr - qi, pi + qr);
-        put(u, Q - k, pr + qi, pi - qr);
+        put(u, kn, pr + qi, pi - qr);
     }
 }
 
 template <typename T, int P, int Q> struct PfaStageA;
 
-// FP64 stage A: fragments a0 = L[8m+g][4s+q]; operand b0 = V[4s+q][col g];
-// result c_i = out[8m+g][col 2q+i].
+// 3^i mod 43: the order of the FP64 stage A
+__host__ __device__ constexpr int pfa_pow3(int i) {
+    int v = 1;
+    for (int k = 0; k < i; ++k) v = v * 3 % 43;
+    return v;
+}
+
+// FP64 stage A.  Lane (g, q): operand rows r = 4s + q (s = 0, 1; r = 7 stands for
+// x_0), result row r' = g (7: X_0) of column u = 4nt + q, parts re and im.
 template <int P, int Q> struct PfaStageA<double, P, Q> {
     using D = PfaDims<P, Q>;
-    static constexpr int M = D::M, MTA = D::MTA, KSA = D::KSA;
-    double Ac[MTA][KSA], As[MTA][KSA];
+    static constexpr int PITCH = PfaStore<double, P, Q>::PITCH;
+    double Cd[2], Cw[2][4], Sd[2], Sw[2][4];  // constant part, rest; cos, sin
 
     __device__ __forceinline__ void init(const double *frag, int lane) {
-        int j = 0;
+        const double *f = frag + lane;
 #pragma unroll
-        for (int m = 0; m < MTA; ++m)
+        for (int s = 0; s < 2; ++s, f += 32) Cd[s] = *f;
 #pragma unroll
-            for (int s = 0; s < KSA; ++s) Ac[m][s] = frag[32 * j++ + lane];
+        for (int m = 0; m < 2; ++m)
 #pragma unroll
-        for (int m = 0; m < MTA; ++m)
+            for (int s = 0; s < 4; ++s, f += 32) Cw[m][s] = *f;
 #pragma unroll
-            for (int s = 0; s < KSA; ++s) As[m][s] = frag[32 * j++ + lane];
+        for (int s = 0; s < 2; ++s, f += 32) Sd[s] = *f;
+#pragma unroll
+        for (int m = 0; m < 2; ++m)
+#pragma unroll
+            for (int s = 0; s < 4; ++s, f += 32) Sw[m][s] = *f;
     }
 
     // Two operand tiles per pass: twice the independent accumulator chains
@@ -126,53 +178,75 @@ template <int P, int Q> struct PfaStageA<double, P, Q> {
     __device__ __forceinline__ void run(PfaBuf<double> in, Put put, int g, int q) const {
 #pragma unroll 1
         for (int n0 = 0; n0 < D::NTA; n0 += 2) {
-            double pa[2][MTA][2], qa[2][MTA][2];
+            double pc[2][3][2], ps[2][3][2];  // u, w_0, w_1 of the cos and sin products
 #pragma unroll
             for (int j = 0; j < 2; ++j)
 #pragma unroll
-                for (int m = 0; m < MTA; ++m)
-                    pa[j][m][0] = pa[j][m][1] = qa[j][m][0] = qa[j][m][1] = 0.0;
-            const double *pl = (g & 1) ? in.im : in.re;
+                for (int m = 0; m < 3; ++m)
+                    pc[j][m][0] = pc[j][m][1] = ps[j][m][0] = ps[j][m][1] = 0.0;
 #pragma unroll
-            for (int s = 0; s < KSA; ++s) {
-                const int t = 4 * s + q;
+            for (int s = 0; s < 2; ++s) {
 #pragma unroll
                 for (int j = 0; j < 2; ++j) {
                     const int uc = 4 * (n0 + j) + (g >> 1);  // operand column (u, part g&1)
-                    double a = 0.0, b = 0.0;
-                    if (uc < D::U && t <= M) {
-                        const double xt = pl[uc * Q + t];
-                        if (t == 0) {
-                            a = xt;
-                        } else {
-                            const double xr = pl[uc * Q + (Q - t)];
-                            a = xt + xr;
-                            b = xt - xr;
-                        }
+                    // rows r = 4s + q (row 7: entries of other rows, times zero)
+                    const double *x = in.re((uc < D::U ? uc : 0) * PITCH + 4 * s + q) + (g & 1);
+                    double a[3], b[3];
+#pragma unroll
+                    for (int p = 0; p < 3; ++p) {
+                        const double xt = x[2 * (7 * p)], xr = x[2 * (7 * p + 21)];
+                        a[p] = xt + xr;
+                        b[p] = xt - xr;
+                    }
+                    // row 7 of the constant part is x_0 itself
+                    const double sa = s == 1 && q == 3 ? x[2 * (42 - 7)] : a[0] + a[1] + a[2];
+                    const double sb = b[0] - b[1] + b[2];
+                    const double a0 = a[0] - a[2], a1 = a[1] - a[2];
+                    const double b0 = b[0] - b[2], b1 = b[1] + b[2];
+                    pfa_mma(pc[j][0][0], pc[j][0][1], Cd[s], sa);
+                    pfa_mma(ps[j][0][0], ps[j][0][1], Sd[s], sb);
+#pragma unroll
+                    for (int m = 0; m < 2; ++m) {
+                        pfa_mma(pc[j][1 + m][0], pc[j][1 + m][1], Cw[m][s], a0);
+                        pfa_mma(ps[j][1 + m][0], ps[j][1 + m][1], Sw[m][s], b0);
                     }
 #pragma unroll
-                    for (int m = 0; m < MTA; ++m) {
-                        pfa_mma(pa[j][m][0], pa[j][m][1], Ac[m][s], a);
-                        pfa_mma(qa[j][m][0], qa[j][m][1], As[m][s], b);
+                    for (int m = 0; m < 2; ++m) {
+                        pfa_mma(pc[j][1 + m][0], pc[j][1 + m][1], Cw[m][2 + s], a1);
+                        pfa_mma(ps[j][1 + m][0], ps[j][1 + m][1], Sw[m][2 + s], b1);
                     }
                 }
             }
-            // lane holds rows k = 8m+g, column u = 4nt+q, parts re (0) and im (1).
             // The tiles write only their own columns, after all their reads:
             // stage A may run in place.
             __syncwarp();
 #pragma unroll
             for (int j = 0; j < 2; ++j) {
                 const int u = 4 * (n0 + j) + q;
-                if (u < D::U) {
-#pragma unroll
-                    for (int m = 0; m < MTA; ++m) {
-                        const int k = 8 * m + g;
-                        if (k > M) continue;
-                        pfa_unfold<SIGN, Q>(u, k, pa[j][m][0], pa[j][m][1], qa[j][m][0],
-                                            qa[j][m][1], put);
-                    }
+                if (u >= D::U) continue;
+                const double(&c)[3][2] = pc[j];
+                const double(&e)[3][2] = ps[j];
+                if (g == 7) {
+                    put(u, 42, c[0][0], c[0][1]);
+                    continue;
                 }
+                double pr[3], pi[3], qr[3], qi[3];
+                pr[0] = c[0][0] + c[1][0];
+                pi[0] = c[0][1] + c[1][1];
+                pr[1] = c[0][0] + c[2][0];
+                pi[1] = c[0][1] + c[2][1];
+                pr[2] = c[0][0] - (c[1][0] + c[2][0]);
+                pi[2] = c[0][1] - (c[1][1] + c[2][1]);
+                qr[0] = e[0][0] + e[1][0];
+                qi[0] = e[0][1] + e[1][1];
+                qr[1] = -(e[0][0] + e[2][0]);
+                qi[1] = -(e[0][1] + e[2][1]);
+                qr[2] = e[0][0] - (e[1][0] + e[2][0]);
+                qi[2] = e[0][1] - (e[1][1] + e[2][1]);
+#pragma unroll
+                for (int p = 0; p < 3; ++p)
+                    pfa_unfold<SIGN>(u, g + 7 * p, g + 7 * p + 21, pr[p], pi[p], qr[p], qi[p],
+                                     put);
             }
         }
     }
@@ -215,7 +289,7 @@ template <int P, int Q> struct PfaStageA<float, P, Q> {
                 for (int m = 0; m < MT; ++m)
 #pragma unroll
                     for (int r = 0; r < 4; ++r) pa[j][m][r] = qa[j][m][r] = 0.0f;
-            const float *pl = (g & 1) ? in.im : in.re;
+            const float *pl = (g & 1) ? in.m : in.r;
 #pragma unroll
             for (int s = 0; s < KS; ++s) {
 #pragma unroll
@@ -267,8 +341,12 @@ template <int P, int Q> struct PfaStageA<float, P, Q> {
                         for (int h = 0; h < 2; ++h) {
                             const int k = 16 * m + g + 8 * h;
                             if (k > M) continue;
-                            pfa_unfold<SIGN, Q>(u, k, pa[j][m][2 * h], pa[j][m][2 * h + 1],
-                                                qa[j][m][2 * h], qa[j][m][2 * h + 1], put);
+                            if (k == 0)
+                                put(u, 0, pa[j][m][2 * h], pa[j][m][2 * h + 1]);
+                            else
+                                pfa_unfold<SIGN>(u, k, Q - k, pa[j][m][2 * h],
+                                                 pa[j][m][2 * h + 1], qa[j][m][2 * h],
+                                                 qa[j][m][2 * h + 1], put);
                         }
                 }
             }
@@ -278,11 +356,14 @@ template <int P, int Q> struct PfaStageA<float, P, Q> {
 
 template <typename T, int P, int Q> struct PfaWarp {
     using D = PfaDims<P, Q>;
+    using S = PfaStore<T, P, Q>;
     static constexpr int N = D::N;
     PfaStageA<T, P, Q> sa;
     int lane, g, q;
+    const unsigned short *k2tab;  // FP64: entry at each position
 
-    __device__ __forceinline__ void init(const T *frag) {
+    __device__ __forceinline__ void init(const T *frag, const unsigned short *k2) {
+        k2tab = k2;
         lane = threadIdx.x & 31;
         g = lane >> 2;
         q = lane & 3;
@@ -290,10 +371,17 @@ template <typename T, int P, int Q> struct PfaWarp {
     }
 
     // Stage A along t for every column u of `in`; SIGN -1 forward, +1 inverse.
-    // The result X(u, k) goes to put(u, k, re, im) for k = 0..Q-1.
+    // The result X(u, k) goes to put(u, e, re, im), e the position of k.
     template <int SIGN, typename Put>
     __device__ __forceinline__ void stage_a(PfaBuf<T> in, Put put) const {
         sa.template run<SIGN>(in, put, g, q);
+    }
+    // entry at position e of a column
+    __device__ __forceinline__ int entry(int e) const {
+        if constexpr (S::kPow)
+            return __ldg(k2tab + e);
+        else
+            return e;
     }
 
     // Stage B on the CUDA cores, a lane per column (line, k2), in the
@@ -307,14 +395,9 @@ template <typename T, int P, int Q> struct PfaWarp {
         constexpr int H = (P - 1) / 2;
 #pragma unroll 1
         for (int col = lane; col < D::CB; col += 32) {
-            const int ln = col / Q, k2 = col - ln * Q;
+            const int ln = col / Q, e2 = col - ln * Q, k2 = entry(e2);
             T zr[P], zi[P], xr[P], xi[P];
-#pragma unroll
-            for (int n1 = 0; n1 < P; ++n1) {
-                const int e = (ln * P + n1) * Q + k2;
-                zr[n1] = in.re[e];
-                zi[n1] = in.im[e];
-            }
+            load(in, ln, e2, zr, zi);
             if (FWD) {
                 dft_real_pair<-1, H>(zr, zi, xr, xi, cs);
             } else {
@@ -335,12 +418,24 @@ template <typename T, int P, int Q> struct PfaWarp {
                     zi[k1] = xi[k1];
                 }
             }
+            store(out, ln, e2, zr, zi);
+        }
+    }
+    __device__ __forceinline__ static void load(PfaBuf<T> b, int ln, int e2, T (&zr)[P], T (&zi)[P]) {
 #pragma unroll
-            for (int n1 = 0; n1 < P; ++n1) {
-                const int e = (ln * P + n1) * Q + k2;
-                out.re[e] = zr[n1];
-                out.im[e] = zi[n1];
-            }
+        for (int n1 = 0; n1 < P; ++n1) {
+            const int e = (ln * P + n1) * S::PITCH + e2;
+            const C2<T> v = b.get(e);
+            zr[n1] = v.x;
+            zi[n1] = v.y;
+        }
+    }
+    __device__ __forceinline__ static void store(PfaBuf<T> b, int ln, int e2, const T (&zr)[P],
+                                                 const T (&zi)[P]) {
+#pragma unroll
+        for (int n1 = 0; n1 < P; ++n1) {
+            const int e = (ln * P + n1) * S::PITCH + e2;
+            b.put(e, zr[n1], zi[n1]);
         }
     }
 
@@ -370,6 +465,32 @@ template <typename T, int P, int Q> struct PfaWarp {
                 im *= m;
             }
         });
+    }
+
+    // first and second derivative of a field after stage A in one pass over its
+    // spectrum: the first into `out`, the second in place
+    __device__ __forceinline__ void stage_b_deriv12(PfaBuf<T> in, PfaBuf<T> out, T s1, T s2,
+                                                    const T (&cs)[2][P]) const {
+        constexpr int H = (P - 1) / 2;
+#pragma unroll 1
+        for (int col = lane; col < D::CB; col += 32) {
+            const int ln = col / Q, e2 = col - ln * Q, k2 = entry(e2);
+            T zr[P], zi[P], xr[P], xi[P], yr[P], yi[P];
+            load(in, ln, e2, zr, zi);
+            dft_real_pair<-1, H>(zr, zi, xr, xi, cs);
+#pragma unroll
+            for (int k1 = 0; k1 < P; ++k1) {
+                const T w = wavenumber(k1, k2), m = s1 * w, m2 = s2 * w * w;
+                yr[k1] = -m * xi[k1];
+                yi[k1] = m * xr[k1];
+                xr[k1] *= m2;
+                xi[k1] *= m2;
+            }
+            dft_real_pair<+1, H>(yr, yi, zr, zi, cs);
+            store(out, ln, e2, zr, zi);
+            dft_real_pair<+1, H>(xr, xi, zr, zi, cs);
+            store(in, ln, e2, zr, zi);
+        }
     }
 
     // P-point DFT of (xr, xi) into (yr, yi), sign SIGN, real-pair form.
@@ -423,16 +544,44 @@ template <int P, int Q> double pfa_matrix(int part, int k, int t) {
     return (t == 0 || k == 0) ? 0.0 : std::sin(two_pi * ((t * k) % Q) / Q);
 }
 
-// Host side: the per-lane FP64 fragment table (NFRAG x 32 doubles).
+// Host side: the per-lane FP64 fragment table (NFRAG x 32 doubles): constant part
+// and rest of the cos, then of the sin matrix, in the order of powers of 3.
 template <int P, int Q> void pfa_fragments(double *tab) {
-    using D = PfaDims<P, Q>;
+    const long double two_pi = 6.283185307179586476925286766559005768L;
+    // c(n) = cos(2 pi 3^n/43), period 21; s(n) = (-1)^n sin(2 pi 3^n/43), period 21
+    auto kern = [&](int part, int n) -> long double {
+        n %= 21;
+        const long double t = two_pi * pfa_pow3(n) / Q;
+        return part == 0 ? std::cos(t) : (n % 2 ? -std::sin(t) : std::sin(t));
+    };
+    auto mean = [&](int part, int m) {
+        return (kern(part, m) + kern(part, m + 7) + kern(part, m + 14)) / 3;
+    };
     int j = 0;
-    for (int part = 0; part < 2; ++part)  // 0: cos, 1: sin
-        for (int m = 0; m < D::MTA; ++m)
-            for (int s = 0; s < D::KSA; ++s, ++j)
-                for (int lane = 0; lane < 32; ++lane)
-                    tab[32 * j + lane] =
-                        pfa_matrix<P, Q>(part, 8 * m + (lane >> 2), 4 * s + (lane & 3));
+    for (int part = 0; part < 2; ++part) {
+        // sin: rows and columns carry (-1)^index, the p = 1 terms another sign
+        auto sg = [&](int i) { return part == 1 && i % 2 ? -1.0L : 1.0L; };
+        for (int s = 0; s < 2; ++s, ++j)
+            for (int lane = 0; lane < 32; ++lane) {
+                const int i = lane >> 2, r = 4 * s + (lane & 3);
+                long double v;
+                if (i < 7 && r < 7)
+                    v = sg(i) * sg(r) * mean(part, i + r);
+                else
+                    v = part == 0 ? 1 : 0;  // x_0 in every P_k, all of it in X_0
+                tab[32 * j + lane] = (double)v;
+            }
+        for (int m = 0; m < 2; ++m)
+            for (int s = 0; s < 4; ++s, ++j)
+                for (int lane = 0; lane < 32; ++lane) {
+                    const int i = lane >> 2, r = 4 * (s & 1) + (lane & 3), d = s >> 1;
+                    long double v = 0;
+                    if (i < 7 && r < 7)
+                        v = sg(i) * sg(r) * (part == 1 && d == 1 ? -1 : 1) *
+                            (kern(part, i + r + 7 * (m + d)) - mean(part, i + r));
+                    tab[32 * j + lane] = (double)v;
+                }
+    }
 }
 
 // TF32 rounding (to nearest, ties away from zero) of a float on the host:

@@ -17,6 +17,23 @@ cudaError_t pfa_init_301() {
     pfa_fragments32<HQT_PFA_P, HQT_PFA_Q>(frag32.data());
     if (e == cudaSuccess)
         e = cudaMemcpyToSymbol(g_pfa_frag32, frag32.data(), sizeof(float) * frag32.size());
+    // positions of the FP64 storage order
+    constexpr int P = HQT_PFA_P, Q = HQT_PFA_Q, N = P * Q;
+    using D = PfaDims<P, Q>;
+    constexpr int PITCH = PfaStore<double, P, Q>::PITCH;
+    unsigned short at[Q], k2[Q], pos[kPfaLines * N], spos[kPfaLines * N];
+    at[0] = Q - 1;
+    for (int i = 0; i < Q - 1; ++i) at[pfa_pow3(i)] = (unsigned short)i;
+    for (int t = 0; t < Q; ++t) k2[at[t]] = (unsigned short)t;
+    for (int n = 0; n < N; ++n)
+        for (int ln = 0; ln < kPfaLines; ++ln) {
+            pos[kPfaLines * n + ln] = (unsigned short)((ln * P + n * D::QIP % P) * PITCH +
+                                                       at[n * D::PIQ % Q]);
+            spos[kPfaLines * n + ln] = (unsigned short)((ln * P + n % P) * PITCH + at[n % Q]);
+        }
+    if (e == cudaSuccess) e = cudaMemcpyToSymbol(g_pfa_pos, pos, sizeof(pos));
+    if (e == cudaSuccess) e = cudaMemcpyToSymbol(g_pfa_spos, spos, sizeof(spos));
+    if (e == cudaSuccess) e = cudaMemcpyToSymbol(g_pfa_k2, k2, sizeof(k2));
     return e;
 }
 
