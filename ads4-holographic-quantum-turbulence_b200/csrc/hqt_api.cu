@@ -262,13 +262,16 @@ LineTab<double> line_tab(const hqt_ctx *c, bool y, bool half) {
     t.g.n_ = p.n;
     t.g.nbl_ = nbl;
     t.g.np_ = p.np;
-    t.g.th_ = lthreads(p.n, nbl);
-    t.g.swz_ = lswz(p.n, nbl, sizeof(double2));
+    for (int i = 0; i < 2; ++i) t.g.th_[i] = lthreads_rt(p, nbl, i + 1);
+    t.g.swz_ = lswz(p.n, nbl, !y);
+    auto magic = [](int d) { return (unsigned)(((1ull << 32) + d - 1) / d); };
+    t.g.mn_ = magic(p.n);
     for (int i = 0; i < p.np; ++i) {
         t.g.R_[i] = p.R[i];
         t.g.s_[i] = p.s[i];
         t.g.tw_[i] = p.tw[i];
-        t.g.mg_[i] = (unsigned)(((1ull << 32) + p.s[i] - 1) / p.s[i]);
+        t.g.mg_[i] = magic(p.s[i]);
+        t.g.mr_[i] = magic(p.n / p.R[i]);
     }
     return t;
 }

@@ -21,10 +21,14 @@
 // Twiddles come from a table packed per pass as [k][j], so that consecutive
 // butterflies read consecutive entries (through L1).
 //
-// Shared-memory layout: element e of line b at (e << nbl) + b, with an XOR of
-// e's low bits where n is a multiple of 8 (the strided rows of the last
-// forward pass otherwise fall on the same banks); threads run over b first, so
-// a warp touches 2^nbl lines by 32 >> nbl consecutive butterflies.
+// Threads and shared memory.  x lines: threads run along a line, element e of line
+// b at b n + e, so a quarter warp's global access is one 128-byte run.  (With
+// threads running over the lines first it touched a 128-byte line per line of
+// the block: 17 of 57 wavefronts of the L1 data pipe, which bounds these passes,
+// at 512x512x25.)  y lines: threads run over the adjacent columns first, element
+// e of line b at (e << nbl) + b.  In both, an XOR of e's low bits where n is a
+// multiple of 8: the strided rows of the last forward pass otherwise fall on the
+// same banks.
 //
 // The plan is a compile-time constant (SGeo) for the lengths of HQT_CN_LIST
 // and a kernel argument (RGeo, divisions by multiply-high) for every other
@@ -334,8 +338,9 @@ template <typename T, int SIGN> struct LDft<T, 10, SIGN> : LDftPrimeFactor<T, 2,
 template <typename T, int SIGN> struct LDft<T, 12, SIGN> : LDftPrimeFactor<T, 4, 3, SIGN> {};
 
 // ---- the transform --------------------------------------------------------
-// NT threads of the block work on the lines; A and B are its two buffers.
-template <typename T, class G> struct LineEng {
+// The threads of a block work on its lines; A and B are its two buffers.  AX: lines
+// along x.
+template <typename T, class G, bool AX> struct LineEng {
     using C = C2<T>;
     // a runtime plan stays in the kernel's parameters (its dynamic indexing
     // would put a copy on the stack)
@@ -348,35 +353,48 @@ template <typename T, class G> struct LineEng {
         : g(t.g), A(sptr<T>(0)), B(sptr<T>(0) + (g.n() << g.nbl())), tw(t.tw), freq(t.freq),
           posn(t.pos) {}
 
-    // bank swizzle of row e (rows stay inside their group of 8)
-    __device__ __forceinline__ int row(int e) const {
-        const int m = g.template swz<T>();
-        if (G::kStatic && m == 0) return e << g.nbl();
-        return (e ^ (((e >> 3) ^ (e >> 6) ^ (e >> 9)) & m)) << g.nbl();
+    __device__ __forceinline__ int threads() const {
+        if constexpr (G::kStatic)
+            return G::threads();
+        else
+            return blockDim.x;
+    }
+    // element e of line b, its low bits swizzled inside the group of 8
+    __device__ __forceinline__ int at(int b, int e) const {
+        const int m = g.template swz<T, AX>();
+        if (!G::kStatic || m != 0) e ^= ((e >> 3) ^ (e >> 6) ^ (e >> 9)) & m;
+        return AX ? b * g.n() + e : (e << g.nbl()) + b;
     }
     __device__ __forceinline__ static int div(unsigned x, int s, unsigned mg) {
         if constexpr (G::kStatic) return (int)x / s;
         return s == 1 ? (int)x : (int)__umulhi(x, mg);
     }
-    // f(b, jj) for every butterfly jj < n/R of every line b
-    template <int R, typename F> __device__ __forceinline__ void each(F f) const {
-        const int cnt = (g.n() / R) << g.nbl();
+    // f(b, jj) for every butterfly jj < n/R of every line b (mr: the magic of n/R)
+    template <int R, typename F> __device__ __forceinline__ void each(unsigned mr, F f) const {
+        const int nr = g.n() / R, cnt = nr << g.nbl();
 #pragma unroll 1
-        for (int t = threadIdx.x; t < cnt; t += g.threads())
-            f(t & ((1 << g.nbl()) - 1), t >> g.nbl());
+        for (int t = threadIdx.x; t < cnt; t += threads()) {
+            if constexpr (AX) {
+                const int b = div(t, nr, mr);
+                f(b, t - b * nr);
+            } else {
+                f(t & ((1 << g.nbl()) - 1), t >> g.nbl());
+            }
+        }
     }
-    // f(integral_constant<int, R>, stride, magic, twiddle offset) of pass p
+    // f(integral_constant<int, R>, stride s, magics of s and n/R, twiddle offset) of
+    // pass p
     template <int P, typename F> __device__ __forceinline__ void at_static(F f) const {
         constexpr LPlan pl = lplan(G::N);
         constexpr int R = pl.R[P], s = pl.s[P], o = pl.tw[P];
-        f(std::integral_constant<int, R>{}, s, 0u, o);
+        f(std::integral_constant<int, R>{}, s, 0u, 0u, o);
     }
     template <typename F> __device__ __forceinline__ void at(int p, F f) const {
         const int s = g.s(p), o = g.tw(p);
-        const unsigned mg = g.mg(p);
+        const unsigned mg = g.mg(p), mr = g.mr(p);
         switch (g.R(p)) {
 #define HQT_LR(RR) \
-    case RR: f(std::integral_constant<int, RR>{}, s, mg, o); break;
+    case RR: f(std::integral_constant<int, RR>{}, s, mg, mr, o); break;
             HQT_LR(2) HQT_LR(3) HQT_LR(4) HQT_LR(5) HQT_LR(6) HQT_LR(7) HQT_LR(8) HQT_LR(9)
             HQT_LR(10) HQT_LR(11) HQT_LR(12) HQT_LR(13)
 #undef HQT_LR
@@ -413,60 +431,178 @@ template <typename T, class G> struct LineEng {
         }
     }
 
-    // butterfly of one pass in place: forward (with twiddles) or inverse
+    // f(x, b, jj) for every butterfly of A (x = 0) and, if `two`, of B (x = 1).  For
+    // runtime plans: their counts leave a part of the block's threads idle, and their
+    // larger radices spill with twiddles held for both buffers (y_rhs 1.54 -> 1.75 ms
+    // at 1001x1001x20).  A compile-time plan takes A and B in one iteration with the
+    // twiddles in registers.
+    template <int R, typename F>
+    __device__ __forceinline__ void each_of(bool two, unsigned mr, F f) const {
+        const int nr = g.n() / R, cnt = nr << g.nbl();
+#pragma unroll 1
+        for (int t = threadIdx.x; t < (two ? 2 * cnt : cnt); t += threads()) {
+            const bool x = t >= cnt;
+            const int u = x ? t - cnt : t;
+            if constexpr (AX) {
+                const int b = div(u, nr, mr);
+                f(x, b, u - b * nr);
+            } else {
+                f(x, u & ((1 << g.nbl()) - 1), u >> g.nbl());
+            }
+        }
+    }
+    // twiddles of a butterfly: held in registers, or (runtime plan) loaded at use
+    template <int R> struct Twiddles {
+        const C *p;
+        int s;
+        C w[G::kStatic ? R : 1];
+        __device__ __forceinline__ Twiddles(const C *p_, int s_) : p(p_), s(s_) {
+            if constexpr (G::kStatic) {
+#pragma unroll
+                for (int r = 1; r < R; ++r) w[r] = __ldg(p + (r - 1) * s);
+            }
+        }
+        __device__ __forceinline__ C operator()(int r) const {
+            if constexpr (G::kStatic)
+                return w[r];
+            else
+                return __ldg(p + (r - 1) * s);
+        }
+    };
+    // one butterfly in place at rows e0 + r s
     template <int R, int SIGN>
-    __device__ __forceinline__ void step(C *X, int s, unsigned mg, int o) const {
-        each<R>([&](int b, int jj) {
-            const int blk = div(jj, s, mg), j = jj - blk * s, e0 = blk * s * R + j;
-            C v[R];
+    __device__ __forceinline__ void fly(C *X, int b, int e0, int s, const Twiddles<R> &w) const {
+        C v[R];
 #pragma unroll
-            for (int r = 0; r < R; ++r) v[r] = X[row(e0 + r * s) + b];
-            if (SIGN > 0) {
+        for (int r = 0; r < R; ++r) v[r] = X[at(b, e0 + r * s)];
+        if (SIGN > 0) {
 #pragma unroll
-                for (int r = 1; r < R; ++r)
-                    v[r] = lf_cmulc<T>(v[r], __ldg(tw + o + (r - 1) * s + j));
-            }
-            ldft<T, R, SIGN>(v);
-            if (SIGN < 0) {
+            for (int r = 1; r < R; ++r) v[r] = lf_cmulc<T>(v[r], w(r));
+        }
+        ldft<T, R, SIGN>(v);
+        if (SIGN < 0) {
 #pragma unroll
-                for (int r = 1; r < R; ++r)
-                    v[r] = lf_cmul<T>(v[r], __ldg(tw + o + (r - 1) * s + j));
-            }
+            for (int r = 1; r < R; ++r) v[r] = lf_cmul<T>(v[r], w(r));
+        }
 #pragma unroll
-            for (int r = 0; r < R; ++r) X[row(e0 + r * s) + b] = v[r];
-        });
+        for (int r = 0; r < R; ++r) X[at(b, e0 + r * s)] = v[r];
+    }
+    // butterflies of one pass in place, of A or (two) of A and B: forward or inverse
+    template <int R, int SIGN>
+    __device__ __forceinline__ void step(bool two, int s, unsigned mg, unsigned mr, int o) const {
+        if constexpr (G::kStatic) {
+            each<R>(mr, [&](int b, int jj) {
+                const int blk = div(jj, s, mg), j = jj - blk * s;
+                const Twiddles<R> w(tw + o + j, s);
+#pragma unroll 1
+                for (int x = 0; x < (two ? 2 : 1); ++x)
+                    fly<R, SIGN>(x ? B : A, b, blk * s * R + j, s, w);
+            });
+        } else {
+            each_of<R>(two, mr, [&](bool x, int b, int jj) {
+                const int blk = div(jj, s, mg), j = jj - blk * s;
+                fly<R, SIGN>(x ? B : A, b, blk * s * R + j, s, Twiddles<R>(tw + o + j, s));
+            });
+        }
+    }
+    // last inverse pass of one butterfly: row j of the plan's first stride s
+    template <int R>
+    __device__ __forceinline__ void fly_last(const C *X, int b, int j, int s, C (&v)[R],
+                                             const Twiddles<R> &w) const {
+#pragma unroll
+        for (int r = 0; r < R; ++r) v[r] = X[at(b, j + r * s)];
+#pragma unroll
+        for (int r = 1; r < R; ++r) v[r] = lf_cmulc<T>(v[r], w(r));
+        ldft<T, R, 1>(v);
+    }
+    template <int R, typename Get, typename Sa>
+    __device__ __forceinline__ void last_a(int b, int j, int s, const Twiddles<R> &w, Get get,
+                                           Sa sa) const {
+        constexpr int H = R > 8 ? 4 : R;
+        C v[R];
+        fly_last<R>(A, b, j, s, v, w);
+#pragma unroll
+        for (int r0 = 0; r0 < R; r0 += H) {
+            decltype(get(0, 0)) x[H];
+#pragma unroll
+            for (int r = 0; r < H; ++r)
+                if (r0 + r < R) x[r] = get(b, j + (r0 + r) * s);
+#pragma unroll
+            for (int r = 0; r < H; ++r)
+                if (r0 + r < R) sa(b, j + (r0 + r) * s, v[r0 + r], x[r]);
+        }
+    }
+    template <int R, typename Sb>
+    __device__ __forceinline__ void last_b(int b, int j, int s, const Twiddles<R> &w, Sb sb) const {
+        C v[R];
+        fly_last<R>(B, b, j, s, v, w);
+#pragma unroll
+        for (int r = 0; r < R; ++r) sb(b, j + r * s, v[r]);
     }
 
-    // first forward pass from ld(b, e) into X; then the middle passes
+    // first forward pass from ld(b, e) into X
     template <typename Ld> __device__ __forceinline__ void first(C *X, Ld ld) const {
-        at_first([&](auto rc, int s, unsigned, int o) {
+        first(X, false, [](int) { return mk2<T>(T(1), T(0)); }, ld);
+    }
+    // ... for a derivative: where the plan has an odd radix, of the line less its
+    // first element.  A constant drops out anyway, but an odd radix rounds it into
+    // every mode: div A of a nearly uniform flow at 180x180x12 was 4 times less exact
+    // than with radices 2, 3 and 5 one by one.  (Powers of two: differences of equal
+    // values are exact.)
+    static constexpr bool kLevel = !G::kStatic || (G::kN & (G::kN - 1)) != 0;
+    template <typename Ld> __device__ __forceinline__ void first_d(C *X, Ld ld) const {
+        at_first([&](auto rc, int s, unsigned, unsigned mr, int o) {
             constexpr int R = decltype(rc)::value;
-            each<R>([&](int b, int j) {
+            each<R>(mr, [&](int b, int j) {
                 C v[R];
 #pragma unroll
                 for (int r = 0; r < R; ++r) v[r] = ld(b, j + r * s);
-                ldft<T, R, -1>(v);
+                if (kLevel) {
+                    const C x0 = ld(b, 0);
 #pragma unroll
-                for (int r = 1; r < R; ++r)
-                    v[r] = lf_cmul<T>(v[r], __ldg(tw + o + (r - 1) * s + j));
-#pragma unroll
-                for (int r = 0; r < R; ++r) X[row(j + r * s) + b] = v[r];
+                    for (int r = 0; r < R; ++r) v[r] = v[r] - x0;
+                }
+                first_fly<R>(X, b, j, s, o, v);
             });
         });
     }
-    // middle passes of nx buffers (A, then B); starts and ends at a barrier
-    __device__ __forceinline__ void forward_mid(int nx) const {
-        __syncthreads();
-        at_mid<1>([&](auto rc, int s, unsigned mg, int o) {
-#pragma unroll 1
-            for (int x = 0; x < nx; ++x) step<decltype(rc)::value, -1>(x ? B : A, s, mg, o);
+    template <int R>
+    __device__ __forceinline__ void first_fly(C *X, int b, int j, int s, int o, C (&v)[R]) const {
+        ldft<T, R, -1>(v);
+#pragma unroll
+        for (int r = 1; r < R; ++r) v[r] = lf_cmul<T>(v[r], __ldg(tw + o + (r - 1) * s + j));
+#pragma unroll
+        for (int r = 0; r < R; ++r) X[at(b, j + r * s)] = v[r];
+    }
+    // ... times ph(b) if `turn`
+    template <typename Ph, typename Ld>
+    __device__ __forceinline__ void first(C *X, bool turn, Ph ph, Ld ld) const {
+        at_first([&](auto rc, int s, unsigned, unsigned mr, int o) {
+            constexpr int R = decltype(rc)::value;
+            each<R>(mr, [&](int b, int j) {
+                C v[R];
+#pragma unroll
+                for (int r = 0; r < R; ++r) v[r] = ld(b, j + r * s);
+                if (turn) {
+                    const C p = ph(b);
+#pragma unroll
+                    for (int r = 0; r < R; ++r) v[r] = lf_cmul<T>(v[r], p);
+                }
+                first_fly<R>(X, b, j, s, o, v);
+            });
         });
     }
-    __device__ __forceinline__ void inverse_mid(int nx) const {
+    // middle passes of A, or of A and B; starts and ends at a barrier
+    __device__ __forceinline__ void forward_mid(bool two) const {
         __syncthreads();
-        at_mid<-1>([&](auto rc, int s, unsigned mg, int o) {
-#pragma unroll 1
-            for (int x = 0; x < nx; ++x) step<decltype(rc)::value, 1>(x ? B : A, s, mg, o);
+        at_mid<1>([&](auto rc, int s, unsigned mg, unsigned mr, int o) {
+            step<decltype(rc)::value, -1>(two, s, mg, mr, o);
+        });
+    }
+    __device__ __forceinline__ void inverse_mid(bool two) const {
+        __syncthreads();
+        at_mid<-1>([&](auto rc, int s, unsigned mg, unsigned mr, int o) {
+            step<decltype(rc)::value, 1>(two, s, mg, mr, o);
         });
     }
     template <int P> __device__ __forceinline__ static int mode0_static(int rem, int mult) {
@@ -510,16 +646,16 @@ template <typename T, class G> struct LineEng {
     template <int R> __device__ __forceinline__ void put(C *X, int b, int blk, C (&v)[R]) const {
         ldft<T, R, 1>(v);
 #pragma unroll
-        for (int r = 0; r < R; ++r) X[row(blk * R + r) + b] = v[r];
+        for (int r = 0; r < R; ++r) X[at(b, blk * R + r)] = v[r];
     }
     template <typename F> __device__ __forceinline__ void middle(const C *X, F f) const {
-        at_last([&](auto rc, int, unsigned, int) {
+        at_last([&](auto rc, int, unsigned, unsigned mr, int) {
             constexpr int R = decltype(rc)::value;
             const int st = g.n() / R;
-            each<R>([&](int b, int blk) {
+            each<R>(mr, [&](int b, int blk) {
                 C v[R];
 #pragma unroll
-                for (int r = 0; r < R; ++r) v[r] = X[row(blk * R + r) + b];
+                for (int r = 0; r < R; ++r) v[r] = X[at(b, blk * R + r)];
                 ldft<T, R, -1>(v);
                 f(v, b, blk, mode0(blk), st);
             });
@@ -530,12 +666,20 @@ template <typename T, class G> struct LineEng {
         middle(A, [&](auto &v, int b, int blk, int k0, int st) {
             constexpr int R = sizeof(v) / sizeof(C);
             C u[R];
+            if (R > 8) {  // two of them spill: the spectrum waits in B
+#pragma unroll
+                for (int i = 0; i < R; ++i) B[at(b, blk * R + i)] = v[i];
+            }
 #pragma unroll
             for (int i = 0; i < R; ++i) {
                 const T m = s1 * wave(k0 + i * st);
                 u[i] = mk2<T>(-m * v[i].y, m * v[i].x);
             }
             put<R>(A, b, blk, u);
+            if (R > 8) {
+#pragma unroll
+                for (int i = 0; i < R; ++i) v[i] = B[at(b, blk * R + i)];
+            }
 #pragma unroll
             for (int i = 0; i < R; ++i) {
                 const T k = wave(k0 + i * st), m = s2 * k * k;
@@ -567,67 +711,71 @@ template <typename T, class G> struct LineEng {
             put<R>(X, b, blk, v);
         });
     }
-    // last inverse pass of X: st(b, e, v) for every element
-    template <typename St> __device__ __forceinline__ void last(const C *X, St st) const {
-        last(X, [](int, int) { return 0; }, [&](int b, int e, C v, int) { st(b, e, v); });
+    // last inverse pass of A: st(b, e, v) for every element
+    template <typename St> __device__ __forceinline__ void last(St st) const {
+        last2(false, [](int, int) { return 0; }, [&](int b, int e, C v, int) { st(b, e, v); },
+              [](int, int, C) {});
     }
-    // ... with x = get(b, e) read for up to 8 elements ahead of their stores (a
-    // read after a store could not move ahead of it)
-    template <typename Get, typename St>
-    __device__ __forceinline__ void last(const C *X, Get get, St st) const {
-        at_first([&](auto rc, int s, unsigned, int o) {
-            constexpr int R = decltype(rc)::value, H = R > 8 ? 4 : R;
-            each<R>([&](int b, int j) {
-                C v[R];
-#pragma unroll
-                for (int r = 0; r < R; ++r) v[r] = X[row(j + r * s) + b];
-#pragma unroll
-                for (int r = 1; r < R; ++r)
-                    v[r] = lf_cmulc<T>(v[r], __ldg(tw + o + (r - 1) * s + j));
-                ldft<T, R, 1>(v);
-#pragma unroll
-                for (int r0 = 0; r0 < R; r0 += H) {
-                    decltype(get(0, 0)) x[H];
-#pragma unroll
-                    for (int r = 0; r < H; ++r)
-                        if (r0 + r < R) x[r] = get(b, j + (r0 + r) * s);
-#pragma unroll
-                    for (int r = 0; r < H; ++r)
-                        if (r0 + r < R) st(b, j + (r0 + r) * s, v[r0 + r], x[r]);
-                }
-            });
+    // ... of A and B with the twiddles loaded once: sa(b, e, v, x) with
+    // x = get(b, e), sb(b, e, v).  x is read for up to 8 elements ahead of their
+    // stores (a read after a store could not move ahead of it).
+    template <typename Get, typename Sa, typename Sb>
+    __device__ __forceinline__ void last2(bool two, Get get, Sa sa, Sb sb) const {
+        at_first([&](auto rc, int s, unsigned, unsigned mr, int o) {
+            constexpr int R = decltype(rc)::value;
+            if constexpr (G::kStatic) {
+                each<R>(mr, [&](int b, int j) {
+                    const Twiddles<R> w(tw + o + j, s);
+                    last_a<R>(b, j, s, w, get, sa);
+                    if (two) last_b<R>(b, j, s, w, sb);
+                });
+            } else {
+                each_of<R>(two, mr, [&](bool x, int b, int j) {
+                    const Twiddles<R> w(tw + o + j, s);
+                    if (x)
+                        last_b<R>(b, j, s, w, sb);
+                    else
+                        last_a<R>(b, j, s, w, get, sa);
+                });
+            }
         });
     }
-    // f(b, k) over all modes of all lines, b fastest
+    // f(b, k) over all modes of all lines
     template <typename F> __device__ __forceinline__ void modes(F f) const {
-        const int cnt = g.n() << g.nbl();
+        const int n = g.n(), cnt = n << g.nbl();
 #pragma unroll 4
-        for (int t = threadIdx.x; t < cnt; t += g.threads())
-            f(t & ((1 << g.nbl()) - 1), t >> g.nbl());
+        for (int t = threadIdx.x; t < cnt; t += threads()) {
+            if constexpr (AX) {
+                const int b = div(t, n, g.mn());
+                f(b, t - b * n);
+            } else {
+                f(t & ((1 << g.nbl()) - 1), t >> g.nbl());
+            }
+        }
     }
     // forward, spectrum left in A by rows pos(k); starts after first(A, ..)
     __device__ __forceinline__ void forward_rest() const {
-        forward_mid(1);
+        forward_mid(false);
         middle(A, [&](auto &v, int b, int blk, int, int) {
             constexpr int R = sizeof(v) / sizeof(C);
 #pragma unroll
-            for (int r = 0; r < R; ++r) A[row(blk * R + r) + b] = v[r];
+            for (int r = 0; r < R; ++r) A[at(b, blk * R + r)] = v[r];
         });
         __syncthreads();
     }
     // inverse of a spectrum in A up to (not including) last(A, ..)
     __device__ __forceinline__ void inverse_begin() const {
         __syncthreads();
-        at_last([&](auto rc, int, unsigned, int) {
+        at_last([&](auto rc, int, unsigned, unsigned mr, int) {
             constexpr int R = decltype(rc)::value;
-            each<R>([&](int b, int blk) {
+            each<R>(mr, [&](int b, int blk) {
                 C v[R];
 #pragma unroll
-                for (int r = 0; r < R; ++r) v[r] = A[row(blk * R + r) + b];
+                for (int r = 0; r < R; ++r) v[r] = A[at(b, blk * R + r)];
                 put<R>(A, b, blk, v);
             });
         });
-        inverse_mid(1);
+        inverse_mid(false);
     }
 };
 

@@ -39,7 +39,7 @@ template <typename T, class GX, class GY> struct LineLaunch {
         const G g(a.lt.g);
         const int per = (1 << g.nbl()) * real;
         const size_t smem = sizeof(C2<T>) * nbuf * ((size_t)g.n() << g.nbl());
-        (void)klaunch(k, dim3((lines + per - 1) / per, ny, nz), dim3(g.threads()), smem, s, a);
+        (void)klaunch(k, dim3((lines + per - 1) / per, ny, nz), dim3(g.block(nbuf)), smem, s, a);
         return cudaGetLastError();
     }
     static cudaError_t launch_x(int kind, const void *args, cudaStream_t s) {

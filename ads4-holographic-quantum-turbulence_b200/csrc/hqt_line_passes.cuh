@@ -8,6 +8,11 @@
 // element and transform) and shared memory.  Two buffers of a block's lines
 // take at most about 66 KB, so three blocks share an SM and one block's loads
 // and stores run behind another's butterflies.
+// Measured, us a launch, with threads over the lines first and the twiddles loaded
+// for each buffer -> as it is: 512x512x25 x_rhs 196 -> 160 (3.6 TB/s), y_rhs 250 ->
+// 244 (3.0 TB/s), filter x forward 154 -> 125, x inverse 183 -> 164; 256x256x25 x_rhs
+// 50 -> 38; with a runtime plan 1001x1001x20 x_rhs 853 -> 864, y_rhs 1540 -> 1517,
+// filter x forward / y / x inverse 636 / 797 / 981 -> 491 / 588 / 659.
 #pragma once
 #include "hqt_line.cuh"
 #include "hqt_passes.cuh"
@@ -26,7 +31,7 @@ template <typename T> __device__ __forceinline__ C2<T> lzero() { return mk2<T>(T
 
 template <typename T, class G>
 __global__ void HQT_L_BOUNDS(G) k_lx_rhs(const __grid_constant__ XRhsArgs<T> a) {
-    const LineEng<T, G> w(a.lt);
+    const LineEng<T, G, true> w(a.lt);
     const int n = w.g.n(), L0 = blockIdx.x << w.g.nbl(), valid = a.nlines - L0;
     const long long g0 = (long long)L0 * n;
     pdl_wait();
@@ -34,25 +39,27 @@ __global__ void HQT_L_BOUNDS(G) k_lx_rhs(const __grid_constant__ XRhsArgs<T> a) 
     // Psi, then C = A_x + i A_y: first and second derivative
 #pragma unroll 1
     for (int f = 0; f < 2; ++f) {
-        w.first(w.A, [&](int b, int e) {
+        w.first_d(w.A, [&](int b, int e) {
             if (b >= valid) return lzero<T>();
             const long long g = at(b, e);
             return f == 0 ? a.psi[g] : a.A[g];
         });
-        w.forward_mid(1);
+        w.forward_mid(false);
         w.middle_deriv12(a.s1, a.s2);
-        w.inverse_mid(2);
+        w.inverse_mid(true);
         C2<T> *d1 = f == 0 ? a.dxpsi : a.E;
-        w.last(w.A, [&](int b, int e, C2<T> v) {
-            if (b < valid) d1[at(b, e)] = v;
-        });
-        w.last(w.B, [&](int b, int e, C2<T> v) {
-            if (b >= valid) return;
-            if (f == 0)
-                a.dxxpsi[at(b, e)] = v;
-            else
-                a.dxxay[at(b, e)] = v.y;
-        });
+        w.last2(
+            true, [](int, int) { return 0; },
+            [&](int b, int e, C2<T> v, int) {
+                if (b < valid) d1[at(b, e)] = v;
+            },
+            [&](int b, int e, C2<T> v) {
+                if (b >= valid) return;
+                if (f == 0)
+                    a.dxxpsi[at(b, e)] = v;
+                else
+                    a.dxxay[at(b, e)] = v.y;
+            });
     }
 }
 
@@ -63,7 +70,7 @@ __global__ void HQT_L_BOUNDS(G) k_lx_rhs(const __grid_constant__ XRhsArgs<T> a) 
 //      = Re(IFFT((s1 k - s2 k^2) W2^)), one real multiplier.
 template <typename T, class G>
 __global__ void HQT_L_BOUNDS(G) k_ly_rhs(const __grid_constant__ YRhsArgs<T> a) {
-    const LineEng<T, G> w(a.lt);
+    const LineEng<T, G, false> w(a.lt);
     const int x0 = blockIdx.x << w.g.nbl(), valid = a.nx - x0;
     const long long zoff = (long long)blockIdx.y * a.ny * a.nx + x0;
     pdl_wait();
@@ -71,37 +78,39 @@ __global__ void HQT_L_BOUNDS(G) k_ly_rhs(const __grid_constant__ YRhsArgs<T> a) 
 #pragma unroll 1
     for (int f = 0; f < 2; ++f) {
         if (f == 0) {
-            w.first(w.A, [&](int b, int e) { return b < valid ? a.psi[at(b, e)] : lzero<T>(); });
+            w.first_d(w.A, [&](int b, int e) { return b < valid ? a.psi[at(b, e)] : lzero<T>(); });
         } else {
-            w.first(w.A, [&](int b, int e) {
+            w.first_d(w.A, [&](int b, int e) {
                 if (b >= valid) return lzero<T>();
                 const long long g = at(b, e);
                 return mk2<T>(a.E[g].x, a.A[g].y);
             });
-            w.first(w.B, [&](int b, int e) {
+            w.first_d(w.B, [&](int b, int e) {
                 if (b >= valid) return lzero<T>();
                 const long long g = at(b, e);
                 return mk2<T>(a.A[g].x, a.E[g].y);
             });
         }
-        w.forward_mid(1 + f);
+        w.forward_mid(f == 1);
         if (f == 0) {
             w.middle_deriv12(a.s1, a.s2);
         } else {
             w.middle_deriv1(w.A, a.s1);
             w.middle_deriv_mix(w.B, a.s1, a.s2);
         }
-        w.inverse_mid(2);
+        w.inverse_mid(true);
         if (f == 0) {
-            w.last(w.A, [&](int b, int e, C2<T> v) {
-                if (b < valid) a.dypsi[at(b, e)] = v;
-            });
-            w.last(w.B, [&](int b, int e, C2<T> v) {
-                if (b < valid) a.dyypsi[at(b, e)] = v;
-            });
+            w.last2(
+                true, [](int, int) { return 0; },
+                [&](int b, int e, C2<T> v, int) {
+                    if (b < valid) a.dypsi[at(b, e)] = v;
+                },
+                [&](int b, int e, C2<T> v) {
+                    if (b < valid) a.dyypsi[at(b, e)] = v;
+                });
         } else {
-            w.last(
-                w.A,
+            w.last2(
+                true,
                 [&](int b, int e) {
                     if (b >= valid) return lzero<T>();
                     const long long g = at(b, e);
@@ -112,71 +121,72 @@ __global__ void HQT_L_BOUNDS(G) k_ly_rhs(const __grid_constant__ YRhsArgs<T> a) 
                     const long long g = at(b, e);
                     a.divA[g] = x.x + v.y;
                     a.B[g].y = x.y - v.x;
+                },
+                [&](int b, int e, C2<T> v) {
+                    if (b < valid) a.B[at(b, e)].x = v.x;
                 });
-            w.last(w.B, [&](int b, int e, C2<T> v) {
-                if (b < valid) a.B[at(b, e)].x = v.x;
-            });
         }
     }
 }
 
 template <typename T, class G>
 __global__ void HQT_L_BOUNDS1(G) k_lx_d1(const __grid_constant__ XD1Args<T> a) {
-    const LineEng<T, G> w(a.lt);
+    const LineEng<T, G, true> w(a.lt);
     const int n = w.g.n(), L0 = blockIdx.x << w.g.nbl(), valid = a.nlines - L0;
     const long long g0 = (long long)L0 * n;
     pdl_wait();
     auto at = [&](int b, int e) { return g0 + (long long)b * n + e; };
-    w.first(w.A, [&](int b, int e) {
+    w.first_d(w.A, [&](int b, int e) {
         return b < valid ? load_field(a.in, at(b, e)) : lzero<T>();
     });
-    w.forward_mid(1);
+    w.forward_mid(false);
     w.middle_deriv1(w.A, a.s1);
-    w.inverse_mid(1);
-    w.last(w.A, [&](int b, int e, C2<T> v) {
+    w.inverse_mid(false);
+    w.last([&](int b, int e, C2<T> v) {
         if (b < valid) store_field(a.out, at(b, e), v);
     });
 }
 
 template <typename T, class G>
 __global__ void HQT_L_BOUNDS1(G) k_ly_d1(const __grid_constant__ YD1Args<T> a) {
-    const LineEng<T, G> w(a.lt);
+    const LineEng<T, G, false> w(a.lt);
     const int x0 = blockIdx.x << w.g.nbl(), valid = a.nx - x0;
     const long long zoff = (long long)blockIdx.y * a.ny * a.nx + x0;
     pdl_wait();
     auto at = [&](int b, int e) { return zoff + (long long)e * a.nx + b; };
-    w.first(w.A, [&](int b, int e) {
+    w.first_d(w.A, [&](int b, int e) {
         return b < valid ? load_field(a.in, at(b, e)) : lzero<T>();
     });
-    w.forward_mid(1);
+    w.forward_mid(false);
     w.middle_deriv1(w.A, a.s1);
-    w.inverse_mid(1);
-    w.last(
-        w.A, [&](int b, int e) { return a.add_re && b < valid ? a.add_re[at(b, e)] : T(0); },
+    w.inverse_mid(false);
+    w.last2(
+        false, [&](int b, int e) { return a.add_re && b < valid ? a.add_re[at(b, e)] : T(0); },
         [&](int b, int e, C2<T> v, T x) {
             v.x += x;
             if (b < valid) store_field(a.out, at(b, e), v);
-        });
+        },
+        [](int, int, C2<T>) {});
 }
 
 // First derivative of a real field into a real field, two real lines per
 // complex line (real_field_d1): complex line b carries real lines 2b and 2b+1.
 template <typename T, class G>
 __global__ void HQT_L_BOUNDS1(G) k_lx_d1r(const __grid_constant__ XD1Args<T> a) {
-    const LineEng<T, G> w(a.lt);
+    const LineEng<T, G, true> w(a.lt);
     const int n = w.g.n(), L0 = blockIdx.x << (w.g.nbl() + 1), nr = a.nlines - L0;
     const int si = a.in.st, so = a.out.st;
     const T *src = a.in.re + (long long)L0 * n * si;
     T *dst = a.out.re + (long long)L0 * n * so;
     pdl_wait();
-    w.first(w.A, [&](int b, int e) {
+    w.first_d(w.A, [&](int b, int e) {
         const long long g = 2ll * b * n + e;
         return mk2<T>(2 * b < nr ? src[g * si] : T(0), 2 * b + 1 < nr ? src[(g + n) * si] : T(0));
     });
-    w.forward_mid(1);
+    w.forward_mid(false);
     w.middle_deriv1(w.A, a.s1);
-    w.inverse_mid(1);
-    w.last(w.A, [&](int b, int e, C2<T> v) {
+    w.inverse_mid(false);
+    w.last([&](int b, int e, C2<T> v) {
         const long long g = 2ll * b * n + e;
         if (2 * b < nr) dst[g * so] = v.x;
         if (2 * b + 1 < nr) dst[(g + n) * so] = v.y;
@@ -185,7 +195,7 @@ __global__ void HQT_L_BOUNDS1(G) k_lx_d1r(const __grid_constant__ XD1Args<T> a) 
 
 template <typename T, class G>
 __global__ void HQT_L_BOUNDS1(G) k_ly_d1r(const __grid_constant__ YD1Args<T> a) {
-    const LineEng<T, G> w(a.lt);
+    const LineEng<T, G, false> w(a.lt);
     const int x0 = blockIdx.x << (w.g.nbl() + 1), nr = a.nx - x0;
     const long long zoff = (long long)blockIdx.y * a.ny * a.nx + x0;
     pdl_wait();
@@ -193,68 +203,63 @@ __global__ void HQT_L_BOUNDS1(G) k_ly_d1r(const __grid_constant__ YD1Args<T> a) 
         const long long g = (zoff + (long long)e * a.nx + 2 * b) * st;
         return mk2<T>(2 * b < nr ? p[g] : T(0), 2 * b + 1 < nr ? p[g + st] : T(0));
     };
-    w.first(w.A, [&](int b, int e) { return pair(a.in.re, a.in.st, b, e); });
-    w.forward_mid(1);
+    w.first_d(w.A, [&](int b, int e) { return pair(a.in.re, a.in.st, b, e); });
+    w.forward_mid(false);
     w.middle_deriv1(w.A, a.s1);
-    w.inverse_mid(1);
-    w.last(
-        w.A, [&](int b, int e) { return a.add_re ? pair(a.add_re, 1, b, e) : lzero<T>(); },
+    w.inverse_mid(false);
+    w.last2(
+        false, [&](int b, int e) { return a.add_re ? pair(a.add_re, 1, b, e) : lzero<T>(); },
         [&](int b, int e, C2<T> v, C2<T> x) {
             const int st = a.out.st;
             const long long g = (zoff + (long long)e * a.nx + 2 * b) * st;
             if (2 * b < nr) a.out.re[g] = v.x + x.x;
             if (2 * b + 1 < nr) a.out.re[g + st] = v.y + x.y;
-        });
+        },
+        [](int, int, C2<T>) {});
 }
 
 // Filter, x forward: spectra in natural order, the weight-zeroed columns left
 // unwritten.
 template <typename T, class G>
 __global__ void HQT_L_BOUNDS1(G) k_lx_filt_fwd(const __grid_constant__ XFiltFwdArgs<T> a) {
-    const LineEng<T, G> w(a.lt);
+    const LineEng<T, G, true> w(a.lt);
     const int n = w.g.n(), L0 = blockIdx.x << w.g.nbl(), valid = a.nlines - L0;
     const long long g0 = (long long)L0 * n;
     pdl_wait();
     const int wnd = a.st ? a.st->winding : 0;
     auto at = [&](int b, int e) { return g0 + (long long)b * n + e; };
-    // winding phase -2 pi y w / ny of this thread's line (a thread keeps its
-    // line: the lines per block divide the block)
-    double sn = 0.0, cs = 1.0;
-    if (wnd != 0) {
-        const int y = (L0 + (threadIdx.x & ((1 << w.g.nbl()) - 1))) % a.ny;
+    // winding phase of line L0 + b (tevol_driven_cluster.m:139)
+    auto phase = [&](int b) {
+        const int y = (L0 + b) % a.ny;
         const long long q = ((long long)y * wnd) % a.ny;
+        double sn, cs;
         sincospi(-2.0 * (double)q / (double)a.ny, &sn, &cs);
-    }
+        return mk2<T>((T)cs, (T)sn);
+    };
 #pragma unroll 1
     for (int f = 0; f < a.nf; ++f) {
         // one load expression per kind of field, without branches an element:
         // the loads of a butterfly are in flight together
         const FieldIn<T> in = a.in[f];
+        const bool turn = f == 0 && wnd != 0;
         if (in.c) {
-            const bool turn = f == 0 && wnd != 0;
-            const T c = turn ? (T)cs : T(1), s = turn ? (T)sn : T(0);
-            w.first(w.A, [&](int b, int e) {
-                const C2<T> v = b < valid ? in.c[at(b, e)] : lzero<T>();
-                return turn ? mk2<T>(v.x * c - v.y * s, v.x * s + v.y * c) : v;
-            });
+            w.first(w.A, turn, phase,
+                    [&](int b, int e) { return b < valid ? in.c[at(b, e)] : lzero<T>(); });
         } else {
             const bool pair = in.im != nullptr;
             const T *im = pair ? in.im : in.re;
-            const bool turn = f == 0 && wnd != 0;
-            const T c = turn ? (T)cs : T(1), s = turn ? (T)sn : T(0);
-            w.first(w.A, [&](int b, int e) {
+            w.first(w.A, turn, phase, [&](int b, int e) {
                 if (b >= valid) return lzero<T>();
                 const long long g = at(b, e);
-                C2<T> v = mk2<T>(in.re[g], im[g]);
-                if (!pair) v.y = T(0);
-                return turn ? mk2<T>(v.x * c - v.y * s, v.x * s + v.y * c) : v;
+                const T re = in.re[g], i = im[g];
+                return mk2<T>(re, pair ? i : T(0));
             });
         }
         w.forward_rest();
         C2<T> *spec = a.spec[f];
         w.modes([&](int b, int k) {
             if (b < valid && filt_col_live(k, a.dead0, a.dead1))
-                spec[at(b, k)] = w.A[w.row(w.pos(k)) + b];
+                spec[at(b, k)] = w.A[w.at(b, w.pos(k))];
         });
         __syncthreads();  // the next field's first pass writes other threads' rows
     }
@@ -263,7 +268,7 @@ __global__ void HQT_L_BOUNDS1(G) k_lx_filt_fwd(const __grid_constant__ XFiltFwdA
 // Filter, y: forward, weight, inverse; blockIdx.z = field
 template <typename T, class G>
 __global__ void HQT_L_BOUNDS1(G) k_ly_filt(const __grid_constant__ YFiltArgs<T> a) {
-    const LineEng<T, G> w(a.lt);
+    const LineEng<T, G, false> w(a.lt);
     const int n = w.g.n(), NB = 1 << w.g.nbl();
     const int x0 = blockIdx.x * NB, valid = min(NB, a.nx - x0);
     const long long zoff = (long long)blockIdx.y * a.ny * a.nx + x0;
@@ -274,7 +279,7 @@ __global__ void HQT_L_BOUNDS1(G) k_ly_filt(const __grid_constant__ YFiltArgs<T> 
     C2<T> *spec = a.spec[blockIdx.z];
     auto at = [&](int b, int e) { return zoff + (long long)e * a.nx + b; };
     w.first(w.A, [&](int b, int e) { return b < valid ? spec[at(b, e)] : lzero<T>(); });
-    w.forward_mid(1);
+    w.forward_mid(false);
     w.middle(w.A, [&](auto &v, int b, int blk, int k0, int st) {
         constexpr int R = sizeof(v) / sizeof(C2<T>);
         const int kx = x0 + min(b, valid - 1), kxm = kx == 0 ? 0 : a.nx - kx;
@@ -287,8 +292,8 @@ __global__ void HQT_L_BOUNDS1(G) k_ly_filt(const __grid_constant__ YFiltArgs<T> 
         }
         w.template put<R>(w.A, b, blk, v);
     });
-    w.inverse_mid(1);
-    w.last(w.A, [&](int b, int e, C2<T> v) {
+    w.inverse_mid(false);
+    w.last([&](int b, int e, C2<T> v) {
         if (b < valid) spec[at(b, e)] = v;
     });
 }
@@ -296,7 +301,7 @@ __global__ void HQT_L_BOUNDS1(G) k_ly_filt(const __grid_constant__ YFiltArgs<T> 
 // Filter, x inverse; a non-finite value sets the status' first bad step
 template <typename T, class G>
 __global__ void HQT_L_BOUNDS1(G) k_lx_filt_inv(const __grid_constant__ XFiltInvArgs<T> a) {
-    const LineEng<T, G> w(a.lt);
+    const LineEng<T, G, true> w(a.lt);
     const int n = w.g.n(), L0 = blockIdx.x << w.g.nbl(), valid = a.nlines - L0;
     const long long g0 = (long long)L0 * n;
     pdl_wait();
@@ -306,12 +311,12 @@ __global__ void HQT_L_BOUNDS1(G) k_lx_filt_inv(const __grid_constant__ XFiltInvA
     for (int f = 0; f < a.nf; ++f) {
         const C2<T> *spec = a.spec[f];
         w.modes([&](int b, int k) {
-            w.A[w.row(w.pos(k)) + b] =
+            w.A[w.at(b, w.pos(k))] =
                 b < valid && filt_col_live(k, a.dead0, a.dead1) ? spec[at(b, k)] : lzero<T>();
         });
         w.inverse_begin();
         const FieldOut<T> out = a.out[f];
-        w.last(w.A, [&](int b, int e, C2<T> v) {
+        w.last([&](int b, int e, C2<T> v) {
             if (!(isfinite(v.x) && isfinite(v.y))) bad = 1;
             if (b < valid) store_field(out, at(b, e), v);
         });
@@ -325,7 +330,7 @@ __global__ void HQT_L_BOUNDS1(G) k_lx_filt_inv(const __grid_constant__ XFiltInvA
 // Forward transform along y of nf complex fields, natural order (spectrum)
 template <typename T, class G>
 __global__ void HQT_L_BOUNDS1(G) k_ly_fwd(const __grid_constant__ YFiltArgs<T> a) {
-    const LineEng<T, G> w(a.lt);
+    const LineEng<T, G, false> w(a.lt);
     const int x0 = blockIdx.x << w.g.nbl(), valid = a.nx - x0;
     const long long zoff = (long long)blockIdx.y * a.ny * a.nx + x0;
     pdl_wait();
@@ -336,7 +341,7 @@ __global__ void HQT_L_BOUNDS1(G) k_ly_fwd(const __grid_constant__ YFiltArgs<T> a
         w.first(w.A, [&](int b, int e) { return b < valid ? spec[at(b, e)] : lzero<T>(); });
         w.forward_rest();
         w.modes([&](int b, int k) {
-            if (b < valid) spec[at(b, k)] = w.A[w.row(w.pos(k)) + b];
+            if (b < valid) spec[at(b, k)] = w.A[w.at(b, w.pos(k))];
         });
         __syncthreads();
     }

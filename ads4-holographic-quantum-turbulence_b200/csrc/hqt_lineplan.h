@@ -68,11 +68,11 @@ __host__ __device__ constexpr LPlan lplan(int n) {
     return p;
 }
 
-// Row swizzle mask (hqt_line.cuh): 128 bytes hold this many rows of 2^nbl
-// elements; 0 where rows have no groups of 8.
-__host__ __device__ constexpr int lswz(int n, int nbl, int esize) {
-    const int rows = (128 / esize) >> nbl;
-    return n % 8 == 0 && rows > 1 ? (rows > 8 ? 7 : rows - 1) : 0;
+// Mask of the element swizzle (hqt_line.cuh): along x 8 elements fill 128 bytes;
+// along y 128 bytes hold this many elements of 2^nbl lines.  0 where a line has no
+// groups of 8.  (FP64)
+__host__ __device__ constexpr int lswz(int n, int nbl, bool along_x) {
+    return n % 8 != 0 ? 0 : along_x ? 7 : nbl < 3 ? (8 >> nbl) - 1 : 0;
 }
 // Threads of a block with 2^nbl lines: one radix-8 butterfly each.
 __host__ __device__ constexpr int lthreads(int n, int nbl) {
@@ -80,20 +80,58 @@ __host__ __device__ constexpr int lthreads(int n, int nbl) {
     return t < 32 ? 32 : (t > kLThreads ? kLThreads : t);
 }
 
+// ... with a runtime plan, whose n / R butterflies seldom fill whole rounds of the
+// threads: the multiple of 32 with the least time per block and share of the SM (128
+// registers a thread, nbuf buffers a block), where a round of radix R counts R + 4.
+// From 96 on, or the count above: with smaller blocks the many of them crowd the L1
+// out (384x384x15, filter_x_fwd 100, 72, 86, 85 us with 64, 96, 128, 192 threads).
+// The choice is within 5% of the best of a sweep of 64..512 for the passes of 384,
+// 250x180, 600, 1001, 96x100; 192 or 512 threads for all, as the rule above has it,
+// cost up to a third more (1001x1001x10, filter_x_inv 338 us by this rule, 452
+// by that).
+inline int lthreads_rt(const LPlan &p, int nbl, int nbuf) {
+    const int lo = lthreads(p.n, nbl) < 96 ? lthreads(p.n, nbl) : 96;
+    int best = lo;
+    double least = 0;
+    for (int t = lo; t <= kLThreads; t += 32) {
+        const int fit = (int)(227 * 1024ll / ((16ll * p.n * nbuf << nbl) + 1024));
+        int blocks = kLThreads / t < fit ? kLThreads / t : fit;
+        double time = 0;
+        for (int i = 0; i < p.np; ++i) {
+            const int cnt = (p.n / p.R[i]) << nbl;
+            const int one = (cnt + t - 1) / t, all = (cnt * nbuf + t - 1) / t;
+            time += (one + (i + 1 < p.np ? all : nbuf * one)) * (p.R[i] + 4.0);
+        }
+        time /= blocks < 1 ? 1 : blocks;
+        if (least == 0 || time < least) {
+            least = time;
+            best = t;
+        }
+    }
+    return best;
+}
+
 // Compile-time geometry: N points, 2^NBL lines per block.
 template <int N_, int NBL_> struct SGeo;
 // Runtime geometry, a kernel argument.
 struct RGeo {
     static constexpr bool kStatic = false;
+    static constexpr int kN = 0;
     static constexpr int kMaxThreads = kLThreads;
-    int n_, nbl_, np_, th_, swz_;
+    int n_, nbl_, np_, swz_;
+    int th_[2];    // threads of a block with one and two buffers
+    unsigned mn_;  // ceil(2^32 / n)
     int R_[kLMaxPass], s_[kLMaxPass], tw_[kLMaxPass];
-    unsigned mg_[kLMaxPass];  // ceil(2^32 / s)
+    unsigned mg_[kLMaxPass], mr_[kLMaxPass];  // ceil(2^32 / s), ceil(2^32 / (n / R))
     __host__ __device__ __forceinline__ int n() const { return n_; }
     __host__ __device__ __forceinline__ int nbl() const { return nbl_; }
     __host__ __device__ __forceinline__ int np() const { return np_; }
-    __host__ __device__ __forceinline__ int threads() const { return th_; }
-    template <typename T> __host__ __device__ __forceinline__ int swz() const { return swz_; }
+    int block(int nbuf) const { return th_[nbuf - 1]; }
+    template <typename T, bool AX> __host__ __device__ __forceinline__ int swz() const {
+        return swz_;
+    }
+    __host__ __device__ __forceinline__ unsigned mn() const { return mn_; }
+    __host__ __device__ __forceinline__ unsigned mr(int p) const { return mr_[p]; }
     __host__ __device__ __forceinline__ int R(int p) const { return R_[p]; }
     __host__ __device__ __forceinline__ int s(int p) const { return s_[p]; }
     __host__ __device__ __forceinline__ int tw(int p) const { return tw_[p]; }
@@ -101,16 +139,18 @@ struct RGeo {
 };
 template <int N_, int NBL_> struct SGeo {
     static constexpr bool kStatic = true;
-    static constexpr int N = N_, NBL = NBL_, kMaxThreads = lthreads(N_, NBL_);
+    static constexpr int N = N_, kN = N_, NBL = NBL_, kMaxThreads = lthreads(N_, NBL_);
     static_assert(lplan(N_).np >= 2, "no in-place plan for this length");
     __host__ __device__ static constexpr int np() { return lplan(N_).np; }
     __host__ __device__ SGeo(const RGeo &) {}
     __host__ __device__ static constexpr int n() { return N_; }
     __host__ __device__ static constexpr int nbl() { return NBL_; }
+    static constexpr int block(int) { return lthreads(N_, NBL_); }
     __host__ __device__ static constexpr int threads() { return lthreads(N_, NBL_); }
-    template <typename T> __host__ __device__ static constexpr int swz() {
-        return lswz(N_, NBL_, 2 * (int)sizeof(T));
+    template <typename T, bool AX> __host__ __device__ static constexpr int swz() {
+        return lswz(N_, NBL_, AX);
     }
+    __host__ __device__ static constexpr unsigned mn() { return 0u; }
 };
 
 // Device tables of one axis and the runtime plan.
@@ -121,17 +161,15 @@ template <typename T> struct LineTab {
     RGeo g;
 };
 
-// log2 of the lines per block.  x lines are contiguous, so 4 lines give a
-// warp 128-byte runs; y lines are adjacent columns, of which 8 fill a 128-byte
-// row.  Two buffers of the block's lines stay within about 64 KB (three
-// blocks per SM); for y lines above HQT_YBIG points four columns (64-byte
-// rows) in up to 128 KB.
-#ifndef HQT_YBUD
-#define HQT_YBUD 130
+// log2 of the lines per block.  Two buffers of the block's lines stay within about
+// 64 KB (three blocks per SM); y lines are adjacent columns, of which 8 fill a
+// 128-byte row, and take up to 128 KB for at least 4 of them.
+#ifndef HQT_YMIN
+#define HQT_YMIN 2
 #endif
 __host__ __device__ constexpr int lnbl(int n, bool along_y) {
     int b = along_y ? 3 : 2;
-    while (b > 0 && (n * 32ll << b) > (along_y && b == 2 ? HQT_YBUD : 66) * 1024ll) --b;
+    while (b > 0 && (n * 32ll << b) > (along_y && b <= HQT_YMIN ? 130 : 66) * 1024ll) --b;
     return b;
 }
 
