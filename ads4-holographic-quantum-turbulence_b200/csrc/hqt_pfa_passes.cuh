@@ -179,7 +179,7 @@ __global__ void __launch_bounds__(32) k_x_rhs_pfa(const __grid_constant__ XRhsAr
     cp_commit();
     cp_wait<0>();
     __syncwarp();
-    w.template stage_a<-1>(L.b0, L_t::in_place(L.b0));
+    w.template stage_a<-1, true>(L.b0, L_t::in_place(L.b0));
     __syncwarp();
     w.stage_b_deriv12(L.b0, L.b1, a.s1, a.s2, cs);
     __syncwarp();
@@ -194,7 +194,7 @@ __global__ void __launch_bounds__(32) k_x_rhs_pfa(const __grid_constant__ XRhsAr
     cp_wait<0>();
     __syncwarp();
     // C: first derivative in b0, second in b1
-    w.template stage_a<-1>(L.b1, L_t::in_place(L.b1));
+    w.template stage_a<-1, true>(L.b1, L_t::in_place(L.b1));
     __syncwarp();
     w.stage_b_deriv12(L.b1, L.b0, a.s1, a.s2, cs);
     __syncwarp();
@@ -237,7 +237,7 @@ __global__ void __launch_bounds__(32) k_y_rhs_pfa(const __grid_constant__ YRhsAr
     cp_commit();
     cp_wait<0>();
     __syncwarp();
-    w.template stage_a<-1>(L.b0, L_t::in_place(L.b0));
+    w.template stage_a<-1, true>(L.b0, L_t::in_place(L.b0));
     __syncwarp();
     w.stage_b_deriv12(L.b0, L.b1, a.s1, a.s2, cs);
     __syncwarp();
@@ -266,10 +266,10 @@ __global__ void __launch_bounds__(32) k_y_rhs_pfa(const __grid_constant__ YRhsAr
     cp_commit();
     cp_wait<1>();
     __syncwarp();
-    w.template stage_a<-1>(L.b1, L_t::in_place(L.b1));
+    w.template stage_a<-1, true>(L.b1, L_t::in_place(L.b1));
     cp_wait<0>();
     __syncwarp();
-    w.template stage_a<-1>(L.b0, L_t::in_place(L.b0));
+    w.template stage_a<-1, true>(L.b0, L_t::in_place(L.b0));
     __syncwarp();
     // C (W1) in c0, E (W2) in c1
     const PfaBuf<T> c0 = L.b1, c1 = L.b0;
@@ -405,7 +405,7 @@ __global__ void __launch_bounds__(32) k_x_d1_pfa(const __grid_constant__ XD1Args
     cp_commit();
     cp_wait<0>();
     __syncwarp();
-    w.template stage_a<-1>(L.b0, L_t::in_place(L.b0));
+    w.template stage_a<-1, true>(L.b0, L_t::in_place(L.b0));
     __syncwarp();
     w.template stage_b_deriv<1>(L.b0, L.b1, a.s1, T(0), cs);
     __syncwarp();
@@ -431,7 +431,7 @@ __global__ void __launch_bounds__(32) k_y_d1_pfa(const __grid_constant__ YD1Args
     cp_commit();
     cp_wait<0>();
     __syncwarp();
-    w.template stage_a<-1>(L.b0, L_t::in_place(L.b0));
+    w.template stage_a<-1, true>(L.b0, L_t::in_place(L.b0));
     __syncwarp();
     w.template stage_b_deriv<1>(L.b0, L.b1, a.s1, T(0), cs);
     __syncwarp();
@@ -475,7 +475,7 @@ __global__ void __launch_bounds__(32) k_x_d1r_pfa(const __grid_constant__ XD1Arg
     cp_commit();
     cp_wait<0>();
     __syncwarp();
-    w.template stage_a<-1>(L.b0, L_t::in_place(L.b0));
+    w.template stage_a<-1, true>(L.b0, L_t::in_place(L.b0));
     __syncwarp();
     w.template stage_b_deriv<1>(L.b0, L.b1, a.s1, T(0), cs);
     __syncwarp();
@@ -511,7 +511,7 @@ __global__ void __launch_bounds__(32) k_y_d1r_pfa(const __grid_constant__ YD1Arg
     cp_commit();
     cp_wait<0>();
     __syncwarp();
-    w.template stage_a<-1>(L.b0, L_t::in_place(L.b0));
+    w.template stage_a<-1, true>(L.b0, L_t::in_place(L.b0));
     __syncwarp();
     w.template stage_b_deriv<1>(L.b0, L.b1, a.s1, T(0), cs);
     __syncwarp();
