@@ -1,5 +1,6 @@
 // hqt_z_impl.cuh -- launchers of the column kernels for one column length
 // HQT_ZN (each hqt_z<N>.cu defines HQT_ZN and includes this file).
+#include <cmath>
 #include <cstring>
 #include <type_traits>
 #include <vector>
@@ -78,12 +79,20 @@ void z_tables<HQT_ZN>(const ZHost &h, std::vector<double> &frag, std::vector<dou
     });
     put(D::MH, D::KO, [&](int i, int j) {
         if (i >= hf || j >= nz / 2) return 0.0;
+        if (j == 0) return 1.0;  // the end values' line
         return 0.5 * (L(i, j) - L(i, n1 - j));
     });
     put(D::M1, D::K1, [&](int i, int j) {
         return i < n1 && j < n1 ? h.Lz1[(size_t)i * n1 + j] : 0.0;
     });
-    tab.assign(3 * HQT_ZN, 0.0);
+    tab.assign(D::ntab, 0.0);
+    // 2 (1 - z_j) = 2 sin^2(j pi/2n'): from zz it would be off by the rounding of
+    // z near 1, which Lz multiplies by n'^2
+    tab[3 * HQT_ZN] = 1.0;
+    for (int j = 1; j < nz / 2; ++j) {
+        const double s = std::sin(j * 3.14159265358979323846 / (2.0 * n1));
+        tab[3 * HQT_ZN + j] = 2.0 * s * s;
+    }
     for (int i = 0; i < nz; ++i) {
         tab[i] = h.zz[i];
         tab[HQT_ZN + i] = 1.0 - h.zz[i] * h.zz[i] * h.zz[i];

@@ -24,6 +24,7 @@ template <int NZP> struct ZsDims {
     static constexpr int MH = (HE + 7) / 8, MP = (HO + 7) / 8;
     static constexpr int KE = (HE + 3) / 4, KO = (HO + 3) / 4;
     static constexpr int M1 = (NZP - 1 + 7) / 8, K1 = (NZP - 1 + 3) / 4;
+    static constexpr int ntab = 3 * NZP + 4 * KE;  // z, f, Lz(nz,:), line factors
     static constexpr int VR = NZP > 4 * K1 ? NZP : 4 * K1;  // rows of a scratch field
     static constexpr int nfrag = MP * KE + MH * KO + M1 * K1;
     // state and accumulator are read straight from global memory instead of staged

@@ -18,6 +18,15 @@
 // instead of 18, of 33 levels 22 instead of 45, and the fragments of both
 // operators fit in registers at 33 levels too (108 instead of 180).
 //
+// e and o mix the two ends of a column, where the entries of Lz are about 2/3 n'^2: a
+// field that vanishes at the boundary would pick up there the rounding of its
+// horizon values (F1 of a nearly static state 3 to 5 times less exact than by the
+// full product).  So the line through the end values is taken out first, x = w +
+// x_{n'} + z d with d = x_0 - x_{n'}: w vanishes at both ends, Lz x = Lz w + d, and
+//   e_j = (x_j - x_0) + (x_{n'-j} - x_{n'}),
+//   o_j = (x_j - x_0) - (x_{n'-j} - x_{n'}) + 2 (1 - z_j) d.
+// e_0 = o_0 = 0, so the slot j = 0 of o carries d, with ones in Lo.
+//
 // A tile's fields come in by TMA, one box per field, in two groups with an mbarrier
 // each: the main inputs, and the RK state and accumulator.  A group's region is
 // refilled with the next tile's as soon as every warp is done with it.  Fields
@@ -77,8 +86,8 @@ template <typename TD, int NZP, int MODE> struct ZsLay {
     static constexpr int oDIV = oYY + rd, oZA = oDIV + rr, oZP = oZA + (z ? rc : 0);
     static constexpr int oKA = oZP + (z ? rc : 0), oKP = oKA + (k ? rc : 0);
     static constexpr int oVA = oKP + (k ? rc : 0), rv = up(ZsDims<NZP>::VR * kZsRow);
-    static constexpr int oVB = oVA + rv, oTAB = oVB + rv;  // z, f, Lz(nz,:)
-    static constexpr int oBAR = oTAB + up(3 * NZP * 8);
+    static constexpr int oVB = oVA + rv, oTAB = oVB + rv;  // z, f, Lz(nz,:), line
+    static constexpr int oBAR = oTAB + up(ZsDims<NZP>::ntab * 8);
     static constexpr int bytes = oBAR + 64 + 128;  // + alignment of the base
 };
 
@@ -171,21 +180,25 @@ template <int NZP> struct ZsOps {
         return *reinterpret_cast<const double *>(
             reinterpret_cast<unsigned char *>(&zs_at<OFF>(sm, j, cop)) + part);
     }
-    // (yA, yB)[m] = Lz x at levels i = 8m + zs_row(g) and n1 - i for the fields at
-    // OFF (into y) and OFF2 (into w): two sets of independent mma chains
-    template <int OFF, int OFF2>
-    __device__ __forceinline__ void lz2(unsigned char *sm, double (&yA)[MH][2], double (&yB)[MH][2],
-                                        double (&wA)[MH][2], double (&wB)[MH][2]) const {
+    // (yA, yB)[m] = Lz x at levels i = 8m + zs_row(g) and n1 - i for the operands
+    // x(level) (into y) and v(level) (into w): two sets of independent mma chains;
+    // line[j]: factor of the end values' difference in o_j
+    template <typename X, typename V>
+    __device__ __forceinline__ void lz2(X x, V v, const double *line, double (&yA)[MH][2],
+                                        double (&yB)[MH][2], double (&wA)[MH][2],
+                                        double (&wB)[MH][2]) const {
 #pragma unroll
         for (int m = 0; m < MH; ++m)
             yA[m][0] = yA[m][1] = yB[m][0] = yB[m][1] = wA[m][0] = wA[m][1] = wB[m][0] =
                 wB[m][1] = 0.0;
+        const double x0 = x(0), xn = x(n1), dx = x0 - xn, v0 = v(0), vn = v(n1), dv = v0 - vn;
 #pragma unroll
         for (int s = 0; s < KE; ++s) {
             const int j = min(4 * s + q, n1), jm = max(n1 - 4 * s - q, 0);
-            const double x1 = operand<OFF>(sm, j), x2 = operand<OFF>(sm, jm);
-            const double v1 = operand<OFF2>(sm, j), v2 = operand<OFF2>(sm, jm);
-            const double e = x1 + x2, o = x1 - x2, ve = v1 + v2, vo = v1 - v2;
+            const double x1 = x(j) - x0, x2 = x(jm) - xn, v1 = v(j) - v0, v2 = v(jm) - vn;
+            const double t = line[4 * s + q];
+            const double e = x1 + x2, o = fma(t, dx, x1 - x2);
+            const double ve = v1 + v2, vo = fma(t, dv, v1 - v2);
 #pragma unroll
             for (int m = 0; m < MP; ++m) {
                 dmma(yA[m][0], yA[m][1], Fe[m][s], e);
@@ -199,16 +212,39 @@ template <int NZP> struct ZsOps {
                 }
             }
         }
-        // P in yA, Q in yB: y_i = P + Q, y_{n1-i} = Q - P
+        merge(yA, yB);
+        merge(wA, wB);
+    }
+    // ... for one
+    template <typename X>
+    __device__ __forceinline__ void lz(X x, const double *line, double (&yA)[MH][2],
+                                       double (&yB)[MH][2]) const {
+#pragma unroll
+        for (int m = 0; m < MH; ++m) yA[m][0] = yA[m][1] = yB[m][0] = yB[m][1] = 0.0;
+        const double x0 = x(0), xn = x(n1), dx = x0 - xn;
+#pragma unroll
+        for (int s = 0; s < KE; ++s) {
+            const int j = min(4 * s + q, n1), jm = max(n1 - 4 * s - q, 0);
+            const double x1 = x(j) - x0, x2 = x(jm) - xn;
+            const double e = x1 + x2, o = fma(line[4 * s + q], dx, x1 - x2);
+#pragma unroll
+            for (int m = 0; m < MP; ++m) dmma(yA[m][0], yA[m][1], Fe[m][s], e);
+            if (s < KO) {
+#pragma unroll
+                for (int m = 0; m < MH; ++m) dmma(yB[m][0], yB[m][1], Fo[m][s < KO ? s : 0], o);
+            }
+        }
+        merge(yA, yB);
+    }
+    // P in yA, Q in yB: y_i = P + Q, y_{n1-i} = Q - P
+    __device__ __forceinline__ static void merge(double (&yA)[MH][2], double (&yB)[MH][2]) {
 #pragma unroll
         for (int m = 0; m < MH; ++m)
 #pragma unroll
             for (int i = 0; i < 2; ++i) {
-                const double p = yA[m][i], r = yB[m][i], u = wA[m][i], v = wB[m][i];
+                const double p = yA[m][i], r = yB[m][i];
                 yA[m][i] = r + p;
                 yB[m][i] = r - p;
-                wA[m][i] = v + u;
-                wB[m][i] = v - u;
             }
     }
     // F[m] = Lz1 x at levels 8m + zs_row(g) (zero at nz - 1 and past it)
@@ -267,8 +303,8 @@ __global__ void __launch_bounds__(kZsThreads, ZsDims<NZP>::min_blocks)
     const unsigned barM = sb + Lay::oBAR, barZ = barM + 8;
     double *tab = reinterpret_cast<double *>(sm + Lay::oTAB);
     const bool leader = threadIdx.x == 0;  // issues the copies
-    // z, f = 1 - z^3 and Lz(nz,:); V rows past nz are zero in every product
-    for (int i = threadIdx.x; i < 3 * NZP; i += kZsThreads) tab[i] = __ldg(a.ztab + i);
+    // z, f = 1 - z^3, Lz(nz,:) and the line's factors; V rows past nz are zero in every product
+    for (int i = threadIdx.x; i < D::ntab; i += kZsThreads) tab[i] = __ldg(a.ztab + i);
     for (int i = threadIdx.x; i < 2 * Lay::rv / 16; i += kZsThreads)
         reinterpret_cast<double2 *>(sm + Lay::oVA)[i] = make_double2(0.0, 0.0);
     if (threadIdx.x == 0) {
@@ -353,7 +389,9 @@ __global__ void __launch_bounds__(kZsThreads, ZsDims<NZP>::min_blocks)
         double dA[MH][2], dB[MH][2];  // dp
         {
             double yA[MH][2], yB[MH][2];
-            ops.template lz2<Lay::oAXY, Lay::oPS>(sm, yA, yB, dA, dB);
+            ops.lz2([&](int j) { return ops.template operand<Lay::oAXY>(sm, j); },
+                    [&](int j) { return ops.template operand<Lay::oPS>(sm, j); }, tab + 3 * NZP,
+                    yA, yB, dA, dB);
             auto put = [&](int i, const double (&y)[2], const double (&d)[2]) {
                 const PD dt = zs_pair<Lay::oDT, TD>(sm, i, col);
                 const double f = tab[NZP + i];
@@ -375,7 +413,9 @@ __global__ void __launch_bounds__(kZsThreads, ZsDims<NZP>::min_blocks)
         double kb = 0.0;  // Lz(nz,:) div A of the column
         {
             double yA[MH][2], yB[MH][2], eA[MH][2], eB[MH][2];
-            ops.template lz2<Lay::oVA, Lay::oVB>(sm, yA, yB, eA, eB);
+            ops.lz2([&](int j) { return ops.template operand<Lay::oVA>(sm, j); },
+                    [&](int j) { return ops.template operand<Lay::oVB>(sm, j); }, tab + 3 * NZP,
+                    yA, yB, eA, eB);
             __syncwarp();  // VA and VB are read: the sources overwrite them
             auto put = [&](int i, const double (&y)[2], const double (&d1)[2],
                            const double (&d2)[2]) {
