@@ -32,7 +32,6 @@
 
 namespace hqt {
 
-static constexpr int kThreadsFFT = 128;
 static constexpr int kThreadsZ = 128;
 static constexpr size_t kSmemBudget = 54 * 1024;
 static constexpr int kPartials = 296;
@@ -642,19 +641,26 @@ int launch_filter(hqt_ctx *c, int nf, const FieldIn<double> *in, const FieldOut<
     return HQT_OK;
 }
 
-// Tensor map of a field [nz][plane] of `comps` values of type T per site: boxes of
-// `width` sites x nz levels.  The level rows must be a multiple of 16 bytes apart.
+// Tensor maps of a field [nz][plane] of `comps` values of type T per site, one per
+// group of levels (ZsSplit): boxes of `width` sites x the group's levels.
 template <typename T>
 int zs_map(hqt_ctx *c, CUtensorMap *m, const void *base, int comps, int width) {
-    const cuuint64_t dims[2] = {(cuuint64_t)comps * c->plane, (cuuint64_t)c->nz};
-    const cuuint64_t strides[1] = {(cuuint64_t)comps * sizeof(T) * c->plane};
-    const cuuint32_t box[2] = {(cuuint32_t)(width * comps), (cuuint32_t)c->nz}, es[2] = {1, 1};
-    const CUresult r = c->tmap_encode(
-        m, sizeof(T) == 8 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT64 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2,
-        const_cast<void *>(base), dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
-        CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-        CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (r != CUDA_SUCCESS) return fail(c, HQT_ECUDA, "tensor map");
+    const long long row = (long long)comps * c->plane * sizeof(T);
+    const ZsSplit sp(c->nz, row, width * comps * (int)sizeof(T));
+    for (int ph = 0; ph < sp.n && ph < c->nz; ++ph) {
+        const int shift = sp.shift(ph);
+        const cuuint64_t dims[2] = {(cuuint64_t)(row + shift) / sizeof(T), (cuuint64_t)sp.rows(ph)};
+        const cuuint64_t strides[1] = {(cuuint64_t)(row << sp.lg)};
+        const cuuint32_t box[2] = {(cuuint32_t)(width * comps), (cuuint32_t)sp.rows(ph)};
+        const cuuint32_t es[2] = {1, 1};
+        const CUresult r = c->tmap_encode(
+            m + ph,
+            sizeof(T) == 8 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT64 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2,
+            const_cast<char *>(static_cast<const char *>(base) + ph * row - shift), dims, strides,
+            box, es, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
+            CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+        if (r != CUDA_SUCCESS) return fail(c, HQT_ECUDA, "tensor map");
+    }
     return HQT_OK;
 }
 
@@ -667,20 +673,17 @@ template <typename TD> int launch_zstage(hqt_ctx *c, int mode, ZStageArgs<TD> a)
     a.frag = c->zfrag;
     a.ztab = c->ztab;
     a.fault = &c->st->fault;
-    a.copy_pairs = c->plane * sizeof(C2<TD>) % 16 != 0;
-    a.copy_real = c->plane * sizeof(TD) % 16 != 0;
     struct {
         CUtensorMap *m;
         const void *p;
     } full[] = {{&a.mPS, a.ypsi}, {&a.mAXY, a.yA},   {&a.mATD, a.atd}, {&a.mZA, a.zA},
                 {&a.mKA, a.kA},   {&a.mZP, a.zpsi}, {&a.mKP, a.kpsi}},
-      pairs[] = {{&a.mDX, a.dxpsi}, {&a.mDY, a.dypsi}, {&a.mDT, a.dAt},
-                 {&a.mB, a.B},      {&a.mXX, a.dxxpsi}, {&a.mYY, a.dyypsi}};
+      pairs[] = {{a.mDX, a.dxpsi}, {a.mDY, a.dypsi}, {a.mDT, a.dAt},
+                 {a.mB, a.B},      {a.mXX, a.dxxpsi}, {a.mYY, a.dyypsi}};
     for (auto &f : full)
         if (f.p) RC(zs_map<double>(c, f.m, f.p, 2, zs_row_td<double>() / 16));
-    if (!a.copy_pairs)
-        for (auto &f : pairs) RC(zs_map<TD>(c, f.m, f.p, 2, zs_row_td<TD>() / (int)sizeof(C2<TD>)));
-    if (!a.copy_real) RC(zs_map<TD>(c, &a.mDIV, a.divA, 1, zs_row_r<TD>() / (int)sizeof(TD)));
+    for (auto &f : pairs) RC(zs_map<TD>(c, f.m, f.p, 2, zs_row_td<TD>() / (int)sizeof(C2<TD>)));
+    RC(zs_map<TD>(c, a.mDIV, a.divA, 1, zs_row_r<TD>() / (int)sizeof(TD)));
     Prof pr(c, K_ZSTAGE);
     switch (c->NZP) {
 #define HQT_Z(N)                                                       \
@@ -708,11 +711,16 @@ int launch_zcons(hqt_ctx *c) {
     a.divA = c->divA;
     a.rho = c->rho;
     a.O = c->O;
+    a.frag = c->zfrag;
+    a.ztab = c->ztab;
+    a.fault = &c->st->fault;
+    RC(zs_map<double>(c, &a.mPS, a.psi, 2, kZcRowP / 16));
+    RC(zs_map<double>(c, a.mDIV, a.divA, 1, kZcRowD / 8));
     Prof pr(c, K_ZCONS);
     switch (c->NZP) {
 #define HQT_Z(N)                                   \
     case N:                                        \
-        CK(z_cons<N>(a, zhost(c), c->stream));     \
+        CK(z_cons<N>(a, c->stream));               \
         return HQT_OK;
         HQT_NZP_LIST(HQT_Z)
 #undef HQT_Z

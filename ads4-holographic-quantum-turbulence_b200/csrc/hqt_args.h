@@ -140,19 +140,17 @@ template <typename T, int NZP> struct ZOps {
 
 // Radial stage (hqt_zstage.cuh).  TD: type of the horizontal-derivative fields
 // written by the line passes; all else is FP64.  Pairs of real fields are
-// interleaved.  Inputs come by the tensor maps, or by the pointers where a
-// field's level rows are not 16 bytes apart modulo 16 (copy_pairs: the TD pairs,
-// copy_real: div A).
+// interleaved.  Inputs come by the tensor maps, one per group of levels (ZsSplit).
 template <typename TD> struct ZStageArgs {
     CUtensorMap mPS, mAXY;        // stage input Psi, (A_x, A_y)
-    CUtensorMap mDX, mDY;         // d_x Psi, d_y Psi
-    CUtensorMap mDT, mB;          // (d_x A_t, d_y A_t), (d_y B, d_x B)
+    CUtensorMap mDX[2], mDY[2];   // d_x Psi, d_y Psi
+    CUtensorMap mDT[2], mB[2];    // (d_x A_t, d_y A_t), (d_y B, d_x B)
     CUtensorMap mZA, mKA;         // state and RK accumulator of (A_x, A_y)
     CUtensorMap mATD;             // (A_t, d_z A_t)
-    CUtensorMap mXX, mYY, mDIV;   // d_xx Psi, d_yy Psi (their sum is lap Psi), div A
+    CUtensorMap mXX[2], mYY[2];   // d_xx Psi, d_yy Psi (their sum is lap Psi)
+    CUtensorMap mDIV[4];          // div A
     CUtensorMap mZP, mKP;         // state and RK accumulator of Psi
     int nz;
-    int copy_pairs, copy_real;
     long long plane;  // nx*ny
     double h;
     const double *frag;  // operator fragments per lane (make_zstage_tables)
@@ -187,6 +185,9 @@ template <typename T> struct ZConsArgs {
     const T *divA;
     const T *rho;  // 2-D
     C2<T> *O;      // 2-D boundary order parameter (may be null)
+    const double *frag, *ztab;  // operand tables (hqt_zdims.h)
+    int *fault;                 // set when a copy never completed
+    CUtensorMap mPS, mDIV[2];   // Psi, div A (ZsSplit)
 };
 
 template <typename T> struct ZColArgs {

@@ -97,7 +97,7 @@ void z_tables(const ZHost &h, std::vector<double> &frag, std::vector<double> &ta
 template <int N> cudaError_t z_stage(int mode, const ZStageArgs<double> &a, cudaStream_t s);
 template <int N> cudaError_t z_stage_mixed(int mode, const ZStageArgs<float> &a, cudaStream_t s);
 template <int N>
-cudaError_t z_cons(const ZConsArgs<double> &a, const ZHost &h, cudaStream_t s);
+cudaError_t z_cons(const ZConsArgs<double> &a, cudaStream_t s);
 template <int N>
 cudaError_t z_misc(const ZColArgs<double> &a, const ZHost &h, int grid, int threads,
                    cudaStream_t s);
@@ -120,7 +120,7 @@ namespace hqt {
     template <> cudaError_t z_stage<N>(int, const ZStageArgs<double> &, cudaStream_t);     \
     template <> cudaError_t z_stage_mixed<N>(int, const ZStageArgs<float> &, cudaStream_t); \
     template <>                                                                            \
-    cudaError_t z_cons<N>(const ZConsArgs<double> &, const ZHost &, cudaStream_t);             \
+    cudaError_t z_cons<N>(const ZConsArgs<double> &, cudaStream_t);                            \
     template <>                                                                            \
     cudaError_t z_misc<N>(const ZColArgs<double> &, const ZHost &, int, int, cudaStream_t);
 HQT_NZP_LIST(HQT_ZDECL)

@@ -7,7 +7,7 @@
 
 #include "hqt_launch.h"
 #include "hqt_zcol.cuh"
-#include "hqt_zfused.cuh"
+#include "hqt_zcons.cuh"
 #include "hqt_zstage.cuh"
 
 #ifndef HQT_ZN
@@ -50,7 +50,7 @@ template <> cudaError_t z_init<HQT_ZN>(int max_smem) {
     opt((const void *)k_zstage<float, HQT_ZN, 2>);
     opt((const void *)k_zstage<float, HQT_ZN, 3>);
     opt((const void *)k_zstage<float, HQT_ZN, 4>);
-    opt((const void *)k_zcons_tc<HQT_ZN>);
+    opt((const void *)k_zcons<HQT_ZN>);
     return e;
 }
 
@@ -145,22 +145,20 @@ cudaError_t z_stage_mixed<HQT_ZN>(int mode, const ZStageArgs<float> &a, cudaStre
 }
 
 template <>
-cudaError_t z_cons<HQT_ZN>(const ZConsArgs<double> &a, const ZHost &h, cudaStream_t s) {
+cudaError_t z_cons<HQT_ZN>(const ZConsArgs<double> &a, cudaStream_t s) {
     static int per_sm = 0, nsm = 0;
-    constexpr size_t smem = zcons_smem_bytes<HQT_ZN>();
+    constexpr int smem = ZcLay<HQT_ZN>::bytes;
     if (per_sm == 0) {
         int dev = 0;
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_zcons_tc<HQT_ZN>, kZThreads,
-                                                      smem);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_zcons<HQT_ZN>, kZsThreads, smem);
         if (per_sm < 1) per_sm = 1;
     }
-    const long long tiles = (a.plane + kZConsSites - 1) / kZConsSites;
+    const long long tiles = (a.plane + kZcSites - 1) / kZcSites;
     const long long full = (long long)per_sm * (nsm > 0 ? nsm : 1);
-    const ZOps<double, HQT_ZN> op = make_zops(h);
-    (void)klaunch(k_zcons_tc<HQT_ZN>, dim3((int)(tiles < full ? tiles : full)), dim3(kZThreads),
-                  smem, s, a, op);
+    (void)klaunch(k_zcons<HQT_ZN>, dim3((int)(tiles < full ? tiles : full)), dim3(kZsThreads),
+                  smem, s, a);
     return cudaGetLastError();
 }
 

@@ -10,8 +10,8 @@
 // of the nz-point operators.
 //
 // k_zcol_misc computes d_z A_t and O alone (set-up and diagnostics).  The
-// RK stages run in k_zstage and the post-combine constraint in k_zcons_tc,
-// both on block tiles and FP64 tensor-core products (hqt_zfused.cuh).
+// RK stages run in k_zstage and the post-combine constraint in k_zcons,
+// both on block tiles and FP64 tensor-core products (hqt_zstage.cuh, hqt_zcons.cuh).
 #pragma once
 #include "hqt_dev.cuh"
 #include "hqt_args.h"

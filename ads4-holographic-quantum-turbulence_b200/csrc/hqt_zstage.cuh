@@ -31,8 +31,9 @@
 // each: the main inputs, and the RK state and accumulator.  A group's region is
 // refilled with the next tile's as soon as every warp is done with it.  Fields
 // whose level rows are not a multiple of 16 bytes apart (a real field or FP32
-// pairs with an odd nx*ny) take cp.async copies by all threads onto the same
-// barrier.
+// pairs with an odd nx*ny) come as two or four groups of levels (ZsSplit).  (By
+// cp.async of all threads, 4 or 8 bytes each, a launch took 1044 us at 1001x1001x20,
+// now 924, and of 301x301x21 in mixed precision 123, now 109.)
 //
 // What bounds it: the copies.  TMA takes about 8.5 cycles per box row whatever its
 // width up to 256 bytes, so 8-column tiles (128-byte rows) loaded 4.5 TB/s however
@@ -64,19 +65,35 @@
 #include "hqt_args.h"
 #include "hqt_dev.cuh"
 #include "hqt_zdims.h"
-#include "hqt_zfused.cuh"
 
 namespace hqt {
 
 constexpr int kZsThreads = 128;
+
+// d += a * b on one 8x8x4 FP64 tensor-core tile
+__device__ __forceinline__ void dmma(double &d0, double &d1, double a, double b) {
+    asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
+        : "+d"(d0), "+d"(d1)
+        : "d"(a), "d"(b));
+}
+// Sum over the 8 lane groups g = lane/4 (same column q): after the shuffles
+// every lane holds the total of its column.
+__device__ __forceinline__ double zf_colsum(double v) {
+    v += __shfl_xor_sync(0xffffffffu, v, 4);
+    v += __shfl_xor_sync(0xffffffffu, v, 8);
+    v += __shfl_xor_sync(0xffffffffu, v, 16);
+    return v;
+}
 
 __device__ __forceinline__ int zs_col(int warp, int k) { return ((k & 1) << 2) + (k >> 1) + 2 * (warp & 1) + 8 * (warp >> 1); }
 
 // Shared-memory layout of a block.
 template <typename TD, int NZP, int MODE> struct ZsLay {
     static constexpr int up(int b) { return (b + 127) / 128 * 128; }
-    static constexpr int rc = up(NZP * kZsRow), rd = up(NZP * zs_row_td<TD>());
-    static constexpr int rr = up(NZP * zs_row_r<TD>());
+    static constexpr int rc = up(NZP * kZsRow);
+    // (a group of levels each, ZsSplit)
+    static constexpr int rd = up(NZP * zs_row_td<TD>()) + (sizeof(TD) == 8 ? 0 : 128);
+    static constexpr int rr = up(NZP * zs_row_r<TD>()) + (sizeof(TD) == 8 ? 128 : 384);
     // state and accumulator staged (DIRECT: read from global memory where they are
     // used; stage 1: the state is the stage input, copied aside for the update)
     static constexpr bool k = MODE >= 2 && !ZsDims<NZP>::direct;
@@ -87,7 +104,8 @@ template <typename TD, int NZP, int MODE> struct ZsLay {
     static constexpr int oKA = oZP + (z ? rc : 0), oKP = oKA + (k ? rc : 0);
     static constexpr int oVA = oKP + (k ? rc : 0), rv = up(ZsDims<NZP>::VR * kZsRow);
     static constexpr int oVB = oVA + rv, oTAB = oVB + rv;  // z, f, Lz(nz,:), line
-    static constexpr int oBAR = oTAB + up(ZsDims<NZP>::ntab * 8);
+    static constexpr int oROW = oTAB + up(ZsDims<NZP>::ntab * 8);  // rows of div A
+    static constexpr int oBAR = oROW + up(NZP * 4);
     static constexpr int bytes = oBAR + 64 + 128;  // + alignment of the base
 };
 
@@ -122,33 +140,18 @@ __device__ __forceinline__ void zs_tma(unsigned dst, const CUtensorMap *map, int
         "l"(map), "r"(x), "r"(0), "r"(bar)
         : "memory");
 }
-// the same by cp.async (sites past the plane are left as they are: their
-// columns are never stored); arrives on `bar` when this thread's are in
-template <typename V, int PITCH>
-__device__ __forceinline__ void zs_copy(unsigned char *dst, const V *src, int nz, long long P,
-                                        long long site0) {
-    for (int e = threadIdx.x; e < nz * kZsCols; e += kZsThreads) {
-        const int l = e / kZsCols, c = e % kZsCols;
-        if (site0 + c < P)
-            cp_async<sizeof(V)>(dst + l * PITCH + c * sizeof(V), src + (long long)l * P + site0 + c);
-    }
-}
-__device__ __forceinline__ void zs_copy_arrive(unsigned bar) {
-    asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];\n" ::"r"(bar) : "memory");
-}
-
-// Element (level, column) of the field at byte OFF: FP64 pairs, TD pairs, real TD.
+// Element (level, column) of the FP64 pair field at byte OFF; (row offset, column) of a
+// field of TD pairs or real TD.
 template <int OFF> __device__ __forceinline__ double2 &zs_at(unsigned char *sm, int l, int c) {
     return *reinterpret_cast<double2 *>(sm + OFF + l * kZsRow + c * 16);
 }
 template <int OFF, typename TD>
-__device__ __forceinline__ C2<TD> zs_pair(unsigned char *sm, int l, int c) {
-    return *reinterpret_cast<const C2<TD> *>(sm + OFF + l * zs_row_td<TD>() +
-                                             c * (int)sizeof(C2<TD>));
+__device__ __forceinline__ C2<TD> zs_pair(unsigned char *sm, int row, int c) {
+    return *reinterpret_cast<const C2<TD> *>(sm + OFF + row + c * (int)sizeof(C2<TD>));
 }
 template <int OFF, typename TD>
-__device__ __forceinline__ double zs_real(unsigned char *sm, int l, int c) {
-    return double(*reinterpret_cast<const TD *>(sm + OFF + l * zs_row_r<TD>() + c * (int)sizeof(TD)));
+__device__ __forceinline__ double zs_real(unsigned char *sm, int row, int c) {
+    return double(*reinterpret_cast<const TD *>(sm + OFF + row + c * (int)sizeof(TD)));
 }
 
 // The operators as A fragments (the context's tables, one value a lane and
@@ -302,48 +305,48 @@ __global__ void __launch_bounds__(kZsThreads, ZsDims<NZP>::min_blocks)
     const unsigned sb = (unsigned)__cvta_generic_to_shared(sm);
     const unsigned barM = sb + Lay::oBAR, barZ = barM + 8;
     double *tab = reinterpret_cast<double *>(sm + Lay::oTAB);
+    int *rowr = reinterpret_cast<int *>(sm + Lay::oROW);
+    const ZsSplit spair(nz, P * (long long)sizeof(PD), zs_row_td<TD>());
+    const ZsSplit sreal(nz, P * (long long)sizeof(TD), zs_row_r<TD>());
+    const int odd = spair.n > 1 ? spair.start(1) + spair.shift(1) : 0;
+    // row of level i in a field of TD pairs
+    auto rowp = [&](int i) {
+        return sizeof(TD) == 8 ? i * kZsRow
+                               : (i >> spair.lg) * zs_row_td<TD>() + (i & spair.lg) * odd;
+    };
     const bool leader = threadIdx.x == 0;  // issues the copies
     // z, f = 1 - z^3, Lz(nz,:) and the line's factors; V rows past nz are zero in every product
     for (int i = threadIdx.x; i < D::ntab; i += kZsThreads) tab[i] = __ldg(a.ztab + i);
+    for (int i = threadIdx.x; i < nz; i += kZsThreads) rowr[i] = sreal.at(i);
     for (int i = threadIdx.x; i < 2 * Lay::rv / 16; i += kZsThreads)
         reinterpret_cast<double2 *>(sm + Lay::oVA)[i] = make_double2(0.0, 0.0);
     if (threadIdx.x == 0) {
-        // arrivals of a phase: the leader's expected bytes, and every thread where
-        // fields of the group come by cp.async
-        zs_bar_init(barM, 1 + (a.copy_pairs || a.copy_real ? kZsThreads : 0));
+        zs_bar_init(barM, 1);  // the leader's expected bytes
         zs_bar_init(barZ, 1);
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     }
     __syncthreads();
     pdl_wait();
 
-    // byte counts of the groups by TMA
-    const int bc = nz * kZsRow, bp = a.copy_pairs ? 0 : nz * zs_row_td<TD>();
-    const int br = a.copy_real ? 0 : nz * zs_row_r<TD>();
-    auto load_pair = [&](int off, const CUtensorMap &map, const PD *src, long long s0,
-                         unsigned bar) {
-        if (a.copy_pairs)
-            zs_copy<PD, zs_row_td<TD>()>(sm + off, src, nz, P, s0);
-        else if (leader)
-            zs_tma(sb + off, &map, (int)(2 * s0), bar);
+    // main inputs; state and accumulator.  All by the leader.
+    const int bc = nz * kZsRow;
+    auto load_split = [&](int off, const CUtensorMap *map, const ZsSplit &sp, int x) {
+        for (int ph = 0; ph < sp.n && ph < nz; ++ph) zs_tma(sb + off + sp.start(ph), map + ph, x, barM);
     };
-    // main inputs; state and accumulator
     auto load_M = [&](long long s0) {
-        if (leader) {
-            zs_expect(barM, 3 * bc + 6 * bp + br);
-            zs_tma(sb + Lay::oPS, &a.mPS, (int)(2 * s0), barM);
-            zs_tma(sb + Lay::oAXY, &a.mAXY, (int)(2 * s0), barM);
-            zs_tma(sb + Lay::oATD, &a.mATD, (int)(2 * s0), barM);
-            if (!a.copy_real) zs_tma(sb + Lay::oDIV, &a.mDIV, (int)s0, barM);
-        }
-        load_pair(Lay::oDX, a.mDX, a.dxpsi, s0, barM);
-        load_pair(Lay::oDY, a.mDY, a.dypsi, s0, barM);
-        load_pair(Lay::oDT, a.mDT, a.dAt, s0, barM);
-        load_pair(Lay::oB, a.mB, a.B, s0, barM);
-        load_pair(Lay::oXX, a.mXX, a.dxxpsi, s0, barM);
-        load_pair(Lay::oYY, a.mYY, a.dyypsi, s0, barM);
-        if (a.copy_real) zs_copy<TD, zs_row_r<TD>()>(sm + Lay::oDIV, a.divA, nz, P, s0);
-        if (a.copy_pairs || a.copy_real) zs_copy_arrive(barM);
+        if (!leader) return;
+        const int x = (int)(2 * s0);
+        zs_expect(barM, 3 * bc + nz * (6 * zs_row_td<TD>() + zs_row_r<TD>()));
+        zs_tma(sb + Lay::oPS, &a.mPS, x, barM);
+        zs_tma(sb + Lay::oAXY, &a.mAXY, x, barM);
+        zs_tma(sb + Lay::oATD, &a.mATD, x, barM);
+        load_split(Lay::oDX, a.mDX, spair, x);
+        load_split(Lay::oDY, a.mDY, spair, x);
+        load_split(Lay::oDT, a.mDT, spair, x);
+        load_split(Lay::oB, a.mB, spair, x);
+        load_split(Lay::oXX, a.mXX, spair, x);
+        load_split(Lay::oYY, a.mYY, spair, x);
+        load_split(Lay::oDIV, a.mDIV, sreal, (int)s0);
     };
     auto load_Z = [&](long long s0) {
         if (kK && leader) {
@@ -393,7 +396,7 @@ __global__ void __launch_bounds__(kZsThreads, ZsDims<NZP>::min_blocks)
                     [&](int j) { return ops.template operand<Lay::oPS>(sm, j); }, tab + 3 * NZP,
                     yA, yB, dA, dB);
             auto put = [&](int i, const double (&y)[2], const double (&d)[2]) {
-                const PD dt = zs_pair<Lay::oDT, TD>(sm, i, col);
+                const PD dt = zs_pair<Lay::oDT, TD>(sm, rowp(i), col);
                 const double f = tab[NZP + i];
                 zs_at<Lay::oVA>(sm, i, col) =
                     make_double2(double(dt.x) + f * y[0], double(dt.y) + f * y[1]);
@@ -420,12 +423,13 @@ __global__ void __launch_bounds__(kZsThreads, ZsDims<NZP>::min_blocks)
             auto put = [&](int i, const double (&y)[2], const double (&d1)[2],
                            const double (&d2)[2]) {
                 const double2 ps = zs_at<Lay::oPS>(sm, i, col), av = zs_at<Lay::oAXY>(sm, i, col);
-                const PD dx = zs_pair<Lay::oDX, TD>(sm, i, col), dy = zs_pair<Lay::oDY, TD>(sm, i, col);
+                const int rp = rowp(i);
+                const PD dx = zs_pair<Lay::oDX, TD>(sm, rp, col), dy = zs_pair<Lay::oDY, TD>(sm, rp, col);
                 const double dxr = double(dx.x), dxi = double(dx.y), dyr = double(dy.x),
                              dyi = double(dy.y);
                 const bool in = i < n1;
                 {  // S = 1/2 Lz g -+ 1/2 d B + Im(conj(Psi) d Psi) - A |Psi|^2
-                    const PD bf = zs_pair<Lay::oB, TD>(sm, i, col);
+                    const PD bf = zs_pair<Lay::oB, TD>(sm, rp, col);
                     const double p2 = ps.x * ps.x + ps.y * ps.y;
                     const double vx = 0.5 * y[0] + 0.5 * -double(bf.x) +
                                       (ps.x * dxi - ps.y * dxr) - av.x * p2;
@@ -434,9 +438,9 @@ __global__ void __launch_bounds__(kZsThreads, ZsDims<NZP>::min_blocks)
                     zs_at<Lay::oVA>(sm, i, col) = make_double2(in ? vx : 0.0, in ? vy : 0.0);
                 }
                 const double2 atd = zs_at<Lay::oATD>(sm, i, col);
-                const PD lxx = zs_pair<Lay::oXX, TD>(sm, i, col), lyy = zs_pair<Lay::oYY, TD>(sm, i, col);
+                const PD lxx = zs_pair<Lay::oXX, TD>(sm, rp, col), lyy = zs_pair<Lay::oYY, TD>(sm, rp, col);
                 const double lpx = double(lxx.x) + double(lyy.x), lpy = double(lxx.y) + double(lyy.y);
-                const double dv = zs_real<Lay::oDIV, TD>(sm, i, col);
+                const double dv = zs_real<Lay::oDIV, TD>(sm, rowr[i], col);
                 kb = fma(tab[2 * NZP + i], dv, kb);
                 const double z = tab[i], f = tab[NZP + i], hh = 0.5;
                 const double a2 = av.x * av.x + av.y * av.y;
