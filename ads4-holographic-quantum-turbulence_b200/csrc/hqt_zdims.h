@@ -55,14 +55,9 @@ template <int NZP> struct ZsDims {
     static constexpr int VR = NZP > 4 * K1 ? NZP : 4 * K1;  // rows of a scratch field
     static constexpr int nfrag = MP * KE + MH * KO + M1 * K1;
     // state and accumulator are read straight from global memory instead of staged
-#ifndef HQT_ZDIR
-#define HQT_ZDIR (NZP > 25)
-#endif
-#ifndef HQT_ZMB
-#define HQT_ZMB 2
-#endif
-    static constexpr bool direct = HQT_ZDIR;
-    static constexpr int min_blocks = HQT_ZMB;
+    // where staging them would leave one block per SM
+    static constexpr bool direct = NZP > 25;
+    static constexpr int min_blocks = 2;
 };
 
 }  // namespace hqt

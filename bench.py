@@ -68,12 +68,12 @@ ALG_BYTES = {"x_rhs": 88, "y_rhs": 112, "zstage": 264, "x_d1": 16, "y_d1": 20,
 # compulsory traffic of a whole FP64 step per site: 4*(S_in + S_k) + 2*S_state
 STEP_BYTES_FP64 = 4 * (40 + 32) + 2 * 40
 # FP64 tensor-core work of the prime-factor line passes (n = 301 = 7*43): one
-# 43-point stage A is 144 mma.sync.m8n8k4.f64 per two lines (2 passes x 6
-# reduction steps x 2 operand tiles x 3 row tiles x cos/sin), 512 flops each;
+# 43-point stage A is 80 mma.sync.m8n8k4.f64 per two lines (2 passes x 2
+# operand tiles x 10 x cos/sin), 512 flops each;
 # x_rhs runs 6 stage A per line pair, y_rhs 7.  The peak is the mma.sync f64
 # throughput measured on B200 at 1965 MHz (37.1 TFLOP/s for the m8n8k4,
 # m16n8k4 and m16n8k16 shapes alike).
-PFA_DMMA_PER_LINE = {"x_rhs": 6 * 144 / 2, "y_rhs": 7 * 144 / 2}
+PFA_DMMA_PER_LINE = {"x_rhs": 6 * 80 / 2, "y_rhs": 7 * 80 / 2}
 FP64_TENSOR_TFLOPS = 37.1
 
 
