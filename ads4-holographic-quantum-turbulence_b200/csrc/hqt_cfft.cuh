@@ -260,10 +260,11 @@ __device__ __forceinline__ void ct_big(int src, int dst, int roots, int sign) {
     }
 }
 
-template <typename T, int N, int NB, int P>
+// passes P .. E-1 of the plan, a barrier after each
+template <typename T, int N, int NB, int P, int E>
 __device__ __forceinline__ int ct_fft_from(int src, int dst, int roots, int sign) {
     constexpr CtPlan pl = ct_plan(N, kCtMaxBits);
-    if constexpr (P >= pl.np) {
+    if constexpr (P >= E) {
         return src;
     } else {
         constexpr int R = pl.R[P];
@@ -273,7 +274,7 @@ __device__ __forceinline__ int ct_fft_from(int src, int dst, int roots, int sign
         else
             ct_big<T, N, NB, R, Ns>(src, dst, roots, sign);
         __syncthreads();
-        return ct_fft_from<T, N, NB, P + 1>(dst, src, roots, sign);
+        return ct_fft_from<T, N, NB, P + 1, E>(dst, src, roots, sign);
     }
 }
 
@@ -283,12 +284,145 @@ __device__ __forceinline__ int ct_fft_from(int src, int dst, int roots, int sign
 // (2016 FMAs at N = 301) overflowed the instruction cache.
 template <typename T, int N, int NB>
 __device__ __noinline__ int ct_fft_rt(int a, int b, int roots, int sign) {
-    return ct_fft_from<T, N, NB, 0>(a, b, roots, sign);
+    return ct_fft_from<T, N, NB, 0, ct_plan(N, kCtMaxBits).np>(a, b, roots, sign);
 }
 template <typename T, int N, int NB, int SIGN>
 __device__ __forceinline__ int ct_fft(int a, int b, int roots) {
     return ct_fft_rt<T, N, NB>(a, b, roots, SIGN);
 }
+
+// ---- plans of small radices: the ends of a transform fused -------------------
+// The first pass takes its elements from ld(e, b), the last hands its results to
+// st(e, b, v), so that lines come from and go to global memory through registers and
+// a derivative's multiplier needs no pass of its own: 22 trips of a line through
+// shared memory for a field's two derivatives instead of 31, half the barriers.  The
+// operations and their order are those of the passes through shared memory.
+// Measured, us a launch before -> after (FP32): 1024x1024x33 x_rhs 1061 -> 957, y_rhs
+// 1921 -> 1565; 512x512x25 y_rhs 295 -> 264, 256x256x25 74 -> 58, 64x64x21 14.8 ->
+// 12.7.  Bound now: the trips that are left (the in-place form of hqt_line.cuh makes
+// 18, but rounds differently).
+__host__ __device__ constexpr int ct_np(int n) { return ct_plan(n, kCtMaxBits).np; }
+__host__ __device__ constexpr bool ct_fused(int n) {
+    const CtPlan p = ct_plan(n, kCtMaxBits);
+    for (int i = 0; i < p.np; ++i)
+        if (!ct_small_radix(p.R[i])) return false;
+    return p.np >= 2;
+}
+template <typename T> struct CtRegs {
+    C2<T> *v;
+    __device__ __forceinline__ C2<T> &operator[](int i) const { return v[i]; }
+};
+template <typename T, int N, int NB, int P> struct CtPass {
+    static constexpr int R = ct_plan(N, kCtMaxBits).R[P], Ns = ct_plan(N, kCtMaxBits).Ns[P];
+    // st(e0, b, out): out[k] is element e0 + k Ns
+    template <typename Ld, typename St>
+    static __device__ __forceinline__ void run(int roots, int sign, Ld ld, St st) {
+        const CtView<T, N> W = ctv<T, N>(roots);
+        constexpr int nR = N / R, qs = N / (Ns * R);
+        for (int t = threadIdx.x; t < NB * nR; t += ct_threads<T, N, NB>()) {
+            const int b = t % NB, j = t / NB, m = (Ns == 1) ? 0 : j % Ns;
+            C2<T> v[R], out[R];
+#pragma unroll
+            for (int r = 0; r < R; ++r) v[r] = ld(j + r * nR, b);
+            if (Ns > 1 && m > 0) {
+                const int step = m * qs;
+#pragma unroll
+                for (int r = 1; r < R; ++r) {
+                    C2<T> w = W[r * step];
+                    if (sign > 0) w.y = -w.y;
+                    v[r] = cmul(v[r], w);
+                }
+            }
+            dft_store<T, R>(v, CtRegs<T>{out}, 0, 1, sign);
+            st((j - m) * R + m, b, out);
+        }
+    }
+};
+// passes P .. E-1 through shared memory; returns the result's buffer
+template <typename T, int N, int NB, int P, int E>
+__device__ __noinline__ int ct_mid(int a, int b, int roots, int sign) {
+    return ct_fft_from<T, N, NB, P, E>(a, b, roots, sign);
+}
+template <typename T, int N, int NB> struct CtLine {
+    static constexpr int np = ct_np(N);
+    using First = CtPass<T, N, NB, 0>;
+    using Last = CtPass<T, N, NB, np - 1>;
+    int roots;
+    static __device__ __forceinline__ T wave(int e) {
+        return T(2 * e < N ? e : (2 * e > N ? e - N : 0));
+    }
+    // all forward passes but the last, from ld, starting in buffer a (free to write);
+    // b is written from the second pass on
+    template <typename Ld> __device__ __forceinline__ int forward(int a, int b, Ld ld) const {
+        const CtView<T, N> D = ctv<T, N>(a);
+        First::run(roots, -1, ld, [&](int e0, int l, C2<T>(&v)[First::R]) {
+#pragma unroll
+            for (int k = 0; k < First::R; ++k) D[(e0 + k * First::Ns) * NB + l] = v[k];
+        });
+        __syncthreads();
+        return ct_mid<T, N, NB, 1, np - 1>(a, b, roots, -1);
+    }
+    // last forward pass of src: the spectrum, its first derivative, or both
+    // derivatives, into other buffers.  A barrier has to follow.
+    __device__ __forceinline__ void spectrum(int src, int dst) const {
+        const CtView<T, N> S = ctv<T, N>(src), D = ctv<T, N>(dst);
+        Last::run(
+            roots, -1, [&](int e, int l) { return S[e * NB + l]; },
+            [&](int e0, int l, C2<T>(&v)[Last::R]) {
+#pragma unroll
+                for (int k = 0; k < Last::R; ++k) D[(e0 + k * Last::Ns) * NB + l] = v[k];
+            });
+    }
+    __device__ __forceinline__ void deriv1(int src, int dst, T s1) const {
+        const CtView<T, N> S = ctv<T, N>(src), D = ctv<T, N>(dst);
+        Last::run(
+            roots, -1, [&](int e, int l) { return S[e * NB + l]; },
+            [&](int e0, int l, C2<T>(&v)[Last::R]) {
+#pragma unroll
+                for (int k = 0; k < Last::R; ++k) {
+                    const int e = e0 + k * Last::Ns;
+                    const T m = s1 * wave(e);
+                    D[e * NB + l] = mk2<T>(-m * v[k].y, m * v[k].x);
+                }
+            });
+    }
+    __device__ __forceinline__ void deriv12(int src, int dst1, int dst2, T s1, T s2) const {
+        const CtView<T, N> S = ctv<T, N>(src), D = ctv<T, N>(dst1), E = ctv<T, N>(dst2);
+        Last::run(
+            roots, -1, [&](int e, int l) { return S[e * NB + l]; },
+            [&](int e0, int l, C2<T>(&v)[Last::R]) {
+#pragma unroll
+                for (int k = 0; k < Last::R; ++k) {
+                    const int e = e0 + k * Last::Ns;
+                    const T kk = wave(e), m = s1 * kk, m2 = s2 * kk * kk;
+                    D[e * NB + l] = mk2<T>(-m * v[k].y, m * v[k].x);
+                    E[e * NB + l] = mk2<T>(m2 * v[k].x, m2 * v[k].y);
+                }
+            });
+    }
+    // all inverse passes but the last; from buffer a, b free to write
+    __device__ __forceinline__ int inverse(int a, int b) const {
+        return ct_mid<T, N, NB, 0, np - 1>(a, b, roots, +1);
+    }
+    // the last inverse pass of src: put(e, b, v, x) with x = get(e, b), read for all
+    // of a butterfly's elements ahead of the writes
+    template <typename Get, typename Put>
+    __device__ __forceinline__ void last(int src, Get get, Put put) const {
+        const CtView<T, N> S = ctv<T, N>(src);
+        Last::run(
+            roots, +1, [&](int e, int l) { return S[e * NB + l]; },
+            [&](int e0, int l, C2<T>(&v)[Last::R]) { out(e0, l, v, get, put); });
+    }
+    template <typename Get, typename Put>
+    static __device__ __forceinline__ void out(int e0, int l, C2<T> (&v)[Last::R], Get get,
+                                               Put put) {
+        decltype(get(0, 0)) x[Last::R];
+#pragma unroll
+        for (int k = 0; k < Last::R; ++k) x[k] = get(e0 + k * Last::Ns, l);
+#pragma unroll
+        for (int k = 0; k < Last::R; ++k) put(e0 + k * Last::Ns, l, v[k], x[k]);
+    }
+};
 
 // dst = m(k) src over the batch (order 1: i*s1*k, order 2: s2*k^2)
 template <typename T, int N, int NB, int ORDER>

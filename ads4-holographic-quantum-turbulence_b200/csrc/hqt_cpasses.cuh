@@ -111,6 +111,35 @@ __global__ void HQT_CT_BOUNDS k_x_rhs_c(XRhsArgs<T> a) {
     const long long g0 = (long long)L0 * N;
     ct_load_roots<T, N>(R, a.roots);
     pdl_wait();
+    if constexpr (ct_fused(N) && NB == 1) {
+        __syncthreads();  // the twiddles are in
+        const CtLine<T, N, NB> w{R};
+        int p = A, q = B, r = C;
+#pragma unroll 1
+        for (int f = 0; f < 2; ++f) {
+            const C2<T> *in = f == 0 ? a.psi : a.A;
+            C2<T> *d1 = f == 0 ? a.dxpsi : a.E;
+            const int s = w.forward(p, q, [&](int e, int) { return in[g0 + e]; });
+            const int o = s == p ? q : p;
+            w.deriv12(s, o, r, a.s1, a.s2);
+            __syncthreads();
+            const int u = w.inverse(o, s), v = u == o ? s : o;
+            w.last(u, [](int, int) { return 0; },
+                   [&](int e, int, C2<T> x, int) { d1[g0 + e] = x; });
+            const int y = w.inverse(r, v);
+            w.last(y, [](int, int) { return 0; }, [&](int e, int, C2<T> x, int) {
+                if (f == 0)
+                    a.dxxpsi[g0 + e] = x;
+                else
+                    a.dxxay[g0 + e] = x.y;
+            });
+            // u is free (read before a barrier), y is being read
+            q = y == r ? v : r;
+            r = y;
+            p = u;
+        }
+        return;
+    }
     cx_load<T, N, NB>(A, valid, [&](int t) { return a.psi[g0 + t]; });
     __syncthreads();
     const int X = ct_fft<T, N, NB, -1>(A, B, R);
@@ -143,6 +172,38 @@ __global__ void HQT_CT_BOUNDS k_x_rhs_c(XRhsArgs<T> a) {
     cx_store<T, N, NB>(r4, valid, [&](int t, C2<T> v) { a.dxxay[g0 + t] = v.y; });
 }
 
+// spectra of C = A_x + i A_y (SC) and E = d_x C (SE) -> those of (div A, d_x B) less
+// their x parts, and of d_y B, in place
+template <typename T, int N, int NB>
+__device__ __forceinline__ void cy_pair(int SC, int SE, T s1, T s2) {
+    const CtView<T, N> sc = ctv<T, N>(SC), se = ctv<T, N>(SE);
+    const T h = T(0.5);
+    for (int t = threadIdx.x; t < (N / 2 + 1) * NB; t += ct_threads<T, N, NB>()) {
+        const int b = t % NB, k = t / NB;
+        const int kp = (N - k) % N;
+        const C2<T> Cc = sc[k * NB + b], Cp = sc[kp * NB + b];
+        const C2<T> Ec = se[k * NB + b], Ep = se[kp * NB + b];
+#pragma unroll
+        for (int side = 0; side < 2; ++side) {
+            if (side == 1 && kp == k) break;
+            const int kk_ = side == 0 ? k : kp;
+            const C2<T> c1 = side == 0 ? Cc : Cp, c2 = side == 0 ? Cp : Cc;
+            const C2<T> e1 = side == 0 ? Ec : Ep, e2 = side == 0 ? Ep : Ec;
+            const T kk = T(wavenum(kk_, N));
+            const T m1 = s1 * kk, m2 = s2 * kk * kk;
+            const C2<T> axh = mk2<T>(h * (c1.x + c2.x), h * (c1.y - c2.y));
+            const C2<T> ayh = mk2<T>(h * (c1.y + c2.y), -h * (c1.x - c2.x));
+            const C2<T> exh = mk2<T>(h * (e1.x + e2.x), h * (e1.y - e2.y));
+            const C2<T> eyh = mk2<T>(h * (e1.y + e2.y), -h * (e1.x - e2.x));
+            const C2<T> q1 = mk2<T>(-m1 * ayh.y, m1 * ayh.x);
+            const C2<T> q2 = mk2<T>(m1 * exh.y, -m1 * exh.x);
+            const C2<T> q3 = mk2<T>(-m1 * eyh.y - m2 * axh.x, m1 * eyh.x - m2 * axh.y);
+            sc[kk_ * NB + b] = mk2<T>(q1.x - q2.y, q1.y + q2.x);
+            se[kk_ * NB + b] = q3;
+        }
+    }
+}
+
 template <typename T, int N>
 __global__ void HQT_CT_BOUNDS k_y_rhs_c(YRhsArgs<T> a) {
     constexpr int NB = ct_lines_y(N, 3, sizeof(C2<T>));
@@ -152,6 +213,56 @@ __global__ void HQT_CT_BOUNDS k_y_rhs_c(YRhsArgs<T> a) {
     constexpr int R = 0, A = N, B = N + NB * N, C = N + 2 * NB * N;
     ct_load_roots<T, N>(R, a.roots);
     pdl_wait();
+    if constexpr (ct_fused(N)) {
+        __syncthreads();  // the twiddles are in
+        const CtLine<T, N, NB> w{R};
+        auto at = [&](int e, int l) { return zoff + (long long)e * a.nx + l; };
+        auto none = [](int, int) { return 0; };
+        const C2<T> zero = mk2<T>(T(0), T(0));
+        int s = w.forward(A, B, [&](int e, int l) { return l < valid ? a.psi[at(e, l)] : zero; });
+        int o = s == A ? B : A;
+        w.deriv12(s, o, C, a.s1, a.s2);
+        __syncthreads();
+        int u = w.inverse(o, s), v = u == o ? s : o;
+        w.last(u, none, [&](int e, int l, C2<T> x, int) {
+            if (l < valid) a.dypsi[at(e, l)] = x;
+        });
+        const int y = w.inverse(C, v), z = y == C ? v : C;
+        w.last(y, none, [&](int e, int l, C2<T> x, int) {
+            if (l < valid) a.dyypsi[at(e, l)] = x;
+        });
+        // u and z are free, y from the next barrier on
+        s = w.forward(u, z, [&](int e, int l) { return l < valid ? a.A[at(e, l)] : zero; });
+        const int SC = y;
+        w.spectrum(s, SC);
+        o = s == u ? z : u;
+        s = w.forward(o, s, [&](int e, int l) { return l < valid ? a.E[at(e, l)] : zero; });
+        const int SE = s == u ? z : u;
+        w.spectrum(s, SE);
+        __syncthreads();
+        cy_pair<T, N, NB>(SC, SE, a.s1, a.s2);
+        __syncthreads();
+        u = w.inverse(SC, s);
+        v = u == SC ? s : SC;
+        w.last(
+            u,
+            [&](int e, int l) {
+                if (l >= valid) return zero;
+                const long long g = at(e, l);
+                return mk2<T>(a.E[g].x, a.dxxay[g]);
+            },
+            [&](int e, int l, C2<T> q, C2<T> x) {
+                if (l >= valid) return;
+                const long long g = at(e, l);
+                a.divA[g] = x.x + q.x;
+                a.B[g].y = x.y + q.y;
+            });
+        const int t = w.inverse(SE, v);
+        w.last(t, none, [&](int e, int l, C2<T> q, int) {
+            if (l < valid) a.B[at(e, l)].x = q.x;
+        });
+        return;
+    }
     // Psi: d_y and d_yy
     cy_load<T, N, NB>(A, valid, a.nx, zoff, [&](long long g) { return a.psi[g]; });
     __syncthreads();
@@ -181,34 +292,7 @@ __global__ void HQT_CT_BOUNDS k_y_rhs_c(YRhsArgs<T> a) {
     cp_wait<0>();
     __syncthreads();  // E is in
     const int SE = ct_fft<T, N, NB, -1>(fr, F1, R);     // E spectrum in fr or F1
-    {
-        const CtView<T, N> sc = ctv<T, N>(SC), se = ctv<T, N>(SE);
-        const T h = T(0.5);
-        for (int t = threadIdx.x; t < (N / 2 + 1) * NB; t += ct_threads<T, N, NB>()) {
-            const int b = t % NB, k = t / NB;
-            const int kp = (N - k) % N;
-            const C2<T> Cc = sc[k * NB + b], Cp = sc[kp * NB + b];
-            const C2<T> Ec = se[k * NB + b], Ep = se[kp * NB + b];
-#pragma unroll
-            for (int side = 0; side < 2; ++side) {
-                if (side == 1 && kp == k) break;
-                const int kk_ = side == 0 ? k : kp;
-                const C2<T> c1 = side == 0 ? Cc : Cp, c2 = side == 0 ? Cp : Cc;
-                const C2<T> e1 = side == 0 ? Ec : Ep, e2 = side == 0 ? Ep : Ec;
-                const T kk = T(wavenum(kk_, N));
-                const T m1 = a.s1 * kk, m2 = a.s2 * kk * kk;
-                const C2<T> axh = mk2<T>(h * (c1.x + c2.x), h * (c1.y - c2.y));
-                const C2<T> ayh = mk2<T>(h * (c1.y + c2.y), -h * (c1.x - c2.x));
-                const C2<T> exh = mk2<T>(h * (e1.x + e2.x), h * (e1.y - e2.y));
-                const C2<T> eyh = mk2<T>(h * (e1.y + e2.y), -h * (e1.x - e2.x));
-                const C2<T> q1 = mk2<T>(-m1 * ayh.y, m1 * ayh.x);
-                const C2<T> q2 = mk2<T>(m1 * exh.y, -m1 * exh.x);
-                const C2<T> q3 = mk2<T>(-m1 * eyh.y - m2 * axh.x, m1 * eyh.x - m2 * axh.y);
-                sc[kk_ * NB + b] = mk2<T>(q1.x - q2.y, q1.y + q2.x);
-                se[kk_ * NB + b] = q3;
-            }
-        }
-    }
+    cy_pair<T, N, NB>(SC, SE, a.s1, a.s2);
     __syncthreads();
     // the third buffer is free: the one that is neither SC nor SE
     const int F2 = (A != SC && A != SE) ? A : ((B != SC && B != SE) ? B : C);
@@ -254,6 +338,25 @@ __global__ void HQT_CT_BOUNDS k_y_d1_c(YD1Args<T> a) {
     constexpr int R = 0, A = N, B = N + NB * N;
     ct_load_roots<T, N>(R, a.roots);
     pdl_wait();
+    if constexpr (ct_fused(N)) {
+        __syncthreads();  // the twiddles are in
+        const CtLine<T, N, NB> w{R};
+        auto at = [&](int e, int l) { return zoff + (long long)e * a.nx + l; };
+        const int s = w.forward(A, B, [&](int e, int l) {
+            return l < valid ? load_field(a.in, at(e, l)) : mk2<T>(T(0), T(0));
+        });
+        const int o = s == A ? B : A;
+        w.deriv1(s, o, a.s1);
+        __syncthreads();
+        w.last(
+            w.inverse(o, s),
+            [&](int e, int l) { return a.add_re && l < valid ? a.add_re[at(e, l)] : T(0); },
+            [&](int e, int l, C2<T> v, T x) {
+                if (a.add_re) v.x += x;
+                if (l < valid) store_field(a.out, at(e, l), v);
+            });
+        return;
+    }
     cy_load<T, N, NB>(A, valid, a.nx, zoff, [&](long long g) { return load_field(a.in, g); });
     __syncthreads();
     const int X = ct_fft<T, N, NB, -1>(A, B, R);
@@ -315,6 +418,27 @@ __global__ void HQT_CT_BOUNDS k_y_d1r_c(YD1Args<T> a) {
     constexpr int R = 0, A = N, B = N + NB * N;
     ct_load_roots<T, N>(R, a.roots);
     pdl_wait();
+    if constexpr (ct_fused(N)) {
+        __syncthreads();  // the twiddles are in
+        const CtLine<T, N, NB> w{R};
+        auto pair = [&](const T *p, int e, int j) {
+            const T *q = p + zoff + (long long)e * a.nx + 2 * j;
+            return mk2<T>(2 * j < nr ? q[0] : T(0), 2 * j + 1 < nr ? q[1] : T(0));
+        };
+        const int s = w.forward(A, B, [&](int e, int j) { return pair(a.in.re, e, j); });
+        const int o = s == A ? B : A;
+        w.deriv1(s, o, a.s1);
+        __syncthreads();
+        w.last(
+            w.inverse(o, s),
+            [&](int e, int j) { return a.add_re ? pair(a.add_re, e, j) : mk2<T>(T(0), T(0)); },
+            [&](int e, int j, C2<T> v, C2<T> x) {
+                const long long g = zoff + (long long)e * a.nx + 2 * j;
+                if (2 * j < nr) a.out.re[g * a.out.st] = v.x + x.x;
+                if (2 * j + 1 < nr) a.out.re[(g + 1) * a.out.st] = v.y + x.y;
+            });
+        return;
+    }
     {  // the layout of cy_load: element (y, j) at y*NB + j
         const CtView<T, N> sa = ctv<T, N>(A);
         for (int t = threadIdx.x; t < N * NB; t += ct_threads<T, N, NB>()) {
