@@ -298,8 +298,8 @@ __device__ __forceinline__ int ct_fft(int a, int b, int roots) {
 // shared memory for a field's two derivatives instead of 31, half the barriers.  The
 // operations and their order are those of the passes through shared memory.
 // Measured, us a launch before -> after (FP32): 1024x1024x33 x_rhs 1061 -> 957, y_rhs
-// 1921 -> 1565; 512x512x25 y_rhs 295 -> 264, 256x256x25 74 -> 58, 64x64x21 14.8 ->
-// 12.7.  Bound now: the trips that are left (the in-place form of hqt_line.cuh makes
+// 1921 -> 1565; 512x512x25 204 -> 168, 295 -> 264; 256x256x25 65 -> 52, 74 -> 58;
+// 64x64x21 14.8 -> 11.8, 14.8 -> 12.7.  Bound now: the trips that are left (the in-place form of hqt_line.cuh makes
 // 18, but rounds differently).
 __host__ __device__ constexpr int ct_np(int n) { return ct_plan(n, kCtMaxBits).np; }
 __host__ __device__ constexpr bool ct_fused(int n) {

@@ -111,28 +111,50 @@ __global__ void HQT_CT_BOUNDS k_x_rhs_c(XRhsArgs<T> a) {
     const long long g0 = (long long)L0 * N;
     ct_load_roots<T, N>(R, a.roots);
     pdl_wait();
-    if constexpr (ct_fused(N) && NB == 1) {
+    if constexpr (ct_fused(N)) {
         __syncthreads();  // the twiddles are in
         const CtLine<T, N, NB> w{R};
+        constexpr int np = ct_np(N);
         int p = A, q = B, r = C;
 #pragma unroll 1
         for (int f = 0; f < 2; ++f) {
             const C2<T> *in = f == 0 ? a.psi : a.A;
             C2<T> *d1 = f == 0 ? a.dxpsi : a.E;
-            const int s = w.forward(p, q, [&](int e, int) { return in[g0 + e]; });
+            auto put2 = [&](long long g, C2<T> x) {
+                if (f == 0)
+                    a.dxxpsi[g] = x;
+                else
+                    a.dxxay[g] = x.y;
+            };
+            int s;
+            if constexpr (NB == 1) {
+                s = w.forward(p, q, [&](int e, int) { return in[g0 + e]; });
+            } else {  // several lines: lanes run over them, global memory along them
+                cx_load<T, N, NB>(p, valid, [&](int t) { return in[g0 + t]; });
+                __syncthreads();
+                s = ct_mid<T, N, NB, 0, np - 1>(p, q, R, -1);
+            }
             const int o = s == p ? q : p;
             w.deriv12(s, o, r, a.s1, a.s2);
             __syncthreads();
-            const int u = w.inverse(o, s), v = u == o ? s : o;
-            w.last(u, [](int, int) { return 0; },
-                   [&](int e, int, C2<T> x, int) { d1[g0 + e] = x; });
-            const int y = w.inverse(r, v);
-            w.last(y, [](int, int) { return 0; }, [&](int e, int, C2<T> x, int) {
-                if (f == 0)
-                    a.dxxpsi[g0 + e] = x;
-                else
-                    a.dxxay[g0 + e] = x.y;
-            });
+            int u, y;
+            if constexpr (NB == 1) {
+                u = w.inverse(o, s);
+                w.last(u, [](int, int) { return 0; },
+                       [&](int e, int, C2<T> x, int) { d1[g0 + e] = x; });
+            } else {
+                u = ct_mid<T, N, NB, 0, np>(o, s, R, +1);
+                cx_store<T, N, NB>(u, valid, [&](int t, C2<T> x) { d1[g0 + t] = x; });
+            }
+            const int v = u == o ? s : o;
+            if constexpr (NB == 1) {
+                y = w.inverse(r, v);
+                w.last(y, [](int, int) { return 0; },
+                       [&](int e, int, C2<T> x, int) { put2(g0 + e, x); });
+            } else {
+                y = ct_mid<T, N, NB, 0, np>(r, v, R, +1);
+                cx_store<T, N, NB>(y, valid, [&](int t, C2<T> x) { put2(g0 + t, x); });
+            }
             // u is free (read before a barrier), y is being read
             q = y == r ? v : r;
             r = y;
