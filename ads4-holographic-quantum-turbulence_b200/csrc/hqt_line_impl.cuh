@@ -7,6 +7,8 @@
 namespace hqt {
 
 template <typename T, class GX, class GY> struct LineLaunch {
+    using OX = typename GX::One;  // of the passes with one buffer
+    using OY = typename GY::One;
     static cudaError_t opt(const void *fn, int max_smem, cudaError_t e) {
         cudaFuncAttributes fa{};
         if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, fn);
@@ -18,18 +20,18 @@ template <typename T, class GX, class GY> struct LineLaunch {
     static cudaError_t init_x(int max_smem) {
         cudaError_t e = cudaSuccess;
         e = opt((const void *)k_lx_rhs<T, GX>, max_smem, e);
-        e = opt((const void *)k_lx_d1<T, GX>, max_smem, e);
-        e = opt((const void *)k_lx_d1r<T, GX>, max_smem, e);
-        e = opt((const void *)k_lx_filt_fwd<T, GX>, max_smem, e);
-        return opt((const void *)k_lx_filt_inv<T, GX>, max_smem, e);
+        e = opt((const void *)k_lx_d1<T, OX>, max_smem, e);
+        e = opt((const void *)k_lx_d1r<T, OX>, max_smem, e);
+        e = opt((const void *)k_lx_filt_fwd<T, OX>, max_smem, e);
+        return opt((const void *)k_lx_filt_inv<T, OX>, max_smem, e);
     }
     static cudaError_t init_y(int max_smem) {
         cudaError_t e = cudaSuccess;
         e = opt((const void *)k_ly_rhs<T, GY>, max_smem, e);
-        e = opt((const void *)k_ly_d1<T, GY>, max_smem, e);
-        e = opt((const void *)k_ly_d1r<T, GY>, max_smem, e);
-        e = opt((const void *)k_ly_filt<T, GY>, max_smem, e);
-        return opt((const void *)k_ly_fwd<T, GY>, max_smem, e);
+        e = opt((const void *)k_ly_d1<T, OY>, max_smem, e);
+        e = opt((const void *)k_ly_d1r<T, OY>, max_smem, e);
+        e = opt((const void *)k_ly_filt<T, OY>, max_smem, e);
+        return opt((const void *)k_ly_fwd<T, OY>, max_smem, e);
     }
     // lines of a pass, in blocks of `per` complex lines of geometry g, nbuf
     // buffers each
@@ -51,16 +53,16 @@ template <typename T, class GX, class GY> struct LineLaunch {
             case CT_X_D1: {
                 const XD1Args<T> &a = *(const XD1Args<T> *)args;
                 if (real_field_d1(a.in, a.out))
-                    return go<GX>(k_lx_d1r<T, GX>, a, a.nlines, 1, 1, 1, 2, s);
-                return go<GX>(k_lx_d1<T, GX>, a, a.nlines, 1, 1, 1, 1, s);
+                    return go<OX>(k_lx_d1r<T, OX>, a, a.nlines, 1, 1, 1, 2, s);
+                return go<OX>(k_lx_d1<T, OX>, a, a.nlines, 1, 1, 1, 1, s);
             }
             case CT_FX_FWD: {
                 const XFiltFwdArgs<T> &a = *(const XFiltFwdArgs<T> *)args;
-                return go<GX>(k_lx_filt_fwd<T, GX>, a, a.nlines, 1, 1, 1, 1, s);
+                return go<OX>(k_lx_filt_fwd<T, OX>, a, a.nlines, 1, 1, 1, 1, s);
             }
             case CT_FX_INV: {
                 const XFiltInvArgs<T> &a = *(const XFiltInvArgs<T> *)args;
-                return go<GX>(k_lx_filt_inv<T, GX>, a, a.nlines, 1, 1, 1, 1, s);
+                return go<OX>(k_lx_filt_inv<T, OX>, a, a.nlines, 1, 1, 1, 1, s);
             }
         }
         return cudaErrorInvalidValue;
@@ -75,16 +77,16 @@ template <typename T, class GX, class GY> struct LineLaunch {
             case CT_Y_D1: {
                 const YD1Args<T> &a = *(const YD1Args<T> *)args;
                 if (real_field_d1(a.in, a.out))
-                    return go<GY>(k_ly_d1r<T, GY>, a, a.nx, nsl, 1, 1, 2, s);
-                return go<GY>(k_ly_d1<T, GY>, a, a.nx, nsl, 1, 1, 1, s);
+                    return go<OY>(k_ly_d1r<T, OY>, a, a.nx, nsl, 1, 1, 2, s);
+                return go<OY>(k_ly_d1<T, OY>, a, a.nx, nsl, 1, 1, 1, s);
             }
             case CT_FY: {
                 const YFiltArgs<T> &a = *(const YFiltArgs<T> *)args;
-                return go<GY>(k_ly_filt<T, GY>, a, a.nx, nsl, a.nf, 1, 1, s);
+                return go<OY>(k_ly_filt<T, OY>, a, a.nx, nsl, a.nf, 1, 1, s);
             }
             case CT_Y_FWD: {
                 const YFiltArgs<T> &a = *(const YFiltArgs<T> *)args;
-                return go<GY>(k_ly_fwd<T, GY>, a, a.nx, nsl, 1, 1, 1, s);
+                return go<OY>(k_ly_fwd<T, OY>, a, a.nx, nsl, 1, 1, 1, s);
             }
         }
         return cudaErrorInvalidValue;

@@ -112,9 +112,13 @@ inline int lthreads_rt(const LPlan &p, int nbl, int nbuf) {
 }
 
 // Compile-time geometry: N points, 2^NBL lines per block.
-template <int N_, int NBL_> struct SGeo;
+// The passes with one buffer (One) take blocks of at most 256 threads: with 512, a
+// block of 1024-point y lines was the only one on its SM (1024x1024x33: filter y 1247
+// -> 1060, y_d1 320 -> 300 us; 1024x1024x17: 647 -> 557, 223 -> 178 us).
+template <int N_, int NBL_, int MAXT = kLThreads> struct SGeo;
 // Runtime geometry, a kernel argument.
 struct RGeo {
+    using One = RGeo;
     static constexpr bool kStatic = false;
     static constexpr int kN = 0;
     static constexpr int kMaxThreads = kLThreads;
@@ -137,16 +141,18 @@ struct RGeo {
     __host__ __device__ __forceinline__ int tw(int p) const { return tw_[p]; }
     __host__ __device__ __forceinline__ unsigned mg(int p) const { return mg_[p]; }
 };
-template <int N_, int NBL_> struct SGeo {
+template <int N_, int NBL_, int MAXT> struct SGeo {
     static constexpr bool kStatic = true;
-    static constexpr int N = N_, kN = N_, NBL = NBL_, kMaxThreads = lthreads(N_, NBL_);
+    static constexpr int N = N_, kN = N_, NBL = NBL_;
+    static constexpr int kMaxThreads = lthreads(N_, NBL_) < MAXT ? lthreads(N_, NBL_) : MAXT;
+    using One = SGeo<N_, NBL_, 256>;
     static_assert(lplan(N_).np >= 2, "no in-place plan for this length");
     __host__ __device__ static constexpr int np() { return lplan(N_).np; }
     __host__ __device__ SGeo(const RGeo &) {}
     __host__ __device__ static constexpr int n() { return N_; }
     __host__ __device__ static constexpr int nbl() { return NBL_; }
-    static constexpr int block(int) { return lthreads(N_, NBL_); }
-    __host__ __device__ static constexpr int threads() { return lthreads(N_, NBL_); }
+    static constexpr int block(int) { return kMaxThreads; }
+    __host__ __device__ static constexpr int threads() { return kMaxThreads; }
     template <typename T, bool AX> __host__ __device__ static constexpr int swz() {
         return lswz(N_, NBL_, AX);
     }
