@@ -153,7 +153,7 @@ template <typename TD> struct ZStageArgs {
     int nz;
     long long plane;  // nx*ny
     double h;
-    const double *frag;  // operator fragments per lane (make_zstage_tables)
+    const double *frag;  // operator fragments per lane (z_tables)
     const double *ztab;  // z, 1 - z^3, Lz(nz,:), NZP each
     const double2 *ypsi, *yA, *atd;
     const C2<TD> *dxpsi, *dypsi, *dAt, *B, *dxxpsi, *dyypsi;

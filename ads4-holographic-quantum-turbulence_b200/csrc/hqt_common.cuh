@@ -74,23 +74,11 @@ __host__ __device__ constexpr int ct_lines(int N, int nbuf, int esize = 16) {
     const int v = ((54 * 1024) / esize / N - 1) / nbuf;
     return v < 1 ? 1 : (v > 16 ? 16 : v);
 }
-// The same for the y passes, whose lines are NB adjacent columns: FP64 lines
-// of 512 points get about 108 KB (two blocks per SM; four lines instead of
-// one), so that a y-line load reads 64 contiguous bytes per row and the radix
-// passes have work for all threads.  Measured at 512x512x25 (FP64): y_rhs
-// 984 -> 835 us, filter_y 611 -> 445 us.  At 256 points (eight lines instead
-// of four) the 32-run ensemble was 9% slower, and the x passes (contiguous
-// lines) and the FP32 passes were slower with the larger blocks: they keep
-// 54 KB.
-// At 1024 points 128 KB holds two FP64 lines of the y pass (one line left a
-// warp's y load 32 rows wide), and 108 KB four FP32 lines.
+// The same for the y passes, whose lines are NB adjacent columns: at 1024 points
+// about 108 KB hold four FP32 lines (1024x1024x33, mixed: y_rhs 5.87 -> 3.03 ms when
+// it was set); shorter lines were slower with the larger blocks.
 __host__ __device__ constexpr int ct_lines_y(int N, int nbuf, int esize = 16) {
-    const int budget = (esize == 16 && N >= 1024   ? 128
-                        : esize == 16 && N >= 512 ? 108
-                        : esize == 8 && N >= 1024 ? 108
-                                                  : 54) *
-                       1024;
-    const int v = (budget / esize / N - 1) / nbuf;
+    const int v = ((N >= 1024 ? 108 : 54) * 1024 / esize / N - 1) / nbuf;
     return v < 1 ? 1 : (v > 16 ? 16 : v);
 }
 
