@@ -256,22 +256,7 @@ LineTab<double> line_tab(const hqt_ctx *c, bool y, bool half) {
     t.tw = y ? c->twy : c->twx;
     t.freq = y ? c->freqy : c->freqx;
     t.pos = y ? c->posy : c->posx;
-    int nbl = lnbl(p.n, y);
-    if (half && nbl > 0) --nbl;
-    t.g.n_ = p.n;
-    t.g.nbl_ = nbl;
-    t.g.np_ = p.np;
-    for (int i = 0; i < 2; ++i) t.g.th_[i] = lthreads_rt(p, nbl, i + 1);
-    t.g.swz_ = lswz(p.n, nbl, !y);
-    auto magic = [](int d) { return (unsigned)(((1ull << 32) + d - 1) / d); };
-    t.g.mn_ = magic(p.n);
-    for (int i = 0; i < p.np; ++i) {
-        t.g.R_[i] = p.R[i];
-        t.g.s_[i] = p.s[i];
-        t.g.tw_[i] = p.tw[i];
-        t.g.mg_[i] = magic(p.s[i]);
-        t.g.mr_[i] = magic(p.n / p.R[i]);
-    }
+    t.g = rgeo(p, y, half);
     return t;
 }
 

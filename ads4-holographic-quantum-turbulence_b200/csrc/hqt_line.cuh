@@ -553,18 +553,40 @@ template <typename T, class G, bool AX> struct LineEng {
     template <typename Ld> __device__ __forceinline__ void first_d(C *X, Ld ld) const {
         at_first([&](auto rc, int s, unsigned, unsigned mr, int o) {
             constexpr int R = decltype(rc)::value;
-            each<R>(mr, [&](int b, int j) {
-                C v[R];
-#pragma unroll
-                for (int r = 0; r < R; ++r) v[r] = ld(b, j + r * s);
-                if (kLevel) {
-                    const C x0 = ld(b, 0);
-#pragma unroll
-                    for (int r = 0; r < R; ++r) v[r] = v[r] - x0;
-                }
-                first_fly<R>(X, b, j, s, o, v);
-            });
+            each<R>(mr, [&](int b, int j) { first_d_fly<R>(X, b, j, s, o, ld); });
         });
+    }
+    // ... of A and B, by the threads that read them in last2.  (With a barrier ahead of a
+    // first_d(B, ..) instead, y_rhs by a runtime plan took 1611 us at 1001x1001x20 and 79.8
+    // at 250x180x20; so 1440 and 77.4.)
+    template <typename LdA, typename LdB>
+    __device__ __forceinline__ void first_d2(LdA lda, LdB ldb) const {
+        if constexpr (G::kStatic) {
+            first_d(A, lda);
+            first_d(B, ldb);
+        } else {
+            at_first([&](auto rc, int s, unsigned, unsigned mr, int o) {
+                constexpr int R = decltype(rc)::value;
+                each_of<R>(true, mr, [&](bool x, int b, int j) {
+                    if (x)
+                        first_d_fly<R>(B, b, j, s, o, ldb);
+                    else
+                        first_d_fly<R>(A, b, j, s, o, lda);
+                });
+            });
+        }
+    }
+    template <int R, typename Ld>
+    __device__ __forceinline__ void first_d_fly(C *X, int b, int j, int s, int o, Ld ld) const {
+        C v[R];
+#pragma unroll
+        for (int r = 0; r < R; ++r) v[r] = ld(b, j + r * s);
+        if (kLevel) {
+            const C x0 = ld(b, 0);
+#pragma unroll
+            for (int r = 0; r < R; ++r) v[r] = v[r] - x0;
+        }
+        first_fly<R>(X, b, j, s, o, v);
     }
     template <int R>
     __device__ __forceinline__ void first_fly(C *X, int b, int j, int s, int o, C (&v)[R]) const {
@@ -719,6 +741,10 @@ template <typename T, class G, bool AX> struct LineEng {
     // ... of A and B with the twiddles loaded once: sa(b, e, v, x) with
     // x = get(b, e), sb(b, e, v).  x is read for up to 8 elements ahead of their
     // stores (a read after a store could not move ahead of it).
+    // No barrier follows: a first_d(A, ..) may come next, or first_d2, in which each
+    // thread takes the butterflies of A and B that it takes here.  (Not a first_d(B, ..):
+    // with a runtime plan each_of deals out B's butterflies after A's, from where it is
+    // in the round of threads, and first_d from thread 0.)
     template <typename Get, typename Sa, typename Sb>
     __device__ __forceinline__ void last2(bool two, Get get, Sa sa, Sb sb) const {
         at_first([&](auto rc, int s, unsigned, unsigned mr, int o) {

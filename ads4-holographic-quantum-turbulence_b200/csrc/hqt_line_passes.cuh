@@ -11,7 +11,7 @@
 // Measured, us a launch, with threads over the lines first and the twiddles loaded
 // for each buffer -> as it is: 512x512x25 x_rhs 196 -> 160 (3.6 TB/s), y_rhs 250 ->
 // 244 (3.0 TB/s), filter x forward 154 -> 125, x inverse 183 -> 164; 256x256x25 x_rhs
-// 50 -> 38; with a runtime plan 1001x1001x20 x_rhs 853 -> 864, y_rhs 1540 -> 1517,
+// 50 -> 38; with a runtime plan 1001x1001x20 x_rhs 853 -> 864, y_rhs 1540 -> 1440,
 // filter x forward / y / x inverse 636 / 797 / 981 -> 491 / 588 / 659.
 #pragma once
 #include "hqt_line.cuh"
@@ -80,16 +80,17 @@ __global__ void HQT_L_BOUNDS(G) k_ly_rhs(const __grid_constant__ YRhsArgs<T> a) 
         if (f == 0) {
             w.first_d(w.A, [&](int b, int e) { return b < valid ? a.psi[at(b, e)] : lzero<T>(); });
         } else {
-            w.first_d(w.A, [&](int b, int e) {
-                if (b >= valid) return lzero<T>();
-                const long long g = at(b, e);
-                return mk2<T>(a.E[g].x, a.A[g].y);
-            });
-            w.first_d(w.B, [&](int b, int e) {
-                if (b >= valid) return lzero<T>();
-                const long long g = at(b, e);
-                return mk2<T>(a.A[g].x, a.E[g].y);
-            });
+            w.first_d2(
+                [&](int b, int e) {
+                    if (b >= valid) return lzero<T>();
+                    const long long g = at(b, e);
+                    return mk2<T>(a.E[g].x, a.A[g].y);
+                },
+                [&](int b, int e) {
+                    if (b >= valid) return lzero<T>();
+                    const long long g = at(b, e);
+                    return mk2<T>(a.A[g].x, a.E[g].y);
+                });
         }
         w.forward_mid(f == 1);
         if (f == 0) {

@@ -176,4 +176,26 @@ __host__ __device__ constexpr int lnbl(int n, bool along_y) {
     return b;
 }
 
+// Runtime geometry of a plan; `half`: half the lines per block.
+inline RGeo rgeo(const LPlan &p, bool along_y, bool half) {
+    RGeo g{};
+    int nbl = lnbl(p.n, along_y);
+    if (half && nbl > 0) --nbl;
+    g.n_ = p.n;
+    g.nbl_ = nbl;
+    g.np_ = p.np;
+    for (int i = 0; i < 2; ++i) g.th_[i] = lthreads_rt(p, nbl, i + 1);
+    g.swz_ = lswz(p.n, nbl, !along_y);
+    auto magic = [](int d) { return (unsigned)(((1ull << 32) + d - 1) / d); };
+    g.mn_ = magic(p.n);
+    for (int i = 0; i < p.np; ++i) {
+        g.R_[i] = p.R[i];
+        g.s_[i] = p.s[i];
+        g.tw_[i] = p.tw[i];
+        g.mg_[i] = magic(p.s[i]);
+        g.mr_[i] = magic(p.n / p.R[i]);
+    }
+    return g;
+}
+
 }  // namespace hqt
