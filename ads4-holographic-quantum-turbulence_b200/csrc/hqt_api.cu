@@ -113,6 +113,7 @@ struct hqt_ctx {
     // radial stage: operand tables (z_tables) and the tensor-map encoder
     double *zfrag = nullptr, *ztab = nullptr;
     PFN_cuTensorMapEncodeTiled_v12000 tmap_encode = nullptr;
+    int copy_polls = kZsPolls;  // polls of a wait for one of its copies
     // launch geometry
     int NBx_rhs = 1, NBx_2 = 1, TXy_rhs = 1, TXy_2 = 1, TXy_filt = 1;
     bool cx = false, cy = false;  // compile-time line passes along x / y
@@ -658,6 +659,7 @@ template <typename TD> int launch_zstage(hqt_ctx *c, int mode, ZStageArgs<TD> a)
     a.frag = c->zfrag;
     a.ztab = c->ztab;
     a.fault = &c->st->fault;
+    a.polls = c->copy_polls;
     struct {
         CUtensorMap *m;
         const void *p;
@@ -699,6 +701,7 @@ int launch_zcons(hqt_ctx *c) {
     a.frag = c->zfrag;
     a.ztab = c->ztab;
     a.fault = &c->st->fault;
+    a.polls = c->copy_polls;
     RC(zs_map<double>(c, &a.mPS, a.psi, 2, kZcRowP / 16));
     RC(zs_map<double>(c, a.mDIV, a.divA, 1, kZcRowD / 8));
     Prof pr(c, K_ZCONS);
@@ -1941,6 +1944,17 @@ int hqt_set_stream(hqt_ctx *c, void *s) {
     DeviceGuard guard(c->device);
     CK(cudaStreamSynchronize(c->stream));
     c->stream = s ? reinterpret_cast<cudaStream_t>(s) : c->own_stream;
+    return HQT_OK;
+}
+
+// Sets how often the radial kernels poll for a copy before it counts as lost (0: each
+// wait gives up at once).  For the tests of that path; not in hqt.h.
+int hqt_set_copy_polls(hqt_ctx *c, int polls) {
+    if (!c || polls < 0) return HQT_EINVAL;
+    DeviceGuard guard(c->device);
+    CK(cudaStreamSynchronize(c->stream));
+    drop_graph(c);
+    c->copy_polls = polls;
     return HQT_OK;
 }
 

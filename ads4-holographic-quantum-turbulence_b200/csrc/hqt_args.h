@@ -173,6 +173,7 @@ template <typename TD> struct ZStageArgs {
     double2 *f1;              // right-hand-side outputs (MODE 0)
     double *f3, *f4, *f2b;
     int *fault;               // set when a copy did not arrive
+    int polls;                // of a wait for a copy before it counts as lost
 };
 
 template <typename T> struct ZConsArgs {
@@ -186,7 +187,8 @@ template <typename T> struct ZConsArgs {
     const T *rho;  // 2-D
     C2<T> *O;      // 2-D boundary order parameter (may be null)
     const double *frag, *ztab;  // operand tables (hqt_zdims.h)
-    int *fault;                 // set when a copy never completed
+    int *fault;                 // set when a copy did not arrive
+    int polls;                  // of a wait for a copy before it counts as lost
     CUtensorMap mPS, mDIV[2];   // Psi, div A (ZsSplit)
 };
 

@@ -202,11 +202,11 @@ __global__ void k_rho_scatter(const double *rho2, int nz, long long plane, doubl
 }
 
 // Guard of a captured step: the step graph runs its body (one RK4 step) only
-// while no earlier step has produced a non-finite value, so a run stops at
-// the first bad step like the reference's NaN guard
-// (scripts/simulation/tevol_driven_cluster.m:182-185).
+// while no earlier step has produced a non-finite value (so a run stops at
+// the first bad step like the reference's NaN guard,
+// scripts/simulation/tevol_driven_cluster.m:182-185) or lost a copy.
 __global__ void k_step_guard(cudaGraphConditionalHandle h, const DevStatus *st) {
-    cudaGraphSetConditional(h, st->first_bad_step == LLONG_MAX ? 1u : 0u);
+    cudaGraphSetConditional(h, st->first_bad_step == LLONG_MAX && st->fault == 0 ? 1u : 0u);
 }
 
 __global__ void k_step_end(DevStatus *st) {

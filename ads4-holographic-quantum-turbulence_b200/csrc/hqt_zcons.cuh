@@ -100,7 +100,13 @@ __global__ void __launch_bounds__(kZsThreads, ZcLay<NZP>::min_blocks)
             return *reinterpret_cast<const double2 *>(ps + i * kZcRowP + c * 16);
         };
         const double rA = okA ? a.rho[sA] : 0.0, rB = okB ? a.rho[sB] : 0.0;
-        zs_wait(bar + 8 * buf, parity, dead);
+        if (!dead && !zs_wait(bar + 8 * buf, parity, a.polls)) {
+            dead = true;
+            if (threadIdx.x == 0) {
+                zs_drain(bar + 8 * buf, parity);
+                if (tile + gridDim.x < ntiles) zs_drain(bar + 8 * (buf ^ 1), parity ^ buf);
+            }
+        }
 
         // ---- cons -> V1 (levels < nz - 1 enter Lzr), O -------------------------
         double oar = 0.0, oai = 0.0, obr = 0.0, obi = 0.0;
@@ -137,7 +143,7 @@ __global__ void __launch_bounds__(kZsThreads, ZcLay<NZP>::min_blocks)
             }
         }
         __syncthreads();  // every warp is done with this buffer
-        load(tile + 2 * (long long)gridDim.x, buf);
+        if (!dead) load(tile + 2 * (long long)gridDim.x, buf);
         {  // v = Lzr(cons) - rhoi -> V2
             double F[M1][2];
             ops.template lz1<Lay::oV1>(sm, F);
@@ -195,7 +201,7 @@ __global__ void __launch_bounds__(kZsThreads, ZcLay<NZP>::min_blocks)
         parity ^= buf;
         buf ^= 1;
     }
-    if (dead && a.fault) *a.fault = 1;
+    if (dead) *a.fault = 1;
 }
 
 }  // namespace hqt

@@ -43,6 +43,9 @@ struct ZsSplit {
     }
 };
 
+// Polls of a wait for a copy before it counts as lost: about a second.
+constexpr int kZsPolls = 1 << 20;
+
 // Row g of an mma tile stands for level 8m + zs_row(g) (bits 0 and 1 swapped).
 __host__ __device__ constexpr int zs_row(int g) { return (g & 4) | ((g & 1) << 1) | ((g >> 1) & 1); }
 

@@ -117,12 +117,10 @@ __device__ __forceinline__ void zs_expect(unsigned bar, int bytes) {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(bar), "r"(bytes)
                  : "memory");
 }
-// Waits for a phase, at most about a second: a group that never completes sets
-// `dead`, after which no wait blocks, and the kernel ends with its fault flag up.
-__device__ __forceinline__ void zs_wait(unsigned bar, int parity, bool &dead) {
-    if (dead) return;
+// Waits for a phase, `polls` times about a microsecond; false if it did not complete.
+__device__ __forceinline__ bool zs_wait(unsigned bar, int parity, int polls) {
     unsigned ok = 0;
-    for (int i = 0; i < (1 << 20) && !ok; ++i)
+    for (int i = 0; i < polls && !ok; ++i)
         asm volatile(
             "{\n.reg .pred p;\n"
             "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n"
@@ -130,7 +128,15 @@ __device__ __forceinline__ void zs_wait(unsigned bar, int parity, bool &dead) {
             : "=r"(ok)
             : "r"(bar), "r"(parity), "r"(1000)
             : "memory");
-    if (!ok) dead = true;
+    return ok;
+}
+// The thread that issues a block's copies, after a wait of its own in vain: it issues no
+// more, and waits once more for those in flight, which must not outlive the block.
+// (Every other thread waits no more either; the block runs to its end on whatever its
+// buffers hold and leaves with the fault flag up.  To leave at once, by a barrier with a
+// reduction of the flag, cost 2% of a launch at 301x301x21.)
+static __device__ __noinline__ void zs_drain(unsigned bar, int parity) {
+    zs_wait(bar, parity, kZsPolls);
 }
 // box of a tile's columns x nz levels at element x of a field's level rows
 __device__ __forceinline__ void zs_tma(unsigned dst, const CUtensorMap *map, int x, unsigned bar) {
@@ -386,7 +392,11 @@ __global__ void __launch_bounds__(kZsThreads, ZsDims<NZP>::min_blocks)
                 }
             }
         };
-        zs_wait(barM, parity, dead);
+        if (!dead && !zs_wait(barM, parity, a.polls)) {
+            dead = true;
+            if (leader) zs_drain(barM, parity);
+            if (kK && leader) zs_drain(barZ, parity);
+        }
 
         // ---- g = d A_t + f Lz A -> VA, dp = Lz Psi -> VB ---------------------
         double dA[MH][2], dB[MH][2];  // dp
@@ -473,7 +483,7 @@ __global__ void __launch_bounds__(kZsThreads, ZsDims<NZP>::min_blocks)
         }
         kb = zf_colsum(kb);
         __syncthreads();  // every warp is done with the main inputs
-        if (more) load_M(next);
+        if (more && !dead) load_M(next);
 
         // ---- F3, F4 = Lzr(S), F1 = Lzr(S1) and the RK updates ------------------
         auto update_A = [&](int i, double fx, double fy, double2 z, double2 K) {
@@ -538,7 +548,11 @@ __global__ void __launch_bounds__(kZsThreads, ZsDims<NZP>::min_blocks)
         } else {
             double F[M1][2], G[M1][2];
             ops.template lz1_2<Lay::oVA, Lay::oVB>(sm, F, G);
-            if (kK) zs_wait(barZ, parity, dead);
+            if (kK && !dead && !zs_wait(barZ, parity, a.polls)) {
+                dead = true;
+                if (leader) zs_drain(barZ, parity);
+                if (leader && more) zs_drain(barM, parity ^ 1);
+            }
             ops.rows(F, g, [&](int, int i, double fx, double fy) {
                 update_A(i, fx, fy, MODE ? zs_at<Lay::oZA>(sm, i, col) : none,
                          kK ? zs_at<Lay::oKA>(sm, i, col) : none);
@@ -562,9 +576,9 @@ __global__ void __launch_bounds__(kZsThreads, ZsDims<NZP>::min_blocks)
             }
         }
         __syncthreads();  // every warp is done with the state (and VA, VB)
-        if (more) load_Z(next);
+        if (more && !dead) load_Z(next);
     }
-    if (dead && a.fault) *a.fault = 1;
+    if (dead) *a.fault = 1;
 }
 
 }  // namespace hqt
