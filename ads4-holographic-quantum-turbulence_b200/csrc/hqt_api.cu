@@ -1035,6 +1035,14 @@ int prestep(hqt_ctx *c) {
 
 int observables(hqt_ctx *c, const double2 *O, const double *rho2, double *out);
 
+constexpr const char *kLostCopy = "the radial stage's copies did not arrive";
+// Reports a fault and takes the flag down: a later call has its own.
+int lost_copy(hqt_ctx *c) {
+    CK(cudaMemsetAsync(&c->st->fault, 0, sizeof(int), c->stream));
+    CK(cudaStreamSynchronize(c->stream));
+    return fail(c, HQT_ECUDA, kLostCopy);
+}
+
 int run_steps(hqt_ctx *c, int64_t nsteps, hqt_diag *diag) {
     DevStatus h0{};
     CK(cudaMemcpyAsync(&h0, c->st, sizeof(DevStatus), cudaMemcpyDeviceToHost, c->stream));
@@ -1083,7 +1091,7 @@ int run_steps(hqt_ctx *c, int64_t nsteps, hqt_diag *diag) {
             DevStatus h{};
             CK(cudaMemcpyAsync(&h, c->st, sizeof(DevStatus), cudaMemcpyDeviceToHost, c->stream));
             CK(cudaStreamSynchronize(c->stream));
-            if (h.fault) return fail(c, HQT_ECUDA, "the radial stage's copies did not arrive");
+            if (h.fault) return lost_copy(c);
             if (h.first_bad_step != LLONG_MAX) {
                 bad = true;
                 if (diag) diag->nonfinite_step = h.first_bad_step - step0;
@@ -2128,7 +2136,7 @@ int hqt_rhs_device(hqt_ctx *c, const void *dZ1, const void *dZ2, const void *dZ3
     int fault = 0;
     CK(cudaMemcpyAsync(&fault, &c->st->fault, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
     CK(cudaStreamSynchronize(c->stream));
-    if (fault) return fail(c, HQT_ECUDA, "the radial stage's copies did not arrive");
+    if (fault) return lost_copy(c);
     return HQT_OK;
 }
 
@@ -2453,9 +2461,16 @@ int hqt_ensemble_step_device(hqt_ensemble *e, void *const *dZ1, void *const *dZ2
                 EK(cudaMemcpyAsync(&hs[i], e->m[i]->st, sizeof(DevStatus),
                                    cudaMemcpyDeviceToHost, e->stream));
             EK(cudaStreamSynchronize(e->stream));
+            bool lost = false;
             for (size_t i = 0; i < n; ++i)
-                if (hs[i].fault)
-                    return efail(e, HQT_ECUDA, "the radial stage's copies did not arrive");
+                if (hs[i].fault) {
+                    lost = true;
+                    EK(cudaMemsetAsync(&e->m[i]->st->fault, 0, sizeof(int), e->stream));
+                }
+            if (lost) {
+                EK(cudaStreamSynchronize(e->stream));
+                return efail(e, HQT_ECUDA, kLostCopy);
+            }
             for (size_t i = 0; i < n; ++i)
                 if (hs[i].first_bad_step != LLONG_MAX) {
                     bad = true;

@@ -42,6 +42,22 @@ def test_a_lost_copy_is_an_error_and_the_context_goes_on(hqt, cuda, nx, ny, nz, 
             assert all(np.array_equal(g, w) for g, w in zip(got, want))
 
 
+def test_a_right_hand_side_after_a_fault(hqt, dev):
+    """A fault is reported by the call it happened in, not by the next one."""
+    to_d, _ = dev
+    state = run_state(hqt, 33, 33, 21)
+    Z = [to_d(a) for a in state[:4]]
+    with hqt.Simulation(33, 33, 21, Lx=16.5, mu=6.0, vy=-2.0) as sim:
+        want = [f.clone() for f in sim.rhs_device(*Z)]
+        for call in (lambda: sim.rhs_device(*Z), lambda: sim.step(*state, nsteps=1)):
+            set_polls(hqt, sim, 0)
+            with pytest.raises(hqt.HQTError, match="copies did not arrive"):
+                call()
+            set_polls(hqt, sim, POLLS)
+            for f, w in zip(sim.rhs_device(*Z), want):
+                assert bool((f == w).all())
+
+
 def test_an_ensemble_reports_a_lost_copy(hqt, dev):
     to_d, from_d = dev
     grids = (24, 33)
