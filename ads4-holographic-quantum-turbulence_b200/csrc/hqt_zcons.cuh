@@ -142,6 +142,7 @@ __global__ void __launch_bounds__(kZsThreads, ZcLay<NZP>::min_blocks)
                 }
             }
         }
+        zs_release();
         __syncthreads();  // every warp is done with this buffer
         if (!dead) load(tile + 2 * (long long)gridDim.x, buf);
         {  // v = Lzr(cons) - rhoi -> V2

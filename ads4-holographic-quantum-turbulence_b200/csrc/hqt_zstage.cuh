@@ -135,8 +135,15 @@ __device__ __forceinline__ bool zs_wait(unsigned bar, int parity, int polls) {
 // (Every other thread waits no more either; the block runs to its end on whatever its
 // buffers hold and leaves with the fault flag up.  To leave at once, by a barrier with a
 // reduction of the flag, cost 2% of a launch at 301x301x21.)
-static __device__ __noinline__ void zs_drain(unsigned bar, int parity) {
+__device__ __forceinline__ void zs_drain(unsigned bar, int parity) {
     zs_wait(bar, parity, kZsPolls);
+}
+// Ahead of a barrier behind which a region is refilled: this thread's reads of it (and
+// writes, of a copy set aside) come before the refill, which another proxy writes.  A
+// value read before the barrier has to be used before it too: loads are only ordered by
+// their use.
+__device__ __forceinline__ void zs_release() {
+    asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
 }
 // box of a tile's columns x nz levels at element x of a field's level rows
 __device__ __forceinline__ void zs_tma(unsigned dst, const CUtensorMap *map, int x, unsigned bar) {
@@ -482,6 +489,7 @@ __global__ void __launch_bounds__(kZsThreads, ZsDims<NZP>::min_blocks)
             }
         }
         kb = zf_colsum(kb);
+        zs_release();
         __syncthreads();  // every warp is done with the main inputs
         if (more && !dead) load_M(next);
 
@@ -575,6 +583,7 @@ __global__ void __launch_bounds__(kZsThreads, ZsDims<NZP>::min_blocks)
                     a.wrho[site] = a.zrho[site] - (1.0 / 6.0) * (a.krho[site] + k);
             }
         }
+        if (kK) zs_release();
         __syncthreads();  // every warp is done with the state (and VA, VB)
         if (more && !dead) load_Z(next);
     }
