@@ -89,7 +89,7 @@ __global__ void __launch_bounds__(kZsThreads, ZcLay<NZP>::min_blocks)
     const int oD = zc_site(warp, kk, part) * 8;
     const int cA = zc_site(warp, q, 0), cB = zc_site(warp, q, 1);  // its result columns
     const int col = zs_col(warp, q), gr = zs_row(g);
-    bool dead = false;
+    int lost = 0;  // 1, 2: waited in vain, with and without the next tile in flight
     int buf = 0, parity = 0;
 #pragma unroll 1
     for (long long tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
@@ -100,13 +100,8 @@ __global__ void __launch_bounds__(kZsThreads, ZcLay<NZP>::min_blocks)
             return *reinterpret_cast<const double2 *>(ps + i * kZcRowP + c * 16);
         };
         const double rA = okA ? a.rho[sA] : 0.0, rB = okB ? a.rho[sB] : 0.0;
-        if (!dead && !zs_wait(bar + 8 * buf, parity, a.polls)) {
-            dead = true;
-            if (threadIdx.x == 0) {
-                zs_drain(bar + 8 * buf, parity);
-                if (tile + gridDim.x < ntiles) zs_drain(bar + 8 * (buf ^ 1), parity ^ buf);
-            }
-        }
+        if (!lost && !zs_wait(bar + 8 * buf, parity, a.polls))
+            lost = tile + gridDim.x < ntiles ? 1 : 2;
 
         // ---- cons -> V1 (levels < nz - 1 enter Lzr), O -------------------------
         double oar = 0.0, oai = 0.0, obr = 0.0, obi = 0.0;
@@ -144,7 +139,7 @@ __global__ void __launch_bounds__(kZsThreads, ZcLay<NZP>::min_blocks)
         }
         zs_release();
         __syncthreads();  // every warp is done with this buffer
-        if (!dead) load(tile + 2 * (long long)gridDim.x, buf);
+        if (!lost) load(tile + 2 * (long long)gridDim.x, buf);
         {  // v = Lzr(cons) - rhoi -> V2
             double F[M1][2];
             ops.template lz1<Lay::oV1>(sm, F);
@@ -199,10 +194,16 @@ __global__ void __launch_bounds__(kZsThreads, ZcLay<NZP>::min_blocks)
                 a.A[gb + sB] = make_double2(0.0, -a.vy);
             }
         }
-        parity ^= buf;
-        buf ^= 1;
+        if (!lost) {
+            parity ^= buf;
+            buf ^= 1;
+        }
     }
-    if (dead) *a.fault = 1;
+    if (lost) {
+        if (threadIdx.x == 0) zs_drain(bar + 8 * buf, parity);
+        if (threadIdx.x == 0 && lost == 1) zs_drain(bar + 8 * (buf ^ 1), parity ^ buf);
+        *a.fault = 1;
+    }
 }
 
 }  // namespace hqt

@@ -130,11 +130,12 @@ __device__ __forceinline__ bool zs_wait(unsigned bar, int parity, int polls) {
             : "memory");
     return ok;
 }
-// The thread that issues a block's copies, after a wait of its own in vain: it issues no
-// more, and waits once more for those in flight, which must not outlive the block.
-// (Every other thread waits no more either; the block runs to its end on whatever its
-// buffers hold and leaves with the fault flag up.  To leave at once, by a barrier with a
-// reduction of the flag, cost 2% of a launch at 301x301x21.)
+// After a wait in vain (`lost`) a thread waits no more and counts no further phases, and
+// the thread that issues the block's copies issues none: the block runs to its end on
+// whatever its buffers hold.  There that thread waits once more for the phases that were
+// in flight (zs_drain), which must not outlive the block, and the fault flag goes up.
+// (To wait for them, or to leave, where the first wait gave up cost 1-2% of a launch at
+// 301x301x21: a call or a loop in the tile's code, a barrier with a reduction.)
 __device__ __forceinline__ void zs_drain(unsigned bar, int parity) {
     zs_wait(bar, parity, kZsPolls);
 }
@@ -375,14 +376,15 @@ __global__ void __launch_bounds__(kZsThreads, ZsDims<NZP>::min_blocks)
     const int gr = zs_row(g);
     const ZsOps<NZP> ops(a.frag, lane, warp, nz);
     const long long ntiles = (P + kZsCols - 1) / kZsCols;
-    bool dead = false;
+    int lost = 0;  // 1: waited in vain for main inputs; 2, 3: for the state, with and
+                   // without the next tile's main inputs in flight
     if ((long long)blockIdx.x < ntiles) {
         load_M((long long)blockIdx.x * kZsCols);
         load_Z((long long)blockIdx.x * kZsCols);
     }
     int parity = 0;
 #pragma unroll 1
-    for (long long tile = blockIdx.x; tile < ntiles; tile += gridDim.x, parity ^= 1) {
+    for (long long tile = blockIdx.x; tile < ntiles; tile += gridDim.x, parity ^= !lost) {
         const long long site = tile * kZsCols + col;  // of this lane's results
         const bool more = tile + gridDim.x < ntiles;
         const long long next = (tile + gridDim.x) * kZsCols;
@@ -399,11 +401,7 @@ __global__ void __launch_bounds__(kZsThreads, ZsDims<NZP>::min_blocks)
                 }
             }
         };
-        if (!dead && !zs_wait(barM, parity, a.polls)) {
-            dead = true;
-            if (leader) zs_drain(barM, parity);
-            if (kK && leader) zs_drain(barZ, parity);
-        }
+        if (!lost && !zs_wait(barM, parity, a.polls)) lost = 1;
 
         // ---- g = d A_t + f Lz A -> VA, dp = Lz Psi -> VB ---------------------
         double dA[MH][2], dB[MH][2];  // dp
@@ -491,7 +489,7 @@ __global__ void __launch_bounds__(kZsThreads, ZsDims<NZP>::min_blocks)
         kb = zf_colsum(kb);
         zs_release();
         __syncthreads();  // every warp is done with the main inputs
-        if (more && !dead) load_M(next);
+        if (more && !lost) load_M(next);
 
         // ---- F3, F4 = Lzr(S), F1 = Lzr(S1) and the RK updates ------------------
         auto update_A = [&](int i, double fx, double fy, double2 z, double2 K) {
@@ -556,11 +554,7 @@ __global__ void __launch_bounds__(kZsThreads, ZsDims<NZP>::min_blocks)
         } else {
             double F[M1][2], G[M1][2];
             ops.template lz1_2<Lay::oVA, Lay::oVB>(sm, F, G);
-            if (kK && !dead && !zs_wait(barZ, parity, a.polls)) {
-                dead = true;
-                if (leader) zs_drain(barZ, parity);
-                if (leader && more) zs_drain(barM, parity ^ 1);
-            }
+            if (kK && !lost && !zs_wait(barZ, parity, a.polls)) lost = more ? 2 : 3;
             ops.rows(F, g, [&](int, int i, double fx, double fy) {
                 update_A(i, fx, fy, MODE ? zs_at<Lay::oZA>(sm, i, col) : none,
                          kK ? zs_at<Lay::oKA>(sm, i, col) : none);
@@ -585,9 +579,13 @@ __global__ void __launch_bounds__(kZsThreads, ZsDims<NZP>::min_blocks)
         }
         if (kK) zs_release();
         __syncthreads();  // every warp is done with the state (and VA, VB)
-        if (more && !dead) load_Z(next);
+        if (more && !lost) load_Z(next);
     }
-    if (dead) *a.fault = 1;
+    if (lost) {
+        if (leader && lost != 3) zs_drain(barM, lost == 1 ? parity : parity ^ 1);
+        if (leader && kK) zs_drain(barZ, parity);
+        *a.fault = 1;
+    }
 }
 
 }  // namespace hqt
