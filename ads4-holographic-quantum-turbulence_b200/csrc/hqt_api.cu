@@ -16,6 +16,7 @@
 #include <cstdlib>
 #include <cstring>
 #include <fstream>
+#include <functional>
 #include <map>
 #include <mutex>
 #include <sstream>
@@ -146,7 +147,7 @@ struct hqt_ctx {
     std::vector<double> prof_ms;
     long long launches = 0;
     std::string tune_json;  // launch geometry and, when tuned, the candidates timed
-    std::vector<void *> allocs;
+    void *arena = nullptr;  // all device arrays
     std::string err;
 };
 
@@ -278,15 +279,33 @@ int line_pass(hqt_ctx *c, bool y, int kind, const void *args, int nsl) {
     return HQT_OK;
 }
 
-template <typename P> int dalloc(hqt_ctx *c, P **ptr, size_t bytes) {
-    void *q = nullptr;
-    cudaError_t e = cudaMalloc(&q, bytes);
-    if (e != cudaSuccess) return fail(c, HQT_ENOMEM, std::string("cudaMalloc: ") + cudaGetErrorString(e));
-    cudaMemset(q, 0, bytes);
-    c->allocs.push_back(q);
-    *ptr = reinterpret_cast<P *>(q);
-    return HQT_OK;
-}
+// The device arrays of a context, in one zeroed allocation.  (An array above 1 MB of its
+// own takes about 0.2 ms to allocate: a context of 64x64x21 6.0 ms with one each, now
+// 0.8.)  Those above 1 MB start on 2 MB pages, as they would by themselves.
+struct Arena {
+    struct Part {
+        size_t at;
+        std::function<void(char *)> set;
+    };
+    std::vector<Part> parts;
+    size_t total = 0;
+    template <typename P> void operator()(P **ptr, size_t bytes) {
+        const size_t unit = bytes >= (1u << 20) ? 2u << 20 : 256;
+        total = (total + unit - 1) / unit * unit;
+        parts.push_back({total, [ptr](char *q) { *ptr = reinterpret_cast<P *>(q); }});
+        total += bytes;
+    }
+    int place(hqt_ctx *c) {
+        const cudaError_t e = cudaMalloc(&c->arena, total);
+        if (e != cudaSuccess) {
+            cudaGetLastError();
+            return fail(c, HQT_ENOMEM, std::string("cudaMalloc: ") + cudaGetErrorString(e));
+        }
+        CK(cudaMemset(c->arena, 0, total));
+        for (const Part &a : parts) a.set(static_cast<char *>(c->arena) + a.at);
+        return HQT_OK;
+    }
+};
 
 size_t smem_x(int n, int nbuf, int NB, size_t esize = sizeof(double2)) {
     return esize * (size_t)n * (1 + (size_t)nbuf * NB);
@@ -1693,10 +1712,17 @@ int hqt_create(const hqt_params *params, int device, hqt_ctx **out) {
         c->err = "line length has too many factors";
         return bail(HQT_EUNSUPPORTED);
     }
-    int rc = HQT_OK;
-    auto A = [&](auto **ptr, size_t bytes) {
-        if (rc == HQT_OK) rc = dalloc(c, ptr, bytes);
-    };
+    // operand tables of the radial stage
+    std::vector<double> frag, tab;
+    switch (c->NZP) {
+#define HQT_Z(N)                          \
+    case N:                               \
+        z_tables<N>(zhost(c), frag, tab); \
+        break;
+        HQT_NZP_LIST(HQT_Z)
+#undef HQT_Z
+    }
+    Arena A;
     A(&c->rootsx, sizeof(double2) * p.nx);
     A(&c->rootsy, sizeof(double2) * p.ny);
     A(&c->mx, sizeof(double) * p.nx);
@@ -1764,7 +1790,9 @@ int hqt_create(const hqt_params *params, int device, hqt_ctx **out) {
     A(&c->obs_partial, sizeof(double2) * kObs * kPartials);
     A(&c->obs_out, sizeof(double) * kObs);
     A(&c->st, sizeof(DevStatus));
-    if (rc != HQT_OK) return bail(rc);
+    A(&c->zfrag, sizeof(double) * frag.size());
+    A(&c->ztab, sizeof(double) * tab.size());
+    if (const int rc = A.place(c)) return bail(rc);
     {
         std::vector<double2> rx = make_roots(p.nx), ry = make_roots(p.ny);
         std::vector<double> hmx(p.nx, 1.0), hmy(p.ny, 1.0);
@@ -1820,20 +1848,8 @@ int hqt_create(const hqt_params *params, int device, hqt_ctx **out) {
             }
         }
     }
-    // operand tables and tensor maps of the radial stage
+    // ... and its tensor maps
     {
-        std::vector<double> frag, tab;
-        switch (c->NZP) {
-#define HQT_Z(N)                                   \
-    case N:                                        \
-        z_tables<N>(zhost(c), frag, tab);          \
-        break;
-            HQT_NZP_LIST(HQT_Z)
-#undef HQT_Z
-        }
-        A(&c->zfrag, sizeof(double) * frag.size());
-        A(&c->ztab, sizeof(double) * tab.size());
-        if (rc != HQT_OK) return bail(rc);
         void *fn = nullptr;
         cudaDriverEntryPointQueryResult q{};
         if (cudaMemcpy(c->zfrag, frag.data(), sizeof(double) * frag.size(),
@@ -1891,20 +1907,25 @@ int hqt_create(const hqt_params *params, int device, hqt_ctx **out) {
         cudaError_t e = fft_init(tc.data(), ts.data(), (int)tc.size(), maxs);
         std::vector<double> bc, bs;
         make_big_tables(bc, bs);
-        if (e == cudaSuccess) e = pfa_init_301();
-        if (e == cudaSuccess) e = line_rt_init_x(maxs);
-        if (e == cudaSuccess) e = line_rt_init_y(maxs);
-#define HQT_CI(N)                                                                            \
-    if (e == cudaSuccess)                                                                    \
-        e = ct_init<N>(tc.data(), ts.data(), (int)tc.size(), bc.data(), bs.data(), (int)bc.size(), maxs);
+        // the kernels of this grid's lengths only, whichever engine is chosen for them
+        // (each costs two calls, the tables a copy: with those of every length a context of
+        // 33x33x10 took 2.0 ms, of 64x64x21 6.8; so 1.3 and 6.0)
+        auto used = [&](int n) { return n == p.nx || n == p.ny; };
+        if (e == cudaSuccess && (pfa_length(p.nx) || pfa_length(p.ny))) e = pfa_init_301();
+        if (e == cudaSuccess && c->lpx.np) e = line_rt_init_x(maxs);
+        if (e == cudaSuccess && c->lpy.np) e = line_rt_init_y(maxs);
+#define HQT_CI(N)                                                                        \
+    if (e == cudaSuccess && c->mixed && used(N))                                         \
+        e = ct_init<N>(tc.data(), ts.data(), (int)tc.size(), bc.data(), bs.data(),       \
+                       (int)bc.size(), maxs);
         HQT_CN_LIST(HQT_CI)
 #undef HQT_CI
 #define HQT_LI(N) \
-    if (e == cudaSuccess) e = ct_init64<N>(maxs);
+    if (e == cudaSuccess && used(N)) e = ct_init64<N>(maxs);
         HQT_LN_LIST(HQT_LI)
 #undef HQT_LI
 #define HQT_Z(N) \
-    if (e == cudaSuccess) e = z_init<N>(maxs);
+    if (e == cudaSuccess && c->NZP == N) e = z_init<N>(maxs);
         HQT_NZP_LIST(HQT_Z)
 #undef HQT_Z
         if (e != cudaSuccess) {
@@ -1938,7 +1959,7 @@ void hqt_destroy(hqt_ctx *c) {
         cudaEventDestroy(e.a);
         cudaEventDestroy(e.b);
     }
-    for (void *q : c->allocs) cudaFree(q);
+    if (c->arena) cudaFree(c->arena);
     if (c->side) cudaStreamSynchronize(c->side);
     if (c->ev_fork) cudaEventDestroy(c->ev_fork);
     if (c->ev_join) cudaEventDestroy(c->ev_join);
