@@ -1736,8 +1736,6 @@ int hqt_create(const hqt_params *params, int device, hqt_ctx **out) {
     const size_t V = (size_t)c->vol, P2 = (size_t)c->plane;
     A(&c->psi, sizeof(double2) * V);
     A(&c->at, sizeof(double) * V);
-    A(&c->ax, sizeof(double) * V);
-    A(&c->ay, sizeof(double) * V);
     A(&c->rho, sizeof(double) * P2);
     for (int b = 0; b < 2; ++b) {
         A(&c->ypsi2[b], sizeof(double2) * V);
@@ -1757,7 +1755,6 @@ int hqt_create(const hqt_params *params, int device, hqt_ctx **out) {
     A(&c->divA, sizeof(double) * V);
     A(&c->B, sizeof(double2) * V);
     A(&c->dAt, sizeof(double2) * V);
-    A(&c->dxax, sizeof(double) * V);
     A(&c->O, sizeof(double2) * P2);
     if (c->mixed) {
         for (int b = 0; b < 3; ++b) {
@@ -1793,6 +1790,13 @@ int hqt_create(const hqt_params *params, int device, hqt_ctx **out) {
     A(&c->zfrag, sizeof(double) * frag.size());
     A(&c->ztab, sizeof(double) * tab.size());
     if (const int rc = A.place(c)) return bail(rc);
+    // A_x and A_y of the host's state are read ahead of a call's first y_rhs and written
+    // behind a step's last: in the meantime their place is B's.  Likewise d_x A_x of the
+    // constraint, behind the last use of d_xx A_y.  (280 bytes a site in FP64; 304 with
+    // arrays of their own.)
+    c->ax = &c->B->x;
+    c->ay = c->ax + V;
+    c->dxax = c->dxxay;
     {
         std::vector<double2> rx = make_roots(p.nx), ry = make_roots(p.ny);
         std::vector<double> hmx(p.nx, 1.0), hmy(p.ny, 1.0);
