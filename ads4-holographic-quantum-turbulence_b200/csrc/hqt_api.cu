@@ -249,6 +249,12 @@ bool in_place(const hqt_ctx *c, bool y) {
     return y ? !c->py && c->lpy.np > 0 : !c->px && c->lpx.np > 0;
 }
 
+// Whether the context has compile-time passes along an axis (301 = 7*43, which has no
+// in-place plan, only those of the FP32 stages).
+bool ct_usable(const hqt_ctx *c, bool y) {
+    return ct_supported(y ? c->ny : c->nx) && (c->mixed || (y ? c->lpy : c->lpx).np > 0);
+}
+
 // Tables and runtime geometry of an in-place axis; `half`: half the lines per
 // block (a candidate of the autotuner).
 LineTab<double> line_tab(const hqt_ctx *c, bool y, bool half) {
@@ -1220,7 +1226,7 @@ void tune_file_append(const std::string &key, const LineGeom &g) {
 // length.
 bool geom_valid(const hqt_ctx *c, const LineGeom &g) {
     if ((g.px && !pfa_length(c->nx)) || (g.py && !pfa_length(c->ny))) return false;
-    if ((g.cx && !ct_supported(c->nx)) || (g.cy && !ct_supported(c->ny))) return false;
+    if ((g.cx && !ct_usable(c, false)) || (g.cy && !ct_usable(c, true))) return false;
     const size_t lim = 227 * 1024 - 1024;
     const int v[5] = {g.NBx_rhs, g.NBx_2, g.TXy_rhs, g.TXy_2, g.TXy_filt};
     for (int x : v)
@@ -1282,13 +1288,12 @@ int autotune(hqt_ctx *c) {
     }
     const LineGeom base = get_geom(c);
     std::vector<LineGeom> cand;
-    std::vector<std::pair<bool, bool>> ex, ey;  // (prime-factor, stockham)
+    std::vector<std::pair<bool, bool>> ex, ey;  // (prime-factor, compile-time)
     if (pfa_length(c->nx)) ex.push_back({true, false});
-    // (a compile-time length without an in-place plan has only FP32 passes)
-    if (ct_supported(c->nx) && (c->mixed || c->lpx.np)) ex.push_back({false, true});
+    if (ct_usable(c, false)) ex.push_back({false, true});
     ex.push_back({false, false});
     if (pfa_length(c->ny)) ey.push_back({true, false});
-    if (ct_supported(c->ny) && (c->mixed || c->lpy.np)) ey.push_back({false, true});
+    if (ct_usable(c, true)) ey.push_back({false, true});
     ey.push_back({false, false});
     for (auto x : ex)
         for (auto y : ey) {
@@ -1874,8 +1879,8 @@ int hqt_create(const hqt_params *params, int device, hqt_ctx **out) {
     c->TXy_rhs = pick_lines(p.ny, 4, 16);
     c->TXy_2 = pick_lines(p.ny, 2, 16);
     c->TXy_filt = pick_lines(p.ny, 6, 16);
-    c->cx = ct_supported(p.nx);
-    c->cy = ct_supported(p.ny);
+    c->cx = ct_usable(c, false);
+    c->cy = ct_usable(c, true);
     c->px = pfa_length(p.nx);
     c->py = pfa_length(p.ny);
     if (const char *env = std::getenv("HQT_PDL")) c->pdl = std::string(env) != "0";
