@@ -1272,7 +1272,9 @@ int time_geom(hqt_ctx *c, const LineGeom &g, double *ms) {
 // reset afterwards.
 int autotune(hqt_ctx *c) {
     char kb[160];
-    std::snprintf(kb, sizeof(kb), "dev%d:%dx%dx%d:%s:f%d:w%d", c->device, c->nx, c->ny, c->nz,
+    // e<n>: the set of engines that was timed, to be raised when one of them changes (a
+    // file's choice among others could be a poor one now)
+    std::snprintf(kb, sizeof(kb), "e2:dev%d:%dx%dx%d:%s:f%d:w%d", c->device, c->nx, c->ny, c->nz,
                   c->mixed ? "mixed" : "fp64", c->p.apply_filter, c->p.remove_winding);
     const std::string key = kb;
     {

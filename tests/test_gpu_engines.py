@@ -1,4 +1,5 @@
-"""The engines that a context reports are those that it runs."""
+"""The engines that a context reports are those that it runs, and a tuning file's choice
+among the engines of an older library is not taken."""
 import json
 import os
 import subprocess
@@ -30,3 +31,12 @@ def report(*args, **env):
 def test_reported_engine_without_the_prime_factor_one(cuda, precision, engine):
     chosen = report(301, 64, 8, precision, False, HQT_LINE_ENGINE="stockham")["chosen"]
     assert (chosen["x_engine"], chosen["y_engine"]) == (engine, "compile-time")
+
+
+def test_an_older_librarys_choice_is_tuned_again(cuda, tmp_path):
+    f = tmp_path / "tune.txt"
+    f.write_text("dev0:64x64x12:fp64:f1:w1 0 0 0 0 1 1 1 1 1\n")
+    first = report(64, 64, 12, "fp64", True, HQT_TUNE_CACHE=str(f))
+    assert first["cached"] is False
+    again = report(64, 64, 12, "fp64", True, HQT_TUNE_CACHE=str(f))
+    assert again["cached"] is True and again["chosen"] == first["chosen"]
