@@ -147,7 +147,7 @@ __device__ __forceinline__ void yl_store_rd(int buf, int n, int nb, int nx, long
 // ------------------------------------------------------------------------
 // x pass of a right-hand side
 // ------------------------------------------------------------------------
-template <typename T> __global__ void HQT_FFT_BOUNDS k_x_rhs(XRhsArgs<T> a) {
+template <typename T> __global__ void HQT_FFT_BOUNDS k_x_rhs(const __grid_constant__ XRhsArgs<T> a) {
     const int n = a.plan.n;
     const int L0 = blockIdx.x * a.NB;
     const int nb = min(a.NB, a.nlines - L0);
@@ -190,7 +190,7 @@ template <typename T> __global__ void HQT_FFT_BOUNDS k_x_rhs(XRhsArgs<T> a) {
 // ------------------------------------------------------------------------
 // y pass of a right-hand side
 // ------------------------------------------------------------------------
-template <typename T> __global__ void HQT_FFT_BOUNDS k_y_rhs(YRhsArgs<T> a) {
+template <typename T> __global__ void HQT_FFT_BOUNDS k_y_rhs(const __grid_constant__ YRhsArgs<T> a) {
     const int n = a.ny;
     const int x0 = blockIdx.x * a.TX;
     const int nb = min(a.TX, a.nx - x0);
@@ -284,7 +284,7 @@ template <typename T> __global__ void HQT_FFT_BOUNDS k_y_rhs(YRhsArgs<T> a) {
 // ------------------------------------------------------------------------
 // single-field first derivatives
 // ------------------------------------------------------------------------
-template <typename T> __global__ void HQT_FFT_BOUNDS k_x_d1(XD1Args<T> a) {
+template <typename T> __global__ void HQT_FFT_BOUNDS k_x_d1(const __grid_constant__ XD1Args<T> a) {
     const int n = a.plan.n;
     const int L0 = blockIdx.x * a.NB;
     const int nb = min(a.NB, a.nlines - L0);
@@ -303,7 +303,7 @@ template <typename T> __global__ void HQT_FFT_BOUNDS k_x_d1(XD1Args<T> a) {
     xl_store<T>(r, n, nb, [&](int t, C2<T> v) { store_field(a.out, g0 + t, v); });
 }
 
-template <typename T> __global__ void HQT_FFT_BOUNDS k_y_d1(YD1Args<T> a) {
+template <typename T> __global__ void HQT_FFT_BOUNDS k_y_d1(const __grid_constant__ YD1Args<T> a) {
     const int n = a.ny;
     const int x0 = blockIdx.x * a.TX;
     const int nb = min(a.TX, a.nx - x0);
@@ -332,7 +332,7 @@ template <typename T> __global__ void HQT_FFT_BOUNDS k_y_d1(YD1Args<T> a) {
 // ------------------------------------------------------------------------
 // Fourier filter: x forward, y (forward, weight, inverse), x inverse
 // ------------------------------------------------------------------------
-template <typename T> __global__ void HQT_FFT_BOUNDS k_x_filt_fwd(XFiltFwdArgs<T> a) {
+template <typename T> __global__ void HQT_FFT_BOUNDS k_x_filt_fwd(const __grid_constant__ XFiltFwdArgs<T> a) {
     const int n = a.plan.n;
     const int L0 = blockIdx.x * a.NB;
     const int nb = min(a.NB, a.nlines - L0);
@@ -365,7 +365,7 @@ template <typename T> __global__ void HQT_FFT_BOUNDS k_x_filt_fwd(XFiltFwdArgs<T
     }
 }
 
-template <typename T> __global__ void HQT_FFT_BOUNDS k_y_filt(YFiltArgs<T> a) {
+template <typename T> __global__ void HQT_FFT_BOUNDS k_y_filt(const __grid_constant__ YFiltArgs<T> a) {
     const int n = a.ny;
     const int x0 = blockIdx.x * a.TX;
     const int nb = min(a.TX, a.nx - x0);
@@ -409,7 +409,7 @@ template <typename T> __global__ void HQT_FFT_BOUNDS k_y_filt(YFiltArgs<T> a) {
     }
 }
 
-template <typename T> __global__ void HQT_FFT_BOUNDS k_x_filt_inv(XFiltInvArgs<T> a) {
+template <typename T> __global__ void HQT_FFT_BOUNDS k_x_filt_inv(const __grid_constant__ XFiltInvArgs<T> a) {
     const int n = a.plan.n;
     const int L0 = blockIdx.x * a.NB;
     const int nb = min(a.NB, a.nlines - L0);
@@ -444,7 +444,7 @@ template <typename T> __global__ void HQT_FFT_BOUNDS k_x_filt_inv(XFiltInvArgs<T
 }
 
 // forward transform along y of nf complex fields (used by the spectrum)
-template <typename T> __global__ void HQT_FFT_BOUNDS k_y_fwd(YFiltArgs<T> a) {
+template <typename T> __global__ void HQT_FFT_BOUNDS k_y_fwd(const __grid_constant__ YFiltArgs<T> a) {
     const int n = a.ny;
     const int x0 = blockIdx.x * a.TX;
     const int nb = min(a.TX, a.nx - x0);
