@@ -166,7 +166,8 @@ template <>
 cudaError_t z_misc<HQT_ZN>(const ZColArgs<double> &a, const ZHost &h, int grid, int threads,
                            cudaStream_t s) {
     const ZOps<double, HQT_ZN> op = make_zops(h);
-    (void)klaunch(k_zcol_misc<double, HQT_ZN>, dim3(grid), dim3(threads), 0, s, a, op);
+    if (a.at) (void)klaunch(k_zcol_misc<double, HQT_ZN>, dim3(grid), dim3(threads), 0, s, a, op);
+    if (a.psi) (void)klaunch(k_zcol_O<double, HQT_ZN>, dim3(grid), dim3(threads), 0, s, a, op);
     return cudaGetLastError();
 }
 
