@@ -9,6 +9,8 @@
 // pairs block kb = w (pairs kb*KB .. kb*KB+KB-1) for 32 butterflies at a time,
 // lane = butterfly, with cos/sin(2 pi t k/R) as constant-bank operands.
 #pragma once
+#include <type_traits>
+
 #include "hqt_fft.cuh"
 
 namespace hqt {
@@ -78,16 +80,10 @@ __host__ __device__ constexpr int big_offset(int R) {
 }
 constexpr int kBigTotal = big_offset(61) + 61;
 namespace {
-__constant__ double c_big_cos_d[kBigTotal];
-__constant__ double c_big_sin_d[kBigTotal];
 __constant__ float c_big_cos_f[kBigTotal];
 __constant__ float c_big_sin_f[kBigTotal];
 }  // namespace
 template <typename T> struct BigTab;
-template <> struct BigTab<double> {
-    static __device__ __forceinline__ double c(int i) { return c_big_cos_d[i]; }
-    static __device__ __forceinline__ double s(int i) { return c_big_sin_d[i]; }
-};
 template <> struct BigTab<float> {
     static __device__ __forceinline__ float c(int i) { return c_big_cos_f[i]; }
     static __device__ __forceinline__ float s(int i) { return c_big_sin_f[i]; }
@@ -116,6 +112,7 @@ template <typename T, int N> __host__ __device__ constexpr bool ct_swizzled() {
     return N % (128 / (int)sizeof(C2<T>)) == 0;
 }
 template <typename T, int N> struct CtView {
+    static_assert(std::is_same<T, float>::value, "only the FP32 tables are filled");
     int base;
     __device__ __forceinline__ C2<T> &operator[](int i) const {
         int e = base + i;

@@ -30,7 +30,7 @@
 // multiple of 8: the strided rows of the last forward pass otherwise fall on the
 // same banks.
 //
-// The plan is a compile-time constant (SGeo) for the lengths of HQT_CN_LIST
+// The plan is a compile-time constant (SGeo) for the lengths of HQT_LN_LIST
 // and a kernel argument (RGeo, divisions by multiply-high) for every other
 // length whose prime factors are at most 13.
 #pragma once
@@ -57,13 +57,6 @@ __host__ __device__ constexpr double lf_cos(int R, int k) {
         case 228: return -0.90096886790241912624;
         case 229: return -0.22252093395631440429;
         case 230: return 0.62348980185873353053;
-        case 257: return 0.7071067811865475244;
-        case 258: return 0.0;
-        case 259: return -0.7071067811865475244;
-        case 260: return -1.0;
-        case 261: return -0.7071067811865475244;
-        case 262: return 0.0;
-        case 263: return 0.7071067811865475244;
         case 289: return 0.7660444431189780352;
         case 290: return 0.17364817766693034885;
         case 291: return -0.5;
@@ -94,21 +87,6 @@ __host__ __device__ constexpr double lf_cos(int R, int k) {
         case 426: return 0.12053668025532305335;
         case 427: return 0.56806474673115580251;
         case 428: return 0.8854560256532098959;
-        case 513: return 0.92387953251128675613;
-        case 514: return 0.7071067811865475244;
-        case 515: return 0.38268343236508977173;
-        case 516: return 0.0;
-        case 517: return -0.38268343236508977173;
-        case 518: return -0.7071067811865475244;
-        case 519: return -0.92387953251128675613;
-        case 520: return -1.0;
-        case 521: return -0.92387953251128675613;
-        case 522: return -0.7071067811865475244;
-        case 523: return -0.38268343236508977173;
-        case 524: return 0.0;
-        case 525: return 0.38268343236508977173;
-        case 526: return 0.7071067811865475244;
-        case 527: return 0.92387953251128675613;
         default: return 1.0;
     }
 }
@@ -126,13 +104,6 @@ __host__ __device__ constexpr double lf_sin(int R, int k) {
         case 228: return -0.43388373911755812048;
         case 229: return -0.97492791218182360702;
         case 230: return -0.78183148246802980871;
-        case 257: return 0.7071067811865475244;
-        case 258: return 1.0;
-        case 259: return 0.7071067811865475244;
-        case 260: return 0.0;
-        case 261: return -0.7071067811865475244;
-        case 262: return -1.0;
-        case 263: return -0.7071067811865475244;
         case 289: return 0.64278760968653932632;
         case 290: return 0.98480775301220805937;
         case 291: return 0.86602540378443864676;
@@ -163,21 +134,6 @@ __host__ __device__ constexpr double lf_sin(int R, int k) {
         case 426: return -0.9927088740980539928;
         case 427: return -0.82298386589365639458;
         case 428: return -0.46472317204376854566;
-        case 513: return 0.38268343236508977173;
-        case 514: return 0.7071067811865475244;
-        case 515: return 0.92387953251128675613;
-        case 516: return 1.0;
-        case 517: return 0.92387953251128675613;
-        case 518: return 0.7071067811865475244;
-        case 519: return 0.38268343236508977173;
-        case 520: return 0.0;
-        case 521: return -0.38268343236508977173;
-        case 522: return -0.7071067811865475244;
-        case 523: return -0.92387953251128675613;
-        case 524: return -1.0;
-        case 525: return -0.92387953251128675613;
-        case 526: return -0.7071067811865475244;
-        case 527: return -0.38268343236508977173;
         default: return 0.0;
     }
 }
@@ -220,41 +176,29 @@ template <typename T, int SIGN> struct LDft<T, 4, SIGN> {
         v[3] = b - d;
     }
 };
-// R = 2 H for power-of-two H: two H-point DFTs of the even and odd elements
-template <typename T, int R, int SIGN> struct LDftPow2 {
-    static __device__ __forceinline__ void run(C2<T> (&v)[R]) {
-        constexpr int H = R / 2;
-        C2<T> e[H], o[H];
+// two 4-point DFTs of the even and odd elements; the turns by +-(1 + SIGN i)/sqrt(2)
+// are two adds and two products
+template <typename T, int SIGN> struct LDft<T, 8, SIGN> {
+    static __device__ __forceinline__ void run(C2<T> (&v)[8]) {
+        C2<T> e[4], o[4];
 #pragma unroll
-        for (int i = 0; i < H; ++i) {
+        for (int i = 0; i < 4; ++i) {
             e[i] = v[2 * i];
             o[i] = v[2 * i + 1];
         }
-        ldft<T, H, SIGN>(e);
-        ldft<T, H, SIGN>(o);
+        ldft<T, 4, SIGN>(e);
+        ldft<T, 4, SIGN>(o);
+        const T h = (T)0.70710678118654752440;
+        const C2<T> q1 = lmuli<T, SIGN>(o[1]), q3 = lmuli<T, SIGN>(o[3]);
+        const C2<T> t[4] = {o[0], mk2<T>(h * (o[1].x + q1.x), h * (o[1].y + q1.y)),
+                            lmuli<T, SIGN>(o[2]), mk2<T>(h * (q3.x - o[3].x), h * (q3.y - o[3].y))};
 #pragma unroll
-        for (int k = 0; k < H; ++k) {
-            C2<T> t;
-            if (k == 0) {
-                t = o[0];
-            } else if (4 * k == R) {
-                t = lmuli<T, SIGN>(o[k]);
-            } else if (8 * k == R || 8 * k == 3 * R) {
-                // +-(1 + SIGN i)/sqrt(2) forms: two adds, two products
-                const T h = (T)0.70710678118654752440;
-                const C2<T> q = lmuli<T, SIGN>(o[k]);
-                t = 8 * k == R ? mk2<T>(h * (o[k].x + q.x), h * (o[k].y + q.y))
-                               : mk2<T>(h * (q.x - o[k].x), h * (q.y - o[k].y));
-            } else {
-                t = lrot<T, R, SIGN>(o[k], k);
-            }
-            v[k] = e[k] + t;
-            v[k + H] = e[k] - t;
+        for (int k = 0; k < 4; ++k) {
+            v[k] = e[k] + t[k];
+            v[k + 4] = e[k] - t[k];
         }
     }
 };
-template <typename T, int SIGN> struct LDft<T, 8, SIGN> : LDftPow2<T, 8, SIGN> {};
-template <typename T, int SIGN> struct LDft<T, 16, SIGN> : LDftPow2<T, 16, SIGN> {};
 // odd prime R in the real-pair form: a_j = x_j + x_{R-j}, b_j = x_j - x_{R-j}
 template <typename T, int R, int SIGN> struct LDftOdd {
     static __device__ __forceinline__ void run(C2<T> (&v)[R]) {

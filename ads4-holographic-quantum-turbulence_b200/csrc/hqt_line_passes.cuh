@@ -6,8 +6,10 @@
 // Bound: each pass streams its fields through HBM once (x_rhs 88, y_rhs 112
 // bytes a site in FP64); next come the FP64 units (about 30 operations an
 // element and transform) and shared memory.  Two buffers of a block's lines
-// take at most about 66 KB, so three blocks share an SM and one block's loads
-// and stores run behind another's butterflies.
+// take at most 66 KB (64 KB at 512 and 1024 points along x, 256 and 512 along y), and with
+// 128 registers a thread 512 threads fit on an SM: two such blocks, one's loads and stores
+// behind the other's butterflies.  Four adjacent y lines take up to 130 KB, and from 900
+// points on such a block is alone on its SM.
 // Measured, us a launch, with threads over the lines first and the twiddles loaded
 // for each buffer -> as it is: 512x512x25 x_rhs 196 -> 160 (3.6 TB/s), y_rhs 250 ->
 // 244 (3.0 TB/s), filter x forward 154 -> 125, x inverse 183 -> 164; 256x256x25 x_rhs

@@ -167,9 +167,9 @@ template <typename T> struct LineTab {
     RGeo g;
 };
 
-// log2 of the lines per block.  Two buffers of the block's lines stay within about
-// 64 KB (three blocks per SM); y lines are adjacent columns, of which 8 fill a
-// 128-byte row, and take up to 128 KB for at least 4 of them.
+// log2 of the lines per block.  Two buffers of the block's lines stay within 66 KB (two
+// or three blocks per SM, as the threads' registers allow); y lines are adjacent columns,
+// of which 8 fill a 128-byte row, and take up to 130 KB for 4 of them (one block from 900 points on).
 __host__ __device__ constexpr int lnbl(int n, bool along_y) {
     int b = along_y ? 3 : 2;
     while (b > 0 && (n * 32ll << b) > (along_y && b <= 2 ? 130 : 66) * 1024ll) --b;
