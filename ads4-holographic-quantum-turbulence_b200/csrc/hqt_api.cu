@@ -1145,8 +1145,8 @@ void use_internal_state(hqt_ctx *c) {
 
 // ---------------------------------------------------------------- autotuner
 // Launch geometry of the line passes: the transform engine per axis
-// (prime-factor tensor-core engine, compile-time Stockham engine, runtime-plan
-// engine) and the lines per block of the runtime-plan engine.
+// (prime-factor tensor-core engine, compile-time plan, runtime plan) and the lines per
+// block of a runtime plan.
 struct LineGeom {
     bool px, py, cx, cy;
     int NBx_rhs, NBx_2, TXy_rhs, TXy_2, TXy_filt;
@@ -1945,7 +1945,9 @@ int hqt_create(const hqt_params *params, int device, hqt_ctx **out) {
             return bail(HQT_ECUDA);
         }
     }
-    if (cudaStreamSynchronize(c->stream) != cudaSuccess) {
+    // (the uploads went through the legacy stream, which the context's own does not wait for)
+    if (cudaStreamSynchronize(cudaStreamLegacy) != cudaSuccess ||
+        cudaStreamSynchronize(c->stream) != cudaSuccess) {
         c->err = "initialisation failed";
         return bail(HQT_ECUDA);
     }
