@@ -63,7 +63,7 @@ def ensemble_runs(n_runs: int = 32):
 # Algorithmic bytes per site of one launch of each kernel kind (FP64): the
 # arrays the kernel must read once and write once.
 ALG_BYTES = {"x_rhs": 88, "y_rhs": 112, "zstage": 264, "x_d1": 16, "y_d1": 20,
-             "zcons": 40, "zcol_misc": 16, "filter_x_fwd": 96, "filter_y": 96,
+             "zcons": 40, "zcol_misc": 24, "filter_x_fwd": 96, "filter_y": 96,
              "filter_x_inv": 96}
 # compulsory traffic of a whole FP64 step per site: 4*(S_in + S_k) + 2*S_state
 STEP_BYTES_FP64 = 4 * (40 + 32) + 2 * 40
@@ -199,8 +199,8 @@ def bench_config(workload: str, w: dict, ws: int) -> dict:
             "remove_winding": w["remove_winding"], "filter": True,
             "noise": w["noise"], "amp": w["amp"], "seed": w["seed"],
             "precision": "fp64", "parallelism": f"replicas{ws}",
-            "l2": "no flush: one step touches ~%.2f GB of distinct arrays (about 300 B "
-                  "per site), %.1fx the 126 MB L2" % (300e-9 * sites, 300 * sites / 126e6)}
+            "l2": "no flush: one step touches ~%.2f GB of distinct arrays (280 B "
+                  "per site), %.1fx the 126 MB L2" % (280e-9 * sites, 280 * sites / 126e6)}
 
 
 def dist_init():
